@@ -130,7 +130,10 @@ typedef struct mdrl_ctx mdrl_ctx;
  * many particles per cell or cells well above rc).  Or, with warps_per_cta = 1 (MDRL_ACC_FIXED64,
  * also in batches), one warp per work item: steps_per_piece (1..4) is then the number of i-tile
  * groups each unit is split into, and prune_steps must be 1 (the kernel always prunes).
- * Default {4, 6, 0}; mdrl_autotune picks among both kinds. */
+ * Default {4, 6, 0}; mdrl_autotune picks among both kinds.
+ * Force evaluations (mdrl_force_eval*, mdrl_batch_force_eval; MDRL_ACC_FIXED64) run a third kernel,
+ * over particle lists, until a CTA tile is asked for; under {1, groups, 1} groups splits its items,
+ * without effect on the result. */
 typedef struct {
     int warps_per_cta;
     int steps_per_piece;

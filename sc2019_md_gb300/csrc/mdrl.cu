@@ -203,6 +203,7 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
     const int nidx = c->nseg * c->bins;
     const int nc = c->order + 1;
     dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_fp2); dfree(&c->d_fc2);
+    dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     auto coef = [&](int f, int k, int idx) { return c->tab[((size_t)f * nc + k) * nidx + idx]; };
     if (c->order == 1) {
         std::vector<float2> f2((size_t)3 * nidx), e2((size_t)3 * nidx);
@@ -215,6 +216,13 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
             fr[(size_t)2 * i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(1, 0, i), coef(1, 1, i));
             fr[(size_t)2 * i + 1] = make_float4(coef(2, 0, i), coef(2, 1, i), 0.0f, 0.0f);
         }
+        std::vector<float4> wa(nidx);
+        std::vector<float2> wc(nidx);
+        for (int i = 0; i < nidx; ++i) { wa[i] = fr[(size_t)2 * i]; wc[i] = f2[(size_t)3 * i + 2]; }
+        MDRL_TRY(dalloc(&c->d_wa, wa.size()));
+        MDRL_TRY(dalloc(&c->d_wc, wc.size()));
+        MDRL_CUDA(cudaMemcpy(c->d_wa, wa.data(), sizeof(float4) * wa.size(), cudaMemcpyHostToDevice));
+        MDRL_CUDA(cudaMemcpy(c->d_wc, wc.data(), sizeof(float2) * wc.size(), cudaMemcpyHostToDevice));
         MDRL_TRY(dalloc(&c->d_fr, fr.size()));
         MDRL_CUDA(cudaMemcpy(c->d_fr, fr.data(), sizeof(float4) * fr.size(), cudaMemcpyHostToDevice));
         MDRL_TRY(dalloc(&c->d_f2, f2.size()));
@@ -232,13 +240,21 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
             }
         if (nc == 3) {
             /* order 2 packed without padding for the one-warp-per-item kernel (36 bytes per index) */
-            std::vector<float4> fp2((size_t)2 * nidx);
+            std::vector<float4> fp2((size_t)2 * nidx), wa(nidx), wb(nidx);
             std::vector<float> fc2((size_t)nidx);
             for (int i = 0; i < nidx; ++i) {
+                wa[i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(0, 2, i), coef(1, 0, i));
+                wb[i] = make_float4(coef(1, 1, i), coef(1, 2, i), coef(2, 0, i), coef(2, 1, i));
                 fp2[(size_t)2 * i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(0, 2, i), coef(1, 0, i));
                 fp2[(size_t)2 * i + 1] = make_float4(coef(1, 1, i), coef(1, 2, i), coef(2, 0, i), coef(2, 1, i));
                 fc2[i] = coef(2, 2, i);
             }
+            MDRL_TRY(dalloc(&c->d_wa, wa.size()));
+            MDRL_TRY(dalloc(&c->d_wb, wb.size()));
+            MDRL_TRY(dalloc(&c->d_w1, fc2.size()));
+            MDRL_CUDA(cudaMemcpy(c->d_wa, wa.data(), sizeof(float4) * wa.size(), cudaMemcpyHostToDevice));
+            MDRL_CUDA(cudaMemcpy(c->d_wb, wb.data(), sizeof(float4) * wb.size(), cudaMemcpyHostToDevice));
+            MDRL_CUDA(cudaMemcpy(c->d_w1, fc2.data(), sizeof(float) * fc2.size(), cudaMemcpyHostToDevice));
             MDRL_TRY(dalloc(&c->d_fp2, fp2.size()));
             MDRL_TRY(dalloc(&c->d_fc2, fc2.size()));
             MDRL_CUDA(cudaMemcpy(c->d_fp2, fp2.data(), sizeof(float4) * fp2.size(), cudaMemcpyHostToDevice));
@@ -266,10 +282,12 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
 TableDev mdrl::table_dev(const mdrl_ctx *c) {
     TableDev t;
     t.f2 = c->d_f2; t.e2 = c->d_e2; t.f4 = c->d_f4; t.e4 = c->d_e4; t.fr = c->d_fr; t.fp2 = c->d_fp2; t.fc2 = c->d_fc2;
+    t.wa = c->d_wa; t.wb = c->d_wb; t.wc = c->d_wc; t.w1 = c->d_w1;
     t.order = c->order; t.nseg = c->nseg; t.bins = c->bins; t.lb = ilog2i(c->bins);
     t.min_log2 = c->min_log2;
     t.r2min = std::ldexp(1.0f, c->min_log2);
     t.local = c->local ? 1 : 0;
+    t.bmask = c->local ? ~((1u << (23 - t.lb)) - 1u) : 0u;
     return t;
 }
 
@@ -363,6 +381,7 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     bonded_free(c);
     free_particles(c);
     dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_fp2); dfree(&c->d_fc2);
+    dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     dfree(&c->d_pcoef);
     dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work);
     dfree(&c->d_tot); dfree(&c->d_err); dfree(&c->d_mt);
@@ -384,13 +403,19 @@ static mdrl_status ensure_cells(mdrl_ctx *c) {
     c->ncells = c->g.nc[0] * c->g.nc[1] * c->g.nc[2];
     MDRL_TRY(dalloc(&c->d_count, c->ncells));
     MDRL_TRY(dalloc(&c->d_start, c->ncells + 1));
-    MDRL_TRY(dalloc(&c->d_unit, (size_t)c->ncells * kHalfShellCells * kMaxItemGroups));
-    MDRL_TRY(dalloc(&c->d_work, 1));
+    MDRL_TRY(dalloc(&c->d_work, 2));
     return MDRL_OK;
 }
 
 mdrl_status mdrl::ensure_capacity(mdrl_ctx *c, int n) {
     MDRL_TRY(ensure_cells(c));
+    /* result slots of any kernel and tile (a batch sizes its own) */
+    const size_t slots = (size_t)c->ncells * std::max(kHalfShellCells * kMaxItemGroups, list_cell_slots(std::max(n, c->cap), c->ncells));
+    if (!c->batch && slots > c->unit_cap) {
+        MDRL_TRY(dalloc(&c->d_unit, slots));
+        c->unit_cap = slots;
+        c->graph_n = -1;
+    }
     if (n <= c->cap) return MDRL_OK;
     free_particles(c);
     const size_t m = (size_t)n;
@@ -443,6 +468,23 @@ force_fn pick_force_batch(int order, bool sep, bool extra, bool prune) {
 }
 }  // namespace mdrl
 
+/* Force evaluations take the list kernel unless a CTA tile was asked for: it is the faster one at
+ * every size measured (92k system, order 1: 250 us against 577 us for the default CTA tile and 374 us
+ * for {1, 1, 1}; 1M system, order 2: 1.71 ms against 4.06 and 2.61; 1,728 atoms: within 2 us of the
+ * CTA kernel's 18 us).  Dynamics keeps the kernels of its tile: its FP32 partial sums, and so every
+ * bit of a trajectory, stay those of runs made before. */
+bool mdrl::list_eval(const mdrl_ctx *c) {
+    return c->p.accum == MDRL_ACC_FIXED64 && (!c->tile_set || c->tile.warps_per_cta == 1);
+}
+
+mdrl_status mdrl::list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid) {
+    int per_sm = 0;
+    MDRL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32 * kWarpsPerCta, smem));
+    *grid = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta,
+                     std::max(1, per_sm) * std::max(1, num_sms));
+    return MDRL_OK;
+}
+
 /* The smem attribute is set once per kernel and device, on the first (uncaptured) launch. */
 mdrl_status mdrl::prepare_force_kernel(force_fn fn, int device) {
     static std::mutex mu;
@@ -458,6 +500,31 @@ mdrl_status mdrl::prepare_force_kernel(force_fn fn, int device) {
 }
 
 int mdrl::eff_order(const mdrl_ctx *c) { return c->p.eval == MDRL_EVAL_DIRECT ? 0 : c->order; }
+
+/* The list kernel's launch over the units of home cells [cell0, cell0 + cells); *slots: its result
+ * slots, one per item. */
+static mdrl_status launch_list(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, int cell0, int cells,
+                               int *slots) {
+    const int G = c->tile_set ? c->tile.steps_per_piece : 1;
+    bool fine;
+    int items = 0, grid = 0;
+    const int cfg = list_cfg(n, c->ncells, cells, G, c->num_sms, &fine, &items);
+    const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
+    list_fn fn = (c->p.flags & MDRL_FLAG_EXACT_DIFF) ? pick_force_list<kDiffExact, false>(eff_order(c), false, extra, coul, fine)
+                                                     : pick_force_list<kDiffShift, false>(eff_order(c), sep, extra, coul, fine);
+    MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
+    const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
+    MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
+    MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
+    if (items > 0)    /* k_scan has zeroed the item counter */
+        fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
+            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n, c->d_F64, c->d_cnt, c->d_unit,
+            ListBatch{}, nullptr, cfg, c->d_err, cell0, c->d_work, items);
+    MDRL_CUDA(cudaGetLastError());
+    MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
+    *slots = items;
+    return MDRL_OK;
+}
 
 /* Result slots of a force launch over `units` units: one per CTA (the warp-item kernel runs
  * steps_per_piece i-tile groups per unit). */
@@ -523,21 +590,21 @@ static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int
  * and the gather reads those.  inv: also record each user index's cell-order position. */
 static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, const float *z,
                             const float *q, const int *type, int buf, bool spatial, bool stage = false,
-                            bool inv = false) {
+                            bool inv = false, bool hilbert = false) {
     MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * c->ncells, c->stream));
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     if (n > 0) {
         k_bin_user<<<nblk(n, 256), 256, 0, c->stream>>>(
             n, x, y, z, c->g, c->d_cell_of, c->d_slot, c->d_count, c->d_err, spatial ? c->d_key : nullptr,
             stage ? q : nullptr, stage ? type : nullptr, stage ? c->d_ux : nullptr, c->d_uy, c->d_uz, c->d_uq,
-            c->d_ut);
+            c->d_ut, hilbert ? 1 : 0);
         if (stage) {
             x = c->d_ux; y = c->d_uy; z = c->d_uz;
             if (q) q = c->d_uq;
             if (type) type = c->d_ut;
         }
     }
-    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot);
+    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work);
     if (n > 0) {
         k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
         k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted,
@@ -628,13 +695,15 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     const bool extra = counts != nullptr || (c->p.flags & MDRL_FLAG_ENERGY);
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
-    MDRL_TRY(bin_user(c, n, x, y, z, q, type, 0, true, stage, true));
-    MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra));
+    const bool list = list_eval(c);
+    int slots = force_slots(c, force_items(c->ncells));
+    MDRL_TRY(bin_user(c, n, x, y, z, q, type, 0, true, stage, true, list));
+    if (list) MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], extra, 0, c->ncells, &slots));
+    else MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra));
     const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
     MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, energy));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, energy));
-    k_totals<<<1, 1024, 0, c->stream>>>(force_slots(c, force_items(c->ncells)), c->d_unit, 0, c->d_kepart, c->d_tot,
-                                       extra ? 1 : 0);
+    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
     if (energy) MDRL_TRY(bonded_add_energy(c, n));
     if (n > 0)
@@ -845,11 +914,15 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
     MDRL_TRY(bin_user(c, n, (const float *)dx, (const float *)dy, (const float *)dz, (const float *)dq,
-                      (const int *)dt, 0, true, direct, true));
-    const int per_layer = c->g.nc[1] * c->g.nc[2] * kHalfShellCells;
-    const int units = (hx1 - hx0) * per_layer;
-    MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr, hx0 * per_layer, units));
-    k_totals<<<1, 1024, 0, c->stream>>>(force_slots(c, units), c->d_unit, 0, c->d_kepart, c->d_tot, 0);
+                      (const int *)dt, 0, true, direct, true, list_eval(c)));
+    const int layer = c->g.nc[1] * c->g.nc[2], cells = (hx1 - hx0) * layer;
+    int slots = force_slots(c, cells * kHalfShellCells);
+    if (list_eval(c))
+        MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], false, hx0 * layer, cells, &slots));
+    else
+        MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr,
+                                   hx0 * layer * kHalfShellCells, cells * kHalfShellCells));
+    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, 0);
     if (n > 0) k_unsort_fixed<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_inv, c->d_F64, Fout);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->ev1, c->stream));
@@ -1241,6 +1314,7 @@ static void drop_graphs(mdrl_ctx *c) {
 namespace mdrl {
 mdrl_status set_tile(mdrl_ctx *c, const mdrl_tile *t, bool allow8, bool allow_warp) {
     MDRL_TRY(check_tile(t, allow8, c->p.accum == MDRL_ACC_FIXED64, allow_warp));
+    c->tile_set = true;
     if (t->warps_per_cta != c->tile.warps_per_cta || t->steps_per_piece != c->tile.steps_per_piece ||
         t->prune_steps != c->tile.prune_steps) {
         MDRL_CUDA(cudaSetDevice(c->p.device));

@@ -48,7 +48,7 @@ __global__ void k_bbin_user(int n, const float *__restrict__ x, const float *__r
                             const float *__restrict__ z, const int *__restrict__ rep_of,
                             const BatchRep *__restrict__ reps, int *__restrict__ cell_of,
                             int *__restrict__ slot, int *__restrict__ count, unsigned *__restrict__ err,
-                            unsigned *__restrict__ key) {
+                            unsigned *__restrict__ key, int hilbert) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const BatchRep &rp = reps[rep_of[i]];
@@ -56,7 +56,7 @@ __global__ void k_bbin_user(int n, const float *__restrict__ x, const float *__r
     const float px = x[i], py = y[i], pz = z[i];
     if (!in_box(g, px, py, pz)) atomicOr(err, kErrPosition);
     const int c = cell_of_pos(g, px, py, pz);
-    key[i] = cell_morton(g, px, py, pz, c);
+    key[i] = hilbert ? cell_hilbert(g, px, py, pz, c) : cell_morton(g, px, py, pz, c);
     const int gc = rp.cell_off + c;
     cell_of[i] = gc;
     slot[i] = cell_slot(count, gc);
@@ -90,6 +90,15 @@ __global__ void k_bkick_drift_bin(int n, float4 *__restrict__ pos, float4 *__res
     slot[k] = cell_slot(count, gc);
 }
 
+/* The result slots of a list launch: first slot and slots per item of the min-image [0] and the
+ * half-shell [1] replicas. */
+struct ListSlots {
+    int on;
+    ListBatch list[2];
+    const int *rep_pos;
+    int first[2], per_item[2];
+};
+
 /* Per-replica totals of the last force evaluation (its items, in item order) and, when vel is
  * given, its kinetic energy (particles in cell order); one CTA per replica, fixed order. */
 /* With a one-warp-per-item tile the slots are laid out as [the other items' CTAs][G slots per
@@ -99,7 +108,7 @@ __global__ void __launch_bounds__(128) k_rep_totals(const int *__restrict__ item
                                                     const int *__restrict__ rep_items,
                                                     const int *__restrict__ item_begin2,
                                                     const int *__restrict__ rep_items2, int slot0, int G,
-                                                    const UnitOut *__restrict__ uout,
+                                                    ListSlots ls, const UnitOut *__restrict__ uout,
                                                     const BatchRep *__restrict__ reps,
                                                     const float4 *__restrict__ vel,
                                                     const int *__restrict__ ptype, const MassTab *__restrict__ mt,
@@ -120,6 +129,20 @@ __global__ void __launch_bounds__(128) k_rep_totals(const int *__restrict__ item
             a += u.e_lj; b += u.e_coul; c += u.virial;
             p += u.pairs; q += u.below;
         }
+    if (ls.on && reps[r].path != kPathAllImages) {
+        const int k = reps[r].path == kPathHalfShell;
+        const ListBatch &l = ls.list[k];
+        const int at = ls.rep_pos[r], m = ls.per_item[k];
+        for (int cls = 0; cls < (k ? kClasses : 1); ++cls) {
+            const int *pre = cls == 2 ? l.pre1 : l.pre0;
+            const int base = ls.first[k] + m * (cls * l.total0);
+            for (int e = m * pre[at] + t; e < m * pre[at + 1]; e += 128) {
+                const UnitOut u = uout[base + e];
+                a += u.e_lj; b += u.e_coul; c += u.virial;
+                p += u.pairs; q += u.below;
+            }
+        }
+    }
     if (vel) {
         const BatchRep &rp = reps[r];
         for (int e = t; e < rp.n; e += 128) {
@@ -164,6 +187,16 @@ struct mdrl_batch {
     int n_hs = 0, n_cp = 0, n_ot = 0;
     BatchItem *d_items_hs = nullptr, *d_items_ot = nullptr;
     int *d_begin_hs = nullptr, *d_list_hs = nullptr, *d_begin_ot = nullptr, *d_list_ot = nullptr;
+    /* the list kernel's items (force evaluations): [0] the min-image replicas, [1] the half-shell ones,
+     * each by falling mean occupancy; rep_pos[r]: a replica's place in its list */
+    struct ListReps {
+        ListBatch dev{nullptr, nullptr, nullptr, 0, 0};
+        int *d_rep = nullptr, *d_pre0 = nullptr, *d_pre1 = nullptr;
+        int items = 0, tile_groups = 0;
+    } lists[2];
+    int *d_rep_pos = nullptr;
+    bool list_slots = false; /* the result slots are those of a list launch: */
+    int list_first[2] = {0, 0}, list_per_item[2] = {1, 1};   /* its first slots and slots per item */
     RepTotals *d_reptot = nullptr;
     bool have_eval = false;  /* the unit outputs hold a force evaluation */
 };
@@ -217,7 +250,8 @@ extern "C" mdrl_status mdrl_batch_destroy(mdrl_batch *b) {
     dfree(&b->d_reps); dfree(&b->d_items); dfree(&b->d_rep_of); dfree(&b->d_item_begin);
     dfree(&b->d_rep_items); dfree(&b->d_reptot);
     dfree(&b->d_items_hs); dfree(&b->d_items_ot); dfree(&b->d_begin_hs); dfree(&b->d_list_hs);
-    dfree(&b->d_begin_ot); dfree(&b->d_list_ot);
+    dfree(&b->d_begin_ot); dfree(&b->d_list_ot); dfree(&b->d_rep_pos);
+    for (auto &l : b->lists) { dfree(&l.d_rep); dfree(&l.d_pre0); dfree(&l.d_pre1); }
     if (b->c) mdrl_destroy(b->c);
     delete b;
     return MDRL_OK;
@@ -247,7 +281,11 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
         hrep[r].p_off = (int)ntot;
         hrep[r].cell_off = (int)ncells;
         ntot += reps[r].n;
-        ncells += (long long)hrep[r].g.nc[0] * hrep[r].g.nc[1] * hrep[r].g.nc[2];
+        const int ncr = hrep[r].g.nc[0] * hrep[r].g.nc[1] * hrep[r].g.nc[2], tg = tile_groups(ncr);
+        hrep[r].tile_groups = tg;
+        hrep[r].split0 = list_split(reps[r].n, ncr, tg & 0xff);
+        hrep[r].split1 = list_split(reps[r].n, ncr, tg >> 8);
+        ncells += ncr;
         if (ntot > (1LL << 28) || ncells > (1LL << 24)) {
             set_error("mdrl_batch_create: too many particles or cells in the batch");
             return MDRL_ERR_RANGE;
@@ -331,6 +369,36 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     std::vector<int> begin_hs, list_hs, begin_ot, list_ot;
     rep_lists(items_hs, begin_hs, list_hs);
     rep_lists(items_ot, begin_ot, list_ot);
+    std::vector<int> lrep[2], lpre0[2], lpre1[2], rep_pos(nrep, 0);
+    {
+        std::vector<int> by_load(nrep);
+        std::iota(by_load.begin(), by_load.end(), 0);
+        auto cells = [&](int r) { return hrep[r].g.nc[0] * hrep[r].g.nc[1] * hrep[r].g.nc[2]; };
+        std::stable_sort(by_load.begin(), by_load.end(), [&](int a, int b) {
+            return (long long)hrep[a].n * cells(b) > (long long)hrep[b].n * cells(a);
+        });
+        for (int k = 0; k < 2; ++k) {
+            long long t0 = 0, t1 = 0;
+            int tg0 = 0, tg1 = 0;
+            for (int r : by_load) {
+                if (hrep[r].path != (k ? kPathHalfShell : kPathMinImage)) continue;
+                rep_pos[r] = (int)lrep[k].size();
+                lrep[k].push_back(r); lpre0[k].push_back((int)t0); lpre1[k].push_back((int)t1);
+                t0 += (long long)cells(r) * hrep[r].split0;
+                t1 += (long long)cells(r) * hrep[r].split1;
+                tg0 = std::max(tg0, hrep[r].tile_groups & 0xff);
+                tg1 = std::max(tg1, hrep[r].tile_groups >> 8);
+                if (2 * t0 + t1 > 2147483647LL / kMaxItemGroups) {
+                    delete bt;
+                    set_error("mdrl_batch_create: work list too long");
+                    return MDRL_ERR_RANGE;
+                }
+            }
+            lpre0[k].push_back((int)t0); lpre1[k].push_back((int)t1);
+            bt->lists[k].items = (int)(k ? 2 * t0 + t1 : t0);
+            bt->lists[k].tile_groups = tg0 | (tg1 << 8);
+        }
+    }
     /* the context carries the force field; its own box is the first replica's (never used) */
     mdrl_params pc = *p;
     for (int d = 0; d < 3; ++d) { pc.box[d] = reps[0].box[d]; pc.ncell[d] = 0; }
@@ -340,11 +408,26 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     auto fail = [&](mdrl_status st) { mdrl_batch_destroy(bt); return st; };
     /* the context's cell buffers sized for the whole batch (ensure_capacity keeps them) */
     c->ncells = bt->ncells;
+    c->batch = true;
+    if ((s = dalloc(&c->d_work, 2)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_count, (size_t)bt->ncells)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_start, (size_t)bt->ncells + 1)) != MDRL_OK) return fail(s);
+    /* result slots of any kernel and tile (fine items run below kFineItems per SM, kRuns slots each) */
+    const size_t list_slots = ((size_t)bt->lists[0].items + bt->lists[1].items) * kMaxItemGroups +
+                              (size_t)2 * kFineItems * c->num_sms * kRuns;
     if ((s = dalloc(&c->d_unit, std::max((size_t)bt->nitems,
-                                         (size_t)bt->n_ot + ((size_t)bt->n_cp + bt->n_hs) * kMaxItemGroups))) != MDRL_OK)
+                                         (size_t)bt->n_ot + std::max(((size_t)bt->n_cp + bt->n_hs) * kMaxItemGroups,
+                                                                     list_slots)))) != MDRL_OK)
         return fail(s);
+    for (int k = 0; k < 2; ++k) {
+        auto &l = bt->lists[k];
+        lrep[k].push_back(0);    /* never empty */
+        if ((s = dalloc(&l.d_rep, lrep[k].size())) != MDRL_OK) return fail(s);
+        if ((s = dalloc(&l.d_pre0, lpre0[k].size())) != MDRL_OK) return fail(s);
+        if ((s = dalloc(&l.d_pre1, lpre1[k].size())) != MDRL_OK) return fail(s);
+        l.dev = ListBatch{l.d_rep, l.d_pre0, l.d_pre1, (int)lrep[k].size() - 1, std::max(1, lpre0[k].back())};
+    }
+    if ((s = dalloc(&bt->d_rep_pos, (size_t)nrep)) != MDRL_OK) return fail(s);
     if ((s = ensure_capacity(c, bt->ntot)) != MDRL_OK) return fail(s);
     std::vector<int> rep_of(bt->ntot);
     for (int r = 0; r < nrep; ++r)
@@ -362,6 +445,13 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     if ((s = dalloc(&bt->d_list_hs, std::max<size_t>(1, list_hs.size()))) != MDRL_OK) return fail(s);
     if ((s = dalloc(&bt->d_list_ot, std::max<size_t>(1, list_ot.size()))) != MDRL_OK) return fail(s);
     cudaError_t e = cudaMemcpy(bt->d_reps, bt->reps.data(), sizeof(BatchRep) * nrep, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(bt->d_rep_pos, rep_pos.data(), sizeof(int) * nrep, cudaMemcpyHostToDevice);
+    for (int k = 0; k < 2; ++k) {
+        auto &l = bt->lists[k];
+        if (e == cudaSuccess) e = cudaMemcpy(l.d_rep, lrep[k].data(), sizeof(int) * lrep[k].size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(l.d_pre0, lpre0[k].data(), sizeof(int) * lpre0[k].size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(l.d_pre1, lpre1[k].data(), sizeof(int) * lpre1[k].size(), cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_items, bt->items.data(), sizeof(BatchItem) * bt->nitems, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_rep_of, rep_of.data(), sizeof(int) * bt->ntot, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_item_begin, bt->item_begin.data(), sizeof(int) * (nrep + 1), cudaMemcpyHostToDevice);
@@ -433,15 +523,58 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
     return MDRL_OK;
 }
 
+/* The list kernel's items of list k (0 min-image, 1 half-shell) and whether they are fine ones. */
+static int list_items(const mdrl_batch *b, int k, bool *fine) {
+    const int items = b->lists[k].items * (b->c->tile_set ? b->c->tile.steps_per_piece : 1);
+    *fine = fine_items(b->lists[k].tile_groups, items, b->c->num_sms);
+    return *fine ? items * kRuns : items;
+}
+
+/* A force evaluation's launches (list_eval): the all-image replicas in the CTA kernel, then the list
+ * kernel over the min-image and the half-shell replicas; *slots: their result slots, in that order. */
+static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int *type, bool extra, int *slots) {
+    mdrl_ctx *c = b->c;
+    const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
+    const int G = c->tile_set ? c->tile.steps_per_piece : 1;
+    const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
+    force_fn fo = pick_force_batch(eff_order(c), sep, extra, false);
+    MDRL_TRY(prepare_force_kernel(fo, c->p.device));
+    MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
+    if (b->n_ot)
+        fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
+            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, nullptr,
+            c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0);
+    *slots = b->n_ot;
+    for (int k = 0; k < 2; ++k) {
+        bool fine;
+        int grid = 0;
+        const int items = list_items(b, k, &fine);
+        b->list_first[k] = *slots;
+        b->list_per_item[k] = G * (fine ? kRuns : 1);
+        if (items == 0) continue;
+        list_fn fn = k ? pick_force_list<kDiffShift, true>(eff_order(c), sep, extra, coul, fine)
+                       : pick_force_list<kDiffWrap, true>(eff_order(c), sep, extra, coul, fine);
+        MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
+        MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
+        fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
+            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, c->d_cnt,
+            c->d_unit + *slots, b->lists[k].dev, b->d_reps, G, c->d_err, 0, c->d_work + k, items);
+        *slots += items;
+    }
+    MDRL_CUDA(cudaGetLastError());
+    MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
+    return MDRL_OK;
+}
+
 /* Bin the user-order arrays already on the device into slot `buf` and clear the accumulators. */
-static mdrl_status batch_bin_user(mdrl_batch *b, const float *q, const int *type, int buf) {
+static mdrl_status batch_bin_user(mdrl_batch *b, const float *q, const int *type, int buf, bool hilbert = false) {
     mdrl_ctx *c = b->c;
     const int n = b->ntot;
     MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * (size_t)b->ncells, c->stream));
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     k_bbin_user<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_ux, c->d_uy, c->d_uz, b->d_rep_of, b->d_reps,
-                                                     c->d_cell_of, c->d_slot, c->d_count, c->d_err, c->d_key);
-    k_scan<<<1, 1024, 0, c->stream>>>(b->ncells, c->d_count, c->d_start, c->d_tot);
+                                                     c->d_cell_of, c->d_slot, c->d_count, c->d_err, c->d_key, hilbert ? 1 : 0);
+    k_scan<<<1, 1024, 0, c->stream>>>(b->ncells, c->d_count, c->d_start, c->d_tot, c->d_work);
     k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
     k_cell_sort<<<b->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted, c->d_key, c->d_sortkey,
                                                    c->d_err);
@@ -501,9 +634,13 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     MDRL_TRY(upload_user(b, x, y, z, q, type));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
-    MDRL_TRY(batch_bin_user(b, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0));
-    MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
-    k_totals<<<1, 1024, 0, c->stream>>>(batch_slots(b), c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
+    const bool list = list_eval(c);
+    int slots = batch_slots(b);
+    MDRL_TRY(batch_bin_user(b, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0, list));
+    if (list) MDRL_TRY(batch_launch_list(b, c->d_pos[0], c->d_type[0], extra, &slots));
+    else MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
+    b->list_slots = list;
+    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], c->d_F64, nullptr, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, counts ? c->d_ocnt : nullptr);
     MDRL_CUDA(cudaGetLastError());
@@ -546,6 +683,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
                                                       c->d_vel[0]);
     const bool extra = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
     MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
+    b->list_slots = false;
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, nullptr, c->d_mt, 0,
                                                 c->d_kepart);
     k_totals<<<1, 1024, 0, c->stream>>>(batch_slots(b), c->d_unit, nblk(n, 256), c->d_kepart, c->d_tot, extra ? 1 : 0);
@@ -656,10 +794,21 @@ extern "C" mdrl_status mdrl_batch_replica_stats(mdrl_batch *b, mdrl_stats *out) 
     MDRL_CUDA(cudaSetDevice(c->p.device));
     const int a = c->cur;
     const bool kin = c->have_state;
-    const bool warp = c->tile.warps_per_cta == 1;
-    k_rep_totals<<<b->nrep, 128, 0, c->stream>>>(warp ? b->d_begin_ot : b->d_item_begin, warp ? b->d_list_ot : b->d_rep_items,
+    const bool list = b->list_slots, warp = !list && c->tile.warps_per_cta == 1;
+    ListSlots ls{};
+    if (list) {
+        ls.on = 1;
+        ls.rep_pos = b->d_rep_pos;
+        for (int k = 0; k < 2; ++k) {
+            ls.list[k] = b->lists[k].dev;
+            ls.first[k] = b->list_first[k];
+            ls.per_item[k] = b->list_per_item[k];
+        }
+    }
+    k_rep_totals<<<b->nrep, 128, 0, c->stream>>>(warp || list ? b->d_begin_ot : b->d_item_begin,
+                                                 warp || list ? b->d_list_ot : b->d_rep_items,
                                                  warp ? b->d_begin_hs : nullptr, warp ? b->d_list_hs : nullptr, b->n_ot,
-                                                 warp ? c->tile.steps_per_piece : 1, c->d_unit, b->d_reps,
+                                                 warp ? c->tile.steps_per_piece : 1, ls, c->d_unit, b->d_reps,
                                                  kin ? c->d_vel[a] : nullptr, c->d_type[a], c->d_mt,
                                                  b->d_reptot);
     MDRL_CUDA(cudaGetLastError());

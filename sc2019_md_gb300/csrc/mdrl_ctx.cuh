@@ -10,7 +10,7 @@
 #include <vector>
 
 #include "mdrl_internal.h"
-#include "mdrl_force.cuh"
+#include "mdrl_force_list.cuh"
 
 using mdrl::set_error;
 
@@ -73,6 +73,9 @@ struct mdrl_ctx {
     float2 *d_f2 = nullptr, *d_e2 = nullptr;
     float4 *d_f4 = nullptr, *d_e4 = nullptr, *d_fp2 = nullptr;
     float *d_fc2 = nullptr;
+    float4 *d_wa = nullptr, *d_wb = nullptr;   /* the list kernel's tables */
+    float2 *d_wc = nullptr;
+    float *d_w1 = nullptr;
     float4 *d_fr = nullptr;      /* order 1: force functions packed per index (32 B) */
     float4 *d_pcoef = nullptr;
     MassTab mt_half, mt_full;
@@ -91,7 +94,7 @@ struct mdrl_ctx {
     int cur = 0;
     int *d_cell_of = nullptr, *d_slot = nullptr, *d_tmp = nullptr, *d_sorted = nullptr;
     int *d_count = nullptr, *d_start = nullptr;
-    int *d_work = nullptr;      /* the persistent warp kernel's item counter */
+    int *d_work = nullptr;      /* the persistent force kernels' item counters [2] */
     unsigned *d_key = nullptr;   /* in-cell sort key (Morton code inside the cell) */
     unsigned long long *d_sortkey = nullptr;   /* sorted chunks of cells above kSortSmall */
     unsigned long long *d_F64 = nullptr;
@@ -100,6 +103,7 @@ struct mdrl_ctx {
     float *d_Fscr32 = nullptr;
     int *d_cnt = nullptr;
     UnitOut *d_unit = nullptr;
+    size_t unit_cap = 0;
     double *d_kepart = nullptr;
     int kecap = 0;
     DevTotals *d_tot = nullptr;
@@ -129,6 +133,8 @@ struct mdrl_ctx {
 
     /* force-kernel tile (mdrl_set_tile / mdrl_autotune) */
     mdrl_tile tile = {mdrl::kFW, mdrl::kStepsPerPiece, 0};
+    bool tile_set = false;       /* by a caller or the tuner */
+    bool batch = false;          /* the buffers of an mdrl_batch (which sizes d_unit itself) */
 };
 
 namespace mdrl {
@@ -139,6 +145,10 @@ mdrl_status check_device_errors(mdrl_ctx *c);
 
 /* Raise the dynamic shared-memory limit of a force kernel once per kernel and device. */
 mdrl_status prepare_force_kernel(force_fn fn, int device);
+/* Whether force evaluations run the list kernel, and its persistent grid: the CTAs that fit on the GPU
+ * at once, or fewer when there are fewer items. */
+bool list_eval(const mdrl_ctx *c);
+mdrl_status list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid);
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
 /* PME (mdrl_pme.cu): setup, teardown, the reciprocal part of a force evaluation, its energies. */
 mdrl_status pme_setup(mdrl_ctx *c, const mdrl_pme_params *p);

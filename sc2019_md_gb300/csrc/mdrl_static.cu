@@ -38,7 +38,7 @@
 #include <string>
 #include <vector>
 
-#include "mdrl_force.cuh"
+#include "mdrl_force_list.cuh"
 
 namespace mdrl {
 
@@ -57,7 +57,7 @@ constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 /* Byte offsets of the sub-buffers inside the array. */
 struct Layout {
     size_t err, tot, count, start, unit, cell_of, slot, tmp, sorted, key, sortkey, pos, type, id, F64, tabf,
-        tabe, tabr, pcoef, end;
+        tabe, wa, wb, wc, pcoef, work, end;
 };
 
 constexpr Layout make_layout() {
@@ -80,8 +80,11 @@ constexpr Layout make_layout() {
     l.F64 = o;     o = align256(o + sizeof(unsigned long long) * 3 * kStaticMaxN);
     l.tabf = o;    o = align256(o + sizeof(float4) * 3 * kStaticMaxTable);
     l.tabe = o;    o = align256(o + sizeof(float4) * 3 * kStaticMaxTable);
-    l.tabr = o;    o = align256(o + sizeof(float4) * 2 * kStaticMaxTable);
+    l.wa = o;      o = align256(o + sizeof(float4) * kStaticMaxTable);
+    l.wb = o;      o = align256(o + sizeof(float4) * kStaticMaxTable);
+    l.wc = o;      o = align256(o + sizeof(float2) * kStaticMaxTable);
     l.pcoef = o;   o = align256(o + sizeof(float4) * MDRL_MAX_TYPES * MDRL_MAX_TYPES);
+    l.work = o;    o = align256(o + 2 * sizeof(int));
     l.end = o;
     return l;
 }
@@ -252,16 +255,18 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
         auto coef = [&](int f, int k, int i) { return tab[((size_t)f * nc + k) * nidx + i]; };
         if (order == 1) {
             std::vector<float2> f2((size_t)3 * nidx), e2((size_t)3 * nidx);
-            std::vector<float4> fr((size_t)2 * nidx);
+            std::vector<float4> wa(nidx);
+            std::vector<float2> wc(nidx);
             for (int i = 0; i < nidx; ++i) {
                 for (int f = 0; f < 3; ++f) {
                     f2[(size_t)3 * i + f] = make_float2(coef(f, 0, i), coef(f, 1, i));
                     e2[(size_t)3 * i + f] = make_float2(coef(3 + f, 0, i), coef(3 + f, 1, i));
                 }
-                fr[(size_t)2 * i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(1, 0, i), coef(1, 1, i));
-                fr[(size_t)2 * i + 1] = make_float4(coef(2, 0, i), coef(2, 1, i), 0.0f, 0.0f);
+                wa[i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(1, 0, i), coef(1, 1, i));
+                wc[i] = make_float2(coef(2, 0, i), coef(2, 1, i));
             }
-            ST_CUDA(cudaMemcpyAsync(b + kLayout.tabr, fr.data(), sizeof(float4) * fr.size(), cudaMemcpyHostToDevice, st));
+            ST_CUDA(cudaMemcpyAsync(b + kLayout.wa, wa.data(), sizeof(float4) * wa.size(), cudaMemcpyHostToDevice, st));
+            ST_CUDA(cudaMemcpyAsync(b + kLayout.wc, wc.data(), sizeof(float2) * wc.size(), cudaMemcpyHostToDevice, st));
             ST_CUDA(cudaMemcpyAsync(b + kLayout.tabf, f2.data(), sizeof(float2) * f2.size(), cudaMemcpyHostToDevice, st));
             ST_CUDA(cudaMemcpyAsync(b + kLayout.tabe, e2.data(), sizeof(float2) * e2.size(), cudaMemcpyHostToDevice, st));
         } else {
@@ -273,6 +278,19 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
                     f4[(size_t)3 * i + f] = make_float4(a[0], a[1], a[2], a[3]);
                     e4[(size_t)3 * i + f] = make_float4(e[0], e[1], e[2], e[3]);
                 }
+            std::vector<float4> wa(nidx), wb(nidx);
+            std::vector<float> w1(nidx);
+            if (order == 2) {
+                for (int i = 0; i < nidx; ++i) {
+                    wa[i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(0, 2, i), coef(1, 0, i));
+                    wb[i] = make_float4(coef(1, 1, i), coef(1, 2, i), coef(2, 0, i), coef(2, 1, i));
+                    w1[i] = coef(2, 2, i);
+                }
+                ST_CUDA(cudaMemcpyAsync(b + kLayout.wa, wa.data(), sizeof(float4) * wa.size(), cudaMemcpyHostToDevice, st));
+                ST_CUDA(cudaMemcpyAsync(b + kLayout.wb, wb.data(), sizeof(float4) * wb.size(), cudaMemcpyHostToDevice, st));
+                ST_CUDA(cudaMemcpyAsync(b + kLayout.wc, w1.data(), sizeof(float) * w1.size(), cudaMemcpyHostToDevice, st));
+                ST_CUDA(cudaStreamSynchronize(st)); /* these vectors go out of scope first */
+            }
             ST_CUDA(cudaMemcpyAsync(b + kLayout.tabf, f4.data(), sizeof(float4) * f4.size(), cudaMemcpyHostToDevice, st));
             ST_CUDA(cudaMemcpyAsync(b + kLayout.tabe, e4.data(), sizeof(float4) * e4.size(), cudaMemcpyHostToDevice, st));
         }
@@ -290,14 +308,17 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     TableDev tab;
     tab.f2 = (const float2 *)(b + kLayout.tabf); tab.e2 = (const float2 *)(b + kLayout.tabe);
     tab.f4 = (const float4 *)(b + kLayout.tabf); tab.e4 = (const float4 *)(b + kLayout.tabe);
-    tab.fr = (const float4 *)(b + kLayout.tabr);
-    tab.fp2 = nullptr;   /* the packed order-2 rows are read by the one-warp-per-item kernel only */
+    tab.fr = nullptr;    /* the rows of the other force kernels */
+    tab.fp2 = nullptr;
     tab.fc2 = nullptr;
+    tab.wa = (const float4 *)(b + kLayout.wa); tab.wb = (const float4 *)(b + kLayout.wb);
+    tab.wc = (const float2 *)(b + kLayout.wc); tab.w1 = (const float *)(b + kLayout.wc);
     tab.order = order; tab.nseg = nseg; tab.bins = bins;
     int lb = 0;
     while ((1 << lb) < bins) ++lb;
     tab.lb = lb; tab.min_log2 = m0; tab.r2min = std::ldexp(1.0f, m0);
     tab.local = order >= 2 ? 1 : 0;   /* as a context fits them */
+    tab.bmask = tab.local ? ~((1u << (23 - lb)) - 1u) : 0u;
 
     /* state that must start at zero; the previous call's contents are otherwise left in place */
     const int nc = (int)ncells;
@@ -305,8 +326,9 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     ST_CUDA(cudaMemsetAsync(d_tot, 0, sizeof(DevTotals), st));
     ST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int) * nc, st));
     const int blk = 256, grid = (n + blk - 1) / blk;
-    if (n > 0) k_bin_user<<<grid, blk, 0, st>>>(n, x, y, z, g, d_cell_of, d_slot, d_count, d_err, d_key);
-    k_scan<<<1, 1024, 0, st>>>(nc, d_count, d_start, d_tot);
+    if (n > 0) k_bin_user<<<grid, blk, 0, st>>>(n, x, y, z, g, d_cell_of, d_slot, d_count, d_err, d_key, nullptr,
+                                             nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 1);
+    k_scan<<<1, 1024, 0, st>>>(nc, d_count, d_start, d_tot, (int *)(b + kLayout.work));
     if (n > 0) {
         k_scatter<<<grid, blk, 0, st>>>(n, d_cell_of, d_slot, d_start, d_tmp);
         k_cell_sort<<<nc, 128, 0, st>>>(d_start, d_tmp, d_sorted, d_key, d_sortkey, d_err);
@@ -314,15 +336,24 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
                                             nullptr, p->ntypes, d_err);
     }
     const int ord = p->eval == MDRL_EVAL_DIRECT ? 0 : order;
-    force_fn fn = pick_force(ord, p->arith == MDRL_ARITH_SEPARATE, false, MDRL_ACC_FIXED64, kFW, false,
-                             (p->flags & MDRL_FLAG_EXACT_DIFF) != 0);
-    const size_t smem = force_smem_bytes(p->ntypes, false);
+    int sms = 0, items = 0, ctas = 0;
+    bool fine;
+    ST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int cfg = list_cfg(n, nc, nc, 1, sms, &fine, &items);
+    if (items > kHalfShellCells * kStaticMaxCells) return fail(MDRL_ERR_RANGE, "too many work items for the static scratch");
+    const bool sep = p->arith == MDRL_ARITH_SEPARATE, coul = p->coulomb_k != 0.0;
+    list_fn fn = (p->flags & MDRL_FLAG_EXACT_DIFF) ? pick_force_list<kDiffExact, false>(ord, false, false, coul, fine)
+                                                   : pick_force_list<kDiffShift, false>(ord, sep, false, coul, fine);
+    const size_t smem = force_list_smem_bytes(p->ntypes, false);
     ST_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)force_smem_bytes(MDRL_MAX_TYPES, true, 8)));
-    fn<<<nc * kHalfShellCells, kFT, smem, st>>>(d_pos, d_type, d_start, g, tab, d_pcoef, p->ntypes,
-                                                (float)p->coulomb_k, n, d_F64, nullptr, nullptr, d_unit, nullptr,
-                                                nullptr, tile_word(kStepsPerPiece, 0), d_err, 0);
-    k_totals<<<1, 1024, 0, st>>>(force_items(nc), d_unit, 0, nullptr, d_tot, 0);
+    int per_sm = 0;
+    ST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32 * kWarpsPerCta, smem));
+    ctas = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta, std::max(1, per_sm) * std::max(1, sms));
+    fn<<<ctas, 32 * kWarpsPerCta, smem, st>>>(d_pos, d_type, d_start, g, tab, d_pcoef, p->ntypes, (float)p->coulomb_k, n,
+                                              d_F64, nullptr, d_unit, ListBatch{}, nullptr, cfg, d_err, 0,
+                                              (int *)(b + kLayout.work), items);
+    k_totals<<<1, 1024, 0, st>>>(items, d_unit, 0, nullptr, d_tot, 0);
     if (n > 0)
         k_unsort<<<grid, blk, 0, st>>>(n, d_id, d_F64, nullptr, nullptr, fx, fy, fz, nullptr);
     ST_CUDA(cudaGetLastError());
