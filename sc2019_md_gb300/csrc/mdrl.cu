@@ -20,6 +20,7 @@
 
 #include "mdrl_ctx.cuh"
 #include "mdrl_force_warp.cuh"
+#include "mdrl_hostio.cuh"
 
 using namespace mdrl;
 
@@ -347,6 +348,7 @@ extern "C" mdrl_status mdrl_create(const mdrl_params *p, mdrl_ctx **out) {
     if (e == cudaSuccess) e = cudaMemcpy(c->d_mt, &c->mt_half, sizeof(MassTab), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(c->d_mt + 1, &c->mt_full, sizeof(MassTab), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, p->device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
     if (e != cudaSuccess) {
         set_error(std::string("context setup: ") + cudaGetErrorString(e));
         mdrl_destroy(c);
@@ -670,26 +672,25 @@ static mdrl_status read_stats(mdrl_ctx *c, mdrl_stats *st, float ms) {
     return MDRL_OK;
 }
 
-/* The device address of p when the context's device can read and write it in place: page-locked
- * host memory (cudaHostAlloc / cudaHostRegister, mapped), managed memory, or memory of this
- * device; nullptr otherwise (pageable host memory: the caller stages through copies). */
+/* device_view of memory that is not pageable: the kernels of a call use it in place throughout. */
 static void *mapped(const mdrl_ctx *c, const void *p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    if (a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged) return a.devicePointer;
-    if (a.type == cudaMemoryTypeDevice && a.device == c->p.device) return a.devicePointer;
-    return nullptr;
+    bool pageable = false;
+    void *v = device_view(c, p, 4, &pageable);
+    return pageable ? nullptr : v;
 }
+
+/* Pageable outputs of a force evaluation, to be populated while the GPU computes. */
+struct Outputs {
+    void *ptr[4];
+    int count = 0;
+};
 
 /* One force evaluation enqueued on the context stream; its last kernel writes the error word and
  * the totals into pinned host memory (copies when there are no particles); force_eval_finish
  * reads them after the one synchronisation of the call. */
 static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const float *y, const float *z,
                                       const float *q, const int *type, float *fx, float *fy, float *fz,
-                                      int *counts, bool stage = false) {
+                                      int *counts, bool stage = false, const Outputs *out = nullptr) {
     MDRL_TRY(ensure_capacity(c, n));
     MDRL_TRY(bonded_check_atoms(c, n));
     const bool extra = counts != nullptr || (c->p.flags & MDRL_FLAG_ENERGY);
@@ -706,6 +707,7 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
     if (energy) MDRL_TRY(bonded_add_energy(c, n));
+    if (out) populate(out->ptr, out->count, 4 * (size_t)n);
     if (n > 0)
         k_unsort_inv<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_inv, c->d_F64, c->d_F32, c->d_cnt, fx, fy,
                                                           fz, counts, c->d_tot, c->h_tot_dev, c->d_err, c->h_err_dev);
@@ -789,23 +791,27 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
             return force_eval_finish(c, st);
         }
     }
-    const size_t fb = sizeof(float) * (size_t)n;
-    if (n > 0) {
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ux, x, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uy, y, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uz, z, fb, cudaMemcpyHostToDevice, c->stream));
-        if (q) MDRL_CUDA(cudaMemcpyAsync(c->d_uq, q, fb, cudaMemcpyHostToDevice, c->stream));
-        if (type) MDRL_CUDA(cudaMemcpyAsync(c->d_ut, type, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    const void *src[5] = {x, y, z, q, type};
+    void *dst[5] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 5, src, dst, false));
+    /* the forces go to the caller's arrays in place when the device can write them all */
+    void *host[4] = {fx, fy, fz, counts}, *view[4] = {nullptr, nullptr, nullptr, nullptr};
+    const void *dev[4] = {c->d_ox, c->d_oy, c->d_oz, c->d_ocnt};
+    bool direct = n > 0;
+    Outputs out;
+    for (int k = 0; k < 4 && direct; ++k) {
+        if (!host[k]) continue;
+        bool pageable = false;
+        view[k] = device_view(c, host[k], 4, &pageable);
+        if (!view[k]) direct = false;
+        else if (pageable) out.ptr[out.count++] = host[k];
     }
-    MDRL_TRY(force_eval_enqueue(c, n, c->d_ux, c->d_uy, c->d_uz, q ? c->d_uq : nullptr,
-                                type ? c->d_ut : nullptr, c->d_ox, c->d_oy, c->d_oz,
-                                counts ? c->d_ocnt : nullptr));
-    if (n > 0) {
-        MDRL_CUDA(cudaMemcpyAsync(fx, c->d_ox, fb, cudaMemcpyDeviceToHost, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(fy, c->d_oy, fb, cudaMemcpyDeviceToHost, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(fz, c->d_oz, fb, cudaMemcpyDeviceToHost, c->stream));
-        if (counts) MDRL_CUDA(cudaMemcpyAsync(counts, c->d_ocnt, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
-    }
+    if (!direct)
+        for (int k = 0; k < 4; ++k) view[k] = host[k] ? const_cast<void *>(dev[k]) : nullptr;
+    MDRL_TRY(force_eval_enqueue(c, n, c->d_ux, c->d_uy, c->d_uz, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr,
+                                (float *)view[0], (float *)view[1], (float *)view[2], (int *)view[3], false,
+                                direct ? &out : nullptr));
+    if (!direct) MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, dev, host, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));   /* the one synchronisation of the call */
     return force_eval_finish(c, st);
 }
@@ -894,17 +900,15 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
         set_error("mdrl_force_eval_fixed: home layers must satisfy 0 <= home_x0 <= home_x1 <= ncell[0]");
         return MDRL_ERR_INVALID_ARG;
     }
-    const size_t fb = sizeof(float) * (size_t)n;
     const void *dx = n ? mapped(c, x) : nullptr, *dy = n ? mapped(c, y) : nullptr, *dz = n ? mapped(c, z) : nullptr;
     const void *dq = (q && n) ? mapped(c, q) : nullptr, *dt = (type && n) ? mapped(c, type) : nullptr;
-    void *dF = n ? mapped(c, F) : nullptr;
+    bool pageable = false;
+    void *dF = n ? device_view(c, F, 8, &pageable) : nullptr;
     const bool direct = n > 0 && dx && dy && dz && (!q || dq) && (!type || dt);
     if (n > 0 && !direct) {
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ux, x, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uy, y, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uz, z, fb, cudaMemcpyHostToDevice, c->stream));
-        if (q) MDRL_CUDA(cudaMemcpyAsync(c->d_uq, q, fb, cudaMemcpyHostToDevice, c->stream));
-        if (type) MDRL_CUDA(cudaMemcpyAsync(c->d_ut, type, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+        const void *src[5] = {x, y, z, q, type};
+        void *dst[5] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut};
+        MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 5, src, dst, false));
         dx = c->d_ux; dy = c->d_uy; dz = c->d_uz;
         dq = q ? c->d_uq : nullptr;
         dt = type ? c->d_ut : nullptr;
@@ -923,6 +927,7 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
         MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr,
                                    hx0 * layer * kHalfShellCells, cells * kHalfShellCells));
     k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, 0);
+    if (dF && pageable) populate((void *const *)&F, 1, 3 * sizeof(int64_t) * (size_t)n);
     if (n > 0) k_unsort_fixed<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_inv, c->d_F64, Fout);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->ev1, c->stream));
@@ -944,16 +949,14 @@ extern "C" mdrl_status mdrl_bin(mdrl_ctx *c, int n, const float *x, const float 
     }
     MDRL_CUDA(cudaSetDevice(c->p.device));
     MDRL_TRY(ensure_capacity(c, n));
-    const size_t fb = sizeof(float) * (size_t)n;
-    if (n > 0) {
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ux, x, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uy, y, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_uz, z, fb, cudaMemcpyHostToDevice, c->stream));
-    }
+    const void *src[3] = {x, y, z};
+    void *dst[3] = {c->d_ux, c->d_uy, c->d_uz};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 3, src, dst, false));
     MDRL_TRY(bin_user(c, n, c->d_ux, c->d_uy, c->d_uz, nullptr, nullptr, 0, false));
-    if (cell_of && n > 0) MDRL_CUDA(cudaMemcpyAsync(cell_of, c->d_cell_of, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream));
+    const void *bsrc[2] = {c->d_cell_of, c->d_sorted};
+    void *bdst[2] = {cell_of, order};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 2, bsrc, bdst, true));
     if (cell_count) MDRL_CUDA(cudaMemcpyAsync(cell_count, c->d_count, sizeof(int) * c->ncells, cudaMemcpyDeviceToHost, c->stream));
-    if (order && n > 0) MDRL_CUDA(cudaMemcpyAsync(order, c->d_sorted, sizeof(int) * n, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_TRY(check_device_errors(c));
     c->have_state = false;
@@ -1096,21 +1099,35 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
         MDRL_TRY(dalloc(&c->d_ptr, n)); MDRL_TRY(dalloc(&c->d_ptn, n)); MDRL_TRY(dalloc(&c->d_paux, n));
         c->pcap = n;
     }
-    MDRL_CUDA(cudaMemcpyAsync(c->d_pr, ref, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(c->d_pn, nbr, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
-    if (tref) MDRL_CUDA(cudaMemcpyAsync(c->d_ptr, tref, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
-    if (tnbr) MDRL_CUDA(cudaMemcpyAsync(c->d_ptn, tnbr, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
+    /* the types are read and the results written in place where the device can; the positions are
+     * copied (4 n elements: two launches' worth of 2^31 at most) */
+    const bool small = n <= 0x7fffffff / 4;
+    const void *src[2] = {ref, nbr};
+    void *dst[2] = {c->d_pr, c->d_pn};
+    if (small) MDRL_CUDA(cudaMemcpyAsyncArrays(c, 4 * n, 2, src, dst, false));
+    else {
+        MDRL_CUDA(cudaMemcpyAsync(c->d_pr, ref, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
+        MDRL_CUDA(cudaMemcpyAsync(c->d_pn, nbr, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
+    }
+    bool pg_out = false, pg_aux = false;
+    const int *vtr = tref ? (const int *)device_view(c, tref, 4) : nullptr, *vtn = tnbr ? (const int *)device_view(c, tnbr, 4) : nullptr;
+    float4 *vout = (uintptr_t)out % 16 ? nullptr : (float4 *)device_view(c, out, 16, &pg_out);
+    float2 *vaux = !aux || (uintptr_t)aux % 8 ? nullptr : (float2 *)device_view(c, aux, 8, &pg_aux);
+    if (tref && !vtr) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptr, tref, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtr = c->d_ptr; }
+    if (tnbr && !vtn) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptn, tnbr, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtn = c->d_ptn; }
+    void *po = out, *pa = aux;
+    if (vout && pg_out) populate(&po, 1, sizeof(float4) * (size_t)n);
+    if (vaux && pg_aux) populate(&pa, 1, sizeof(float2) * (size_t)n);
     Geom g = c->g;
     if (c->p.flags & MDRL_FLAG_NO_PBC)
         for (int d = 0; d < 3; ++d) { g.L[d] = 0.0f; g.h[d] = 0.0f; }
     pair_fn fn = pick_pair(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE);
-    fn<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_pr, c->d_pn, tref ? c->d_ptr : nullptr,
-                                            tnbr ? c->d_ptn : nullptr, g, table_dev(c), c->d_pcoef,
-                                            c->p.ntypes, c->ke, c->d_pout, aux ? c->d_paux : nullptr,
+    fn<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_pr, c->d_pn, vtr, vtn, g, table_dev(c), c->d_pcoef,
+                                            c->p.ntypes, c->ke, vout ? vout : c->d_pout, vaux ? vaux : (aux ? c->d_paux : nullptr),
                                             (c->p.flags & MDRL_FLAG_EXACT_DIFF) ? 1 : 0);
     MDRL_CUDA(cudaGetLastError());
-    MDRL_CUDA(cudaMemcpyAsync(out, c->d_pout, sizeof(float4) * n, cudaMemcpyDeviceToHost, c->stream));
-    if (aux) MDRL_CUDA(cudaMemcpyAsync(aux, c->d_paux, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream));
+    if (!vout) MDRL_CUDA(cudaMemcpyAsync(out, c->d_pout, sizeof(float4) * n, cudaMemcpyDeviceToHost, c->stream));
+    if (aux && !vaux) MDRL_CUDA(cudaMemcpyAsync(aux, c->d_paux, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     return MDRL_OK;
 }
@@ -1127,17 +1144,9 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_CUDA(cudaSetDevice(c->p.device));
     MDRL_TRY(ensure_capacity(c, n));
     MDRL_TRY(bonded_check_atoms(c, n));
-    const size_t fb = sizeof(float) * (size_t)n;
-    MDRL_CUDA(cudaMemcpyAsync(c->d_ux, x, fb, cudaMemcpyHostToDevice, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(c->d_uy, y, fb, cudaMemcpyHostToDevice, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(c->d_uz, z, fb, cudaMemcpyHostToDevice, c->stream));
-    if (q) MDRL_CUDA(cudaMemcpyAsync(c->d_uq, q, fb, cudaMemcpyHostToDevice, c->stream));
-    if (type) MDRL_CUDA(cudaMemcpyAsync(c->d_ut, type, sizeof(int) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
-    if (vx) {
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovx, vx, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovy, vy, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovz, vz, fb, cudaMemcpyHostToDevice, c->stream));
-    }
+    const void *src[8] = {x, y, z, q, type, vx, vy, vz};
+    void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 8, src, dst, false));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     c->cur = 0;
     MDRL_TRY(bin_user(c, n, c->d_ux, c->d_uy, c->d_uz, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0, true));
@@ -1263,11 +1272,9 @@ extern "C" mdrl_status mdrl_get_state(mdrl_ctx *c, float *x, float *y, float *z,
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[a], c->d_F64, c->d_F32, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, nullptr);
     MDRL_CUDA(cudaGetLastError());
-    const size_t fb = sizeof(float) * (size_t)n;
-    float *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
-    const float *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
-    for (int k = 0; k < 9; ++k)
-        if (dst[k]) MDRL_CUDA(cudaMemcpyAsync(dst[k], src[k], fb, cudaMemcpyDeviceToHost, c->stream));
+    void *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
+    const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     return MDRL_OK;
 }

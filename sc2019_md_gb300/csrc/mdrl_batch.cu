@@ -33,6 +33,7 @@
 
 #include "mdrl_ctx.cuh"
 #include "mdrl_force_warp.cuh"
+#include "mdrl_hostio.cuh"
 
 using namespace mdrl;
 
@@ -585,15 +586,13 @@ static mdrl_status batch_bin_user(mdrl_batch *b, const float *q, const int *type
     return MDRL_OK;
 }
 
-static mdrl_status upload_user(mdrl_batch *b, const float *x, const float *y, const float *z,
-                               const float *q, const int *type) {
+static mdrl_status upload_user(mdrl_batch *b, const float *x, const float *y, const float *z, const float *q,
+                               const int *type, const float *vx = nullptr, const float *vy = nullptr,
+                               const float *vz = nullptr) {
     mdrl_ctx *c = b->c;
-    const size_t fb = sizeof(float) * (size_t)b->ntot;
-    MDRL_CUDA(cudaMemcpyAsync(c->d_ux, x, fb, cudaMemcpyHostToDevice, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(c->d_uy, y, fb, cudaMemcpyHostToDevice, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(c->d_uz, z, fb, cudaMemcpyHostToDevice, c->stream));
-    if (q) MDRL_CUDA(cudaMemcpyAsync(c->d_uq, q, fb, cudaMemcpyHostToDevice, c->stream));
-    if (type) MDRL_CUDA(cudaMemcpyAsync(c->d_ut, type, sizeof(int) * (size_t)b->ntot, cudaMemcpyHostToDevice, c->stream));
+    const void *src[8] = {x, y, z, q, type, vx, vy, vz};
+    void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, b->ntot, 8, src, dst, false));
     return MDRL_OK;
 }
 
@@ -645,11 +644,9 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
                                                   c->d_oz, counts ? c->d_ocnt : nullptr);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->ev1, c->stream));
-    const size_t fb = sizeof(float) * (size_t)n;
-    MDRL_CUDA(cudaMemcpyAsync(fx, c->d_ox, fb, cudaMemcpyDeviceToHost, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(fy, c->d_oy, fb, cudaMemcpyDeviceToHost, c->stream));
-    MDRL_CUDA(cudaMemcpyAsync(fz, c->d_oz, fb, cudaMemcpyDeviceToHost, c->stream));
-    if (counts) MDRL_CUDA(cudaMemcpyAsync(counts, c->d_ocnt, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
+    const void *src[4] = {c->d_ox, c->d_oy, c->d_oz, c->d_ocnt};
+    void *dst[4] = {fx, fy, fz, counts};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     float ms = 0.0f;
     MDRL_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
@@ -669,13 +666,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     mdrl_ctx *c = b->c;
     MDRL_CUDA(cudaSetDevice(c->p.device));
     const int n = b->ntot;
-    const size_t fb = sizeof(float) * (size_t)n;
-    MDRL_TRY(upload_user(b, x, y, z, q, type));
-    if (vx) {
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovx, vx, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovy, vy, fb, cudaMemcpyHostToDevice, c->stream));
-        MDRL_CUDA(cudaMemcpyAsync(c->d_ovz, vz, fb, cudaMemcpyHostToDevice, c->stream));
-    }
+    MDRL_TRY(upload_user(b, x, y, z, q, type, vx, vy, vz));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     c->cur = 0;
     MDRL_TRY(batch_bin_user(b, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0));
@@ -778,11 +769,9 @@ extern "C" mdrl_status mdrl_batch_get_state(mdrl_batch *b, float *x, float *y, f
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[a], c->d_F64, nullptr, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, nullptr);
     MDRL_CUDA(cudaGetLastError());
-    const size_t fb = sizeof(float) * (size_t)n;
-    float *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
-    const float *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
-    for (int k = 0; k < 9; ++k)
-        if (dst[k]) MDRL_CUDA(cudaMemcpyAsync(dst[k], src[k], fb, cudaMemcpyDeviceToHost, c->stream));
+    void *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
+    const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
+    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     return MDRL_OK;
 }

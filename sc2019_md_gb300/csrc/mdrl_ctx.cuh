@@ -113,6 +113,7 @@ struct mdrl_ctx {
     unsigned *h_err_dev = nullptr;
     unsigned *d_err = nullptr;
     int num_sms = 0;
+    int host_tables = 0;         /* the device walks the host's page tables: pageable memory in place */
 
     /* pair-eval staging */
     int pcap = 0;
