@@ -338,6 +338,8 @@ extern "C" mdrl_status mdrl_create(const mdrl_params *p, mdrl_ctx **out) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->evf0);
     if (e == cudaSuccess) e = cudaEventCreate(&c->evf1);
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_tot, sizeof(DevTotals));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_totscr, sizeof(TotScratch));
+    if (e == cudaSuccess) e = cudaMemset(c->d_totscr, 0, sizeof(TotScratch));
     if (e == cudaSuccess) e = cudaMalloc((void **)&c->d_err, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_tot, sizeof(DevTotals));
     if (e == cudaSuccess) e = cudaMallocHost((void **)&c->h_err, sizeof(unsigned));
@@ -386,7 +388,7 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     dfree(&c->d_pcoef);
     dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work);
-    dfree(&c->d_tot); dfree(&c->d_err); dfree(&c->d_mt);
+    dfree(&c->d_tot); dfree(&c->d_totscr); dfree(&c->d_err); dfree(&c->d_mt);
     if (c->h_tot) cudaFreeHost(c->h_tot);
     if (c->h_err) cudaFreeHost(c->h_err);
     dfree(&c->d_pr); dfree(&c->d_pn); dfree(&c->d_pout); dfree(&c->d_ptr); dfree(&c->d_ptn); dfree(&c->d_paux);
@@ -485,6 +487,11 @@ mdrl_status mdrl::list_grid(list_fn fn, size_t smem, int items, bool fine, int n
     *grid = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta,
                      std::max(1, per_sm) * std::max(1, num_sms));
     return MDRL_OK;
+}
+
+void mdrl::launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy) {
+    k_totals<<<tot_blocks(nunits, nke), kTotThreads, 0, c->stream>>>(nunits, c->d_unit, nke, c->d_kepart, c->d_tot,
+                                                                    energy ? 1 : 0, c->d_totscr);
 }
 
 /* The smem attribute is set once per kernel and device, on the first (uncaptured) launch. */
@@ -704,7 +711,7 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
     MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, energy));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, energy));
-    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
+    launch_totals(c, slots, 0, extra);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
     if (energy) MDRL_TRY(bonded_add_energy(c, n));
     if (out) populate(out->ptr, out->count, 4 * (size_t)n);
@@ -926,7 +933,7 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     else
         MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr,
                                    hx0 * layer * kHalfShellCells, cells * kHalfShellCells));
-    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, 0);
+    launch_totals(c, slots, 0, false);
     if (dF && pageable) populate((void *const *)&F, 1, 3 * sizeof(int64_t) * (size_t)n);
     if (n > 0) k_unsort_fixed<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_inv, c->d_F64, Fout);
     MDRL_CUDA(cudaGetLastError());
@@ -1158,8 +1165,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, extra));
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, c->d_F32, c->d_mt, 0,
                                                 c->d_kepart);
-    k_totals<<<1, 1024, 0, c->stream>>>(force_slots(c, force_items(c->ncells)), c->d_unit, nblk(n, 256), c->d_kepart, c->d_tot,
-                                       extra ? 1 : 0);
+    launch_totals(c, force_slots(c, force_items(c->ncells)), nblk(n, 256), extra);
     if (extra) MDRL_TRY(pme_add_energy(c, n));
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());
@@ -1196,8 +1202,7 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[b], c->d_type[b], c->d_F64, c->d_F32, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    k_totals<<<1, 1024, 0, c->stream>>>(force_slots(c, force_items(c->ncells)), c->d_unit, extra ? nblk(n, 256) : 0,
-                                       c->d_kepart, c->d_tot, extra ? 1 : 0);
+    launch_totals(c, force_slots(c, force_items(c->ncells)), extra ? nblk(n, 256) : 0, extra);
     if (extra) MDRL_TRY(pme_add_energy(c, n));
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());

@@ -639,7 +639,7 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     if (list) MDRL_TRY(batch_launch_list(b, c->d_pos[0], c->d_type[0], extra, &slots));
     else MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
     b->list_slots = list;
-    k_totals<<<1, 1024, 0, c->stream>>>(slots, c->d_unit, 0, c->d_kepart, c->d_tot, extra ? 1 : 0);
+    launch_totals(c, slots, 0, extra);
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], c->d_F64, nullptr, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, counts ? c->d_ocnt : nullptr);
     MDRL_CUDA(cudaGetLastError());
@@ -677,7 +677,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     b->list_slots = false;
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, nullptr, c->d_mt, 0,
                                                 c->d_kepart);
-    k_totals<<<1, 1024, 0, c->stream>>>(batch_slots(b), c->d_unit, nblk(n, 256), c->d_kepart, c->d_tot, extra ? 1 : 0);
+    launch_totals(c, batch_slots(b), nblk(n, 256), extra);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_TRY(check_device_errors(c));
@@ -710,8 +710,7 @@ static mdrl_status batch_enqueue_step(mdrl_batch *b, bool extra) {
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[d], c->d_type[d], c->d_F64, nullptr, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    k_totals<<<1, 1024, 0, c->stream>>>(batch_slots(b), c->d_unit, extra ? nblk(n, 256) : 0, c->d_kepart, c->d_tot,
-                                       extra ? 1 : 0);
+    launch_totals(c, batch_slots(b), extra ? nblk(n, 256) : 0, extra);
     MDRL_CUDA(cudaGetLastError());
     return MDRL_OK;
 }

@@ -107,6 +107,7 @@ struct mdrl_ctx {
     double *d_kepart = nullptr;
     int kecap = 0;
     DevTotals *d_tot = nullptr;
+    mdrl::TotScratch *d_totscr = nullptr;   /* k_totals' partial sums */
     DevTotals *h_tot = nullptr;  /* pinned host copies, read back with the results of a call */
     unsigned *h_err = nullptr;
     DevTotals *h_tot_dev = nullptr;  /* the same two, as device addresses */
@@ -149,6 +150,8 @@ mdrl_status prepare_force_kernel(force_fn fn, int device);
 /* Whether force evaluations run the list kernel, and its persistent grid: the CTAs that fit on the GPU
  * at once, or fewer when there are fewer items. */
 bool list_eval(const mdrl_ctx *c);
+/* The totals of the last force launch (nunits result slots, nke kinetic-energy partials) into d_tot. */
+void launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy);
 mdrl_status list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid);
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
 /* PME (mdrl_pme.cu): setup, teardown, the reciprocal part of a force evaluation, its energies. */

@@ -350,31 +350,59 @@ static __global__ void k_bin_user(int n, const float *__restrict__ x, const floa
 }
 
 /* Exclusive scan of the cell counts (one CTA), plus the largest occupancy; zeroes the force launches'
- * item counters work[0..1] on the way (a memset less per evaluation). */
+ * item counters work[0..1] on the way (a memset less per evaluation).  Latency-bound: 4 counts per
+ * thread and pass in one 16-byte load, warp scans by shuffles, one barrier per pass of 4,096 cells.
+ * (A strided run of cells per thread and a 20-barrier scan: 486 cells 3.8 us, 10,648 cells 9.9 us, 28k
+ * cells 53 us; now 2.2, 3.3 and 6.) */
 static __global__ void __launch_bounds__(1024) k_scan(int ncells, const int *__restrict__ count,
                                                int *__restrict__ start, DevTotals *tot, int *work = nullptr) {
-    __shared__ int s_sum[1024];
-    __shared__ int s_max[1024];
-    const int t = threadIdx.x;
+    __shared__ int s_sum[2][32], s_max[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (work && t < 2) work[t] = 0;
-    const int per = (ncells + 1023) / 1024;
-    const int b = t * per, e = min(ncells, b + per);
-    int sum = 0, mx = 0;
-    for (int k = b; k < e; ++k) { const int c = count[k]; sum += c; mx = max(mx, c); }
-    s_sum[t] = sum;
-    s_max[t] = mx;
-    __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const int v = (t >= off) ? s_sum[t - off] : 0;
-        const int m = (t >= off) ? s_max[t - off] : 0;
+    int carry = 0, mx = 0, pass = 0;
+    for (int base = 0; base < ncells; base += 4096, pass ^= 1) {
+        const int k = base + 4 * t;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (k + 3 < ncells) c = *reinterpret_cast<const int4 *>(count + k);
+        else {
+            if (k < ncells) c.x = count[k];
+            if (k + 1 < ncells) c.y = count[k + 1];
+            if (k + 2 < ncells) c.z = count[k + 2];
+        }
+        mx = max(mx, max(max(c.x, c.y), max(c.z, c.w)));
+        const int own = c.x + c.y + c.z + c.w;
+        int sum = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += v;
+        }
+        if (lane == 31) s_sum[pass][warp] = sum;
         __syncthreads();
-        s_sum[t] += v;
-        s_max[t] = max(s_max[t], m);
-        __syncthreads();
+        int ws = s_sum[pass][lane];          /* every warp scans the warp sums for itself */
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, ws, o);
+            if (lane >= o) ws += v;
+        }
+        const int before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
+        const int first = carry + (warp ? before : 0) + sum - own;
+        carry += __shfl_sync(0xffffffffu, ws, 31);
+        const int4 r = make_int4(first, first + c.x, first + c.x + c.y, first + c.x + c.y + c.z);
+        if (k + 3 < ncells) *reinterpret_cast<int4 *>(start + k) = r;
+        else {
+            if (k < ncells) start[k] = r.x;
+            if (k + 1 < ncells) start[k + 1] = r.y;
+            if (k + 2 < ncells) start[k + 2] = r.z;
+        }
     }
-    int run = s_sum[t] - sum;
-    for (int k = b; k < e; ++k) { start[k] = run; run += count[k]; }
-    if (t == 1023) { start[ncells] = s_sum[1023]; tot->max_occ = s_max[1023]; }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) s_max[warp] = mx;
+    __syncthreads();
+    if (warp == 0) {
+        mx = __reduce_max_sync(0xffffffffu, s_max[lane]);
+        if (lane == 0) { start[ncells] = carry; tot->max_occ = mx; }
+    }
 }
 
 static __global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__restrict__ slot,
@@ -488,63 +516,83 @@ static __global__ void k_gather_user(int n, const int *__restrict__ sorted, cons
     if (counts) counts[k] = 0;
 }
 
-/* Totals over units and kinetic-energy partials, in a fixed order (one CTA of 1024 threads:
- * strided partial sums, then warp shuffles and a final warp; the same order every call).  GB300
- * runs FP64 at a small fraction of its FP32 rate, so the FP64 energy sums run only when energies
- * were computed. */
-static __global__ void __launch_bounds__(1024) k_totals(int nunits, const UnitOut *__restrict__ uout,
-                                                        int nke, const double *__restrict__ kepart,
-                                                        DevTotals *tot, int with_energy) {
-    __shared__ double s_d[32][4];
-    __shared__ unsigned long long s_u[32][2];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    double a = 0, b = 0, c = 0, k = 0;
-    unsigned long long p = 0, q = 0;
-    /* unrolled so that the loads of several slots are in flight at once (the sums keep their order) */
-#pragma unroll 8
-    for (int u = t; u < nunits; u += 1024) {
-        p += uout[u].pairs;
-        if (with_energy) {
-            a += uout[u].e_lj; b += uout[u].e_coul; c += uout[u].virial;
-            q += uout[u].below;
+/* Totals over units and kinetic-energy partials, in a fixed order: CTA b of nb sums the units and
+ * partials of its threads' stride into part[b], and the last CTA to finish sums those.  GB300 runs
+ * FP64 at a small fraction of its FP32 rate (2 lanes per SM and cycle), so the sums are spread over
+ * SMs and halve the active threads at every level; the FP64 ones run only when energies were computed.
+ * (One CTA of 1,024 threads with warp-shuffle sums: 378 units with energies 10.5 us, 6,804 units 7.3 us,
+ * 149k units 29 us, the 512-replica batch 142 us; now 3, 3, 4 and 8.) */
+constexpr int kTotThreads = 256, kTotBlocks = 128;
+struct TotPart {
+    double e[4];                     /* LJ, Coulomb, virial, kinetic */
+    unsigned long long u[2];         /* pairs, below the table */
+};
+struct TotScratch {
+    TotPart part[kTotBlocks];
+    unsigned done;                   /* CTAs finished; 0 between launches */
+};
+inline int tot_blocks(int nunits, int nke) {
+    const int b = ((nunits > nke ? nunits : nke) + kTotThreads - 1) / kTotThreads;
+    return b < 1 ? 1 : (b > kTotBlocks ? kTotBlocks : b);
+}
+
+__device__ __forceinline__ void tot_tree(TotPart *s, int n, bool fp) {
+    for (int o = kTotThreads / 2; o > 0; o >>= 1) {
+        if (o < n && (int)threadIdx.x < o) {     /* entries from n on are zero */
+            TotPart &a = s[threadIdx.x];
+            const TotPart &b = s[threadIdx.x + o];
+            if (fp) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a.e[k] += b.e[k];
+            }
+            a.u[0] += b.u[0];
+            a.u[1] += b.u[1];
         }
+        __syncthreads();
     }
-#pragma unroll 8
-    for (int u = t; u < nke; u += 1024) k += kepart[u];
+}
+
+static __global__ void __launch_bounds__(kTotThreads) k_totals(int nunits, const UnitOut *__restrict__ uout,
+                                                               int nke, const double *__restrict__ kepart,
+                                                               DevTotals *tot, int with_energy, TotScratch *scr) {
+    __shared__ TotPart s[kTotThreads];
+    __shared__ unsigned s_last;
+    const int t = threadIdx.x, stride = gridDim.x * kTotThreads;
     const bool fp = with_energy || nke > 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        p += __shfl_xor_sync(0xffffffffu, p, o);
-        q += __shfl_xor_sync(0xffffffffu, q, o);
-        if (fp) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
-            c += __shfl_xor_sync(0xffffffffu, c, o);
-            k += __shfl_xor_sync(0xffffffffu, k, o);
+    TotPart a{};
+#pragma unroll 4
+    for (int u = blockIdx.x * kTotThreads + t; u < nunits; u += stride) {
+        a.u[0] += uout[u].pairs;
+        if (with_energy) {
+            a.e[0] += uout[u].e_lj; a.e[1] += uout[u].e_coul; a.e[2] += uout[u].virial;
+            a.u[1] += uout[u].below;
         }
     }
-    if (lane == 0) { s_d[w][0] = a; s_d[w][1] = b; s_d[w][2] = c; s_d[w][3] = k; s_u[w][0] = p; s_u[w][1] = q; }
+#pragma unroll 4
+    for (int u = blockIdx.x * kTotThreads + t; u < nke; u += stride) a.e[3] += kepart[u];
+    s[t] = a;
     __syncthreads();
-    if (w != 0) return;
-    a = s_d[lane][0]; b = s_d[lane][1]; c = s_d[lane][2]; k = s_d[lane][3];
-    p = s_u[lane][0]; q = s_u[lane][1];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        p += __shfl_xor_sync(0xffffffffu, p, o);
-        q += __shfl_xor_sync(0xffffffffu, q, o);
-        if (fp) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
-            c += __shfl_xor_sync(0xffffffffu, c, o);
-            k += __shfl_xor_sync(0xffffffffu, k, o);
+    tot_tree(s, min(kTotThreads, (nunits > nke ? nunits : nke) - (int)blockIdx.x * kTotThreads), fp);
+    if (gridDim.x > 1) {
+        if (t == 0) {
+            scr->part[blockIdx.x] = s[0];
+            __threadfence();
+            s_last = atomicAdd(&scr->done, 1u) == gridDim.x - 1;
         }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        s[t] = t < (int)gridDim.x ? scr->part[t] : TotPart{};
+        if (t == 0) scr->done = 0;
+        __syncthreads();
+        tot_tree(s, gridDim.x, fp);
     }
-    if (lane == 0) {
-        tot->e_lj = a; tot->e_coul = b; tot->virial = c;
+    if (t == 0) {
+        tot->e_lj = s[0].e[0]; tot->e_coul = s[0].e[1]; tot->virial = s[0].e[2];
         tot->e_bond = tot->e_angle = tot->e_dihedral = 0.0;   /* the bonded kernel adds its own */
-        if (nke > 0) tot->kinetic = k;
-        tot->pairs = p; tot->below = q;
-        tot->pairs_total += p;
+        if (nke > 0) tot->kinetic = s[0].e[3];
+        tot->pairs = s[0].u[0]; tot->below = s[0].u[1];
+        tot->pairs_total += s[0].u[0];
     }
 }
 
