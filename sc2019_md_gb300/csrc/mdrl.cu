@@ -203,8 +203,7 @@ static mdrl_status check_cells(mdrl_ctx *c) {
 mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
     const int nidx = c->nseg * c->bins;
     const int nc = c->order + 1;
-    dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_fp2); dfree(&c->d_fc2);
-    dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
+    dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     auto coef = [&](int f, int k, int idx) { return c->tab[((size_t)f * nc + k) * nidx + idx]; };
     if (c->order == 1) {
         std::vector<float2> f2((size_t)3 * nidx), e2((size_t)3 * nidx);
@@ -240,26 +239,20 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
                 e4[(size_t)3 * i + f] = make_float4(b[0], b[1], b[2], b[3]);
             }
         if (nc == 3) {
-            /* order 2 packed without padding for the one-warp-per-item kernel (36 bytes per index) */
-            std::vector<float4> fp2((size_t)2 * nidx), wa(nidx), wb(nidx);
-            std::vector<float> fc2((size_t)nidx);
+            /* order 2 without padding (36 bytes per index) for the one-warp-per-item and list kernels */
+            std::vector<float4> wa(nidx), wb(nidx);
+            std::vector<float> w1(nidx);
             for (int i = 0; i < nidx; ++i) {
                 wa[i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(0, 2, i), coef(1, 0, i));
                 wb[i] = make_float4(coef(1, 1, i), coef(1, 2, i), coef(2, 0, i), coef(2, 1, i));
-                fp2[(size_t)2 * i] = make_float4(coef(0, 0, i), coef(0, 1, i), coef(0, 2, i), coef(1, 0, i));
-                fp2[(size_t)2 * i + 1] = make_float4(coef(1, 1, i), coef(1, 2, i), coef(2, 0, i), coef(2, 1, i));
-                fc2[i] = coef(2, 2, i);
+                w1[i] = coef(2, 2, i);
             }
             MDRL_TRY(dalloc(&c->d_wa, wa.size()));
             MDRL_TRY(dalloc(&c->d_wb, wb.size()));
-            MDRL_TRY(dalloc(&c->d_w1, fc2.size()));
+            MDRL_TRY(dalloc(&c->d_w1, w1.size()));
             MDRL_CUDA(cudaMemcpy(c->d_wa, wa.data(), sizeof(float4) * wa.size(), cudaMemcpyHostToDevice));
             MDRL_CUDA(cudaMemcpy(c->d_wb, wb.data(), sizeof(float4) * wb.size(), cudaMemcpyHostToDevice));
-            MDRL_CUDA(cudaMemcpy(c->d_w1, fc2.data(), sizeof(float) * fc2.size(), cudaMemcpyHostToDevice));
-            MDRL_TRY(dalloc(&c->d_fp2, fp2.size()));
-            MDRL_TRY(dalloc(&c->d_fc2, fc2.size()));
-            MDRL_CUDA(cudaMemcpy(c->d_fp2, fp2.data(), sizeof(float4) * fp2.size(), cudaMemcpyHostToDevice));
-            MDRL_CUDA(cudaMemcpy(c->d_fc2, fc2.data(), sizeof(float) * fc2.size(), cudaMemcpyHostToDevice));
+            MDRL_CUDA(cudaMemcpy(c->d_w1, w1.data(), sizeof(float) * w1.size(), cudaMemcpyHostToDevice));
         }
         MDRL_TRY(dalloc(&c->d_f4, f4.size()));
         MDRL_TRY(dalloc(&c->d_e4, e4.size()));
@@ -282,7 +275,7 @@ mdrl_status mdrl::upload_tables(mdrl_ctx *c) {
 
 TableDev mdrl::table_dev(const mdrl_ctx *c) {
     TableDev t;
-    t.f2 = c->d_f2; t.e2 = c->d_e2; t.f4 = c->d_f4; t.e4 = c->d_e4; t.fr = c->d_fr; t.fp2 = c->d_fp2; t.fc2 = c->d_fc2;
+    t.f2 = c->d_f2; t.e2 = c->d_e2; t.f4 = c->d_f4; t.e4 = c->d_e4; t.fr = c->d_fr;
     t.wa = c->d_wa; t.wb = c->d_wb; t.wc = c->d_wc; t.w1 = c->d_w1;
     t.order = c->order; t.nseg = c->nseg; t.bins = c->bins; t.lb = ilog2i(c->bins);
     t.min_log2 = c->min_log2;
@@ -384,8 +377,7 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     pme_free(c);
     bonded_free(c);
     free_particles(c);
-    dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_fp2); dfree(&c->d_fc2);
-    dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
+    dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     dfree(&c->d_pcoef);
     dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work);
     dfree(&c->d_tot); dfree(&c->d_totscr); dfree(&c->d_err); dfree(&c->d_mt);
@@ -548,8 +540,9 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
     if (c->tile.warps_per_cta == 1) {
         /* one warp per (unit, i-tile group); fixed point only (set_tile checks) */
         const bool exact = (c->p.flags & MDRL_FLAG_EXACT_DIFF) != 0;
-        warp_fn fn = exact ? pick_force_warp_set<0, kDiffExact>(eff_order(c), false, extra)
-                           : pick_force_warp_set<0, kDiffShift>(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE, extra);
+        warp_fn fn = exact ? pick_force_warp_set<0, kDiffExact>(eff_order(c), false, extra, c->ke != 0.0f)
+                           : pick_force_warp_set<0, kDiffShift>(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE, extra,
+                                                              c->ke != 0.0f);
         MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
         const int items = force_slots(c, units);
         const size_t smem = force_warp_smem_bytes(c->p.ntypes, extra);

@@ -487,8 +487,8 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
          * other small replicas (per-pair wrap), then the half-shell units */
         const bool sep = c->p.arith == MDRL_ARITH_SEPARATE;
         force_fn fo = pick_force_batch(eff_order(c), sep, extra, false);
-        warp_fn fp = pick_force_warp_batch(eff_order(c), sep, extra, true);
-        warp_fn fw = pick_force_warp_batch(eff_order(c), sep, extra, false);
+        warp_fn fp = pick_force_warp_batch(eff_order(c), sep, extra, c->ke != 0.0f, true);
+        warp_fn fw = pick_force_warp_batch(eff_order(c), sep, extra, c->ke != 0.0f, false);
         MDRL_TRY(prepare_force_kernel(fo, c->p.device));
         MDRL_TRY(prepare_force_kernel((force_fn)fp, c->p.device));
         MDRL_TRY(prepare_force_kernel((force_fn)fw, c->p.device));

@@ -50,22 +50,40 @@ constexpr int kMaxItemGroups = 4;             /* i-tile groups per unit */
 /* Half-shell offsets in launch order: self, faces, edges, corners (indices into c_halfshell). */
 __constant__ int c_unit_order[kHalfShellCells] = {0, 1, 3, 9, 2, 4, 6, 8, 10, 12, 5, 7, 11, 13};
 
-/* pair_functions_fast with the order-2 force coefficients read from the packed rows (36 bytes per
- * index instead of 48: a smaller L1 footprint); the same values and arithmetic. */
+/* pair_functions_fast with the force coefficients of orders 1 and 2 read from the split tables (24 and
+ * 36 bytes per index, in arrays whose elements spread over every bank group); the same values and
+ * arithmetic. */
 template <int ORDER, bool SEP, bool ENERGY>
-__device__ __forceinline__ void pair_functions_packed(const TableDev &t, float r2, bool coul, float &v14,
-                                                      float &v8, float &v3, float &v12, float &v6, float &v1) {
-    if (ORDER != 2) {
+__device__ __forceinline__ void pair_functions_split(const TableDev &t, float r2, bool coul, float &v14,
+                                                     float &v8, float &v3, float &v12, float &v6, float &v1) {
+    if (ORDER != 2 && ORDER != 1) {
         pair_functions_fast<ORDER, SEP, ENERGY>(t, r2, coul, v14, v8, v3, v12, v6, v1);
         return;
     }
     const float r2e = fmaxf(r2, t.r2min);
-    const int idx = (int)(__float_as_uint(r2e) >> (23 - t.lb)) - ((127 + t.min_log2) << t.lb);
-    const float x = table_variable(t, r2e);
-    const float4 a = __ldg(t.fp2 + 2 * idx), b = __ldg(t.fp2 + 2 * idx + 1);
+    const unsigned bits = __float_as_uint(r2e);
+    const int idx = (int)(bits >> (23 - t.lb)) - ((127 + t.min_log2) << t.lb);
+    if (ORDER == 1) {
+        const float4 a = __ldg(t.wa + idx);
+        v14 = madd<SEP>(a.y, r2e, a.x);
+        v8 = madd<SEP>(a.w, r2e, a.z);
+        v3 = 0.0f;
+        if (coul) { const float2 c = __ldg(t.wc + idx); v3 = madd<SEP>(c.y, r2e, c.x); }
+        if (ENERGY) {
+            const float2 d = __ldg(t.e2 + 3 * idx), e = __ldg(t.e2 + 3 * idx + 1);
+            v12 = madd<SEP>(d.y, r2e, d.x);
+            v6 = madd<SEP>(e.y, r2e, e.x);
+            v1 = 0.0f;
+            if (coul) { const float2 f = __ldg(t.e2 + 3 * idx + 2); v1 = madd<SEP>(f.y, r2e, f.x); }
+        }
+        return;
+    }
+    /* table_variable without its branch: the mask is 0 in the monomial form */
+    const float x = __fsub_rn(r2e, __uint_as_float(bits & t.bmask));
+    const float4 a = __ldg(t.wa + idx), b = __ldg(t.wb + idx);
     v14 = madd<SEP>(madd<SEP>(a.z, x, a.y), x, a.x);
     v8 = madd<SEP>(madd<SEP>(b.y, x, b.x), x, a.w);
-    v3 = coul ? madd<SEP>(madd<SEP>(__ldg(t.fc2 + idx), x, b.w), x, b.z) : 0.0f;
+    v3 = coul ? madd<SEP>(madd<SEP>(__ldg(t.w1 + idx), x, b.w), x, b.z) : 0.0f;
     if (ENERGY) {
         v12 = poly4<ORDER, SEP>(__ldg(t.e4 + 3 * idx), x);
         v6 = poly4<ORDER, SEP>(__ldg(t.e4 + 3 * idx + 1), x);
@@ -89,7 +107,7 @@ typedef void (*warp_fn)(const float4 *, const int *, const int *, Geom, TableDev
 
 /* BATCH: the items are the half-shell units of a batch's replicas, items[b / G] (replica geometry
  * and cell offset from reps); otherwise every unit of one system, in launch order. */
-template <int ORDER, bool SEP, bool EXTRA, int ACC, int MODE, bool BATCH = false>
+template <int ORDER, bool SEP, bool EXTRA, int ACC, int MODE, bool COUL, bool BATCH = false>
 __global__ void __launch_bounds__(32, 16)
 k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, const int *__restrict__ cstart,
              Geom gparam, TableDev tab, const float4 *__restrict__ pcoef, int ntypes, float ke, int n,
@@ -109,7 +127,7 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
 
     const int lane = threadIdx.x, row = lane >> 3, col = lane & 7;
     const int G = tilecfg & 0xff;
-    const bool coul = ke != 0.0f;
+    constexpr bool coul = COUL;    /* ke != 0 */
     const float far = 1.0e18f;
 
     /* item -> (home cell, half-shell neighbour, group).  One system: unit class position first,
@@ -278,6 +296,10 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                 for (int t = 0; t < 24; ++t) fi[t] = 0.0f;
                 int ci[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 
+                /* inside one cell a pair is counted once (i < j) and two particles may coincide;
+                 * between cells neither can happen */
+                auto steps = [&](auto own) {
+                constexpr bool OWN = decltype(own)::value;
                 for (int p = 0; p < nsurv; ++p) {
                     const unsigned e = sList[p];
                     const int st = (int)(e & 31u);
@@ -285,7 +307,7 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                     const int jl = 8 * st + col;                        /* in the chunk */
                     const int jidx = j0 + jl;                           /* in the cell */
                     /* diagonal steps of the self unit need i < j per candidate */
-                    const int jthr = (self && j0 + 8 * st < i0 + 32) ? jidx : 0x7fffffff;
+                    const int jthr = (OWN && j0 + 8 * st < i0 + 32) ? jidx : 0x7fffffff;
                     float xj = -far, yj = -far, zj = -far, qj = 0.0f;
                     int ttj = 0;
                     if (jl < nj) {
@@ -303,10 +325,11 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                         const float dy = pair_diff<MODE>(yi[k], yj, g.L[1], g.h[1], sy);
                         const float dz = pair_diff<MODE>(zi[k], zj, g.L[2], g.h[2], sz);
                         const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-                        const bool ok = (r2 > 0.0f) && (r2 <= g.rc2) && (i0 + row + 4 * k < jthr);
+                        bool ok = r2 <= g.rc2;
+                        if (OWN) ok = ok && r2 > 0.0f && i0 + row + 4 * k < jthr;
                         if (ok) {
                             float v14, v8, v3, v12, v6, v1;
-                            pair_functions_packed<ORDER, SEP, EXTRA>(tab, r2, coul, v14, v8, v3, v12, v6, v1);
+                            pair_functions_split<ORDER, SEP, EXTRA>(tab, r2, coul, v14, v8, v3, v12, v6, v1);
                             const float2 pf = sCoefF[tti[k] + ttj];
                             const float4 pc = make_float4(pf.x, pf.y, 0.0f, 0.0f);
                             const float qq = __fmul_rn(qi[k], qj);
@@ -339,6 +362,9 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                         else if (EXTRA) sCj[jl] += cj;
                     }
                 }
+                };
+                if (self) steps(std::true_type{});
+                else steps(std::false_type{});
                 /* i forces: reduce-scatter over the columns, lane owns i = i0 + row + 4 col */
                 reduce_scatter24(fi, col);
                 int cnt_i = 0;
@@ -391,11 +417,11 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
 /* One set: every order x extra (x arithmetic mode for the reference's difference rule; the exact
  * rule is instantiated with fused arithmetic only). */
 template <int ACC, int DIFF>
-warp_fn pick_force_warp_set(int order, bool sep, bool extra) {
+warp_fn pick_force_warp_set(int order, bool sep, bool extra, bool coul) {
     auto w = [&](auto ord, auto sp, auto ex) -> warp_fn {
         constexpr int O = decltype(ord)::value;
         constexpr bool S = decltype(sp)::value, E = decltype(ex)::value;
-        return k_force_warp<O, S, E, ACC, DIFF>;
+        return coul ? (warp_fn)k_force_warp<O, S, E, ACC, DIFF, true> : (warp_fn)k_force_warp<O, S, E, ACC, DIFF, false>;
     };
     auto se = [&](auto ord) -> warp_fn {
         using T = std::true_type;
@@ -413,9 +439,9 @@ warp_fn pick_force_warp_set(int order, bool sep, bool extra) {
 
 /* the batched-replica sets: half-shell replicas (per-unit shift), and explicit cell pairs of
  * replicas with fewer than 3 cells per axis but every edge above 2 rc (per-pair wrap) */
-warp_fn pick_force_warp_batch(int order, bool sep, bool extra, bool cell_pairs);
+warp_fn pick_force_warp_batch(int order, bool sep, bool extra, bool coul, bool cell_pairs);
 
-extern template warp_fn pick_force_warp_set<0, kDiffShift>(int, bool, bool);
-extern template warp_fn pick_force_warp_set<0, kDiffExact>(int, bool, bool);
+extern template warp_fn pick_force_warp_set<0, kDiffShift>(int, bool, bool, bool);
+extern template warp_fn pick_force_warp_set<0, kDiffExact>(int, bool, bool, bool);
 
 }  // namespace mdrl

@@ -9,12 +9,15 @@
 
 namespace mdrl {
 
-warp_fn pick_force_warp_batch(int order, bool sep, bool extra, bool cell_pairs) {
+warp_fn pick_force_warp_batch(int order, bool sep, bool extra, bool coul, bool cell_pairs) {
     auto w = [&](auto ord, auto sp, auto ex) -> warp_fn {
         constexpr int O = decltype(ord)::value;
         constexpr bool S = decltype(sp)::value, E = decltype(ex)::value;
-        return cell_pairs ? (warp_fn)k_force_warp<O, S, E, 0, kDiffWrap, true>
-                          : (warp_fn)k_force_warp<O, S, E, 0, kDiffShift, true>;
+        if (cell_pairs)
+            return coul ? (warp_fn)k_force_warp<O, S, E, 0, kDiffWrap, true, true>
+                        : (warp_fn)k_force_warp<O, S, E, 0, kDiffWrap, false, true>;
+        return coul ? (warp_fn)k_force_warp<O, S, E, 0, kDiffShift, true, true>
+                    : (warp_fn)k_force_warp<O, S, E, 0, kDiffShift, false, true>;
     };
     auto se = [&](auto ord) -> warp_fn {
         using T = std::true_type;

@@ -38,10 +38,7 @@ struct TableDev {
     const float4 *f4, *e4;
     const float4 *fr;   /* order 1, force functions packed per index in one 32-byte sector:
                            {c0_14, c1_14, c0_8, c1_8}, {c0_3, c1_3, 0, 0} */
-    const float4 *fp2;  /* order 2, the force functions' 9 coefficients without padding: per index
-                           {c0_14, c1_14, c2_14, c0_8}, {c1_8, c2_8, c0_3, c1_3} ... */
-    const float *fc2;   /* ... and c2_3 */
-    /* the list kernel's copies of the force functions, split so that a gather's lanes spread over
+    /* the one-warp-per-item and list kernels' copies of the force functions, split so that a gather's lanes spread over
      * every 16-byte bank group: order 1 wa {c0_14, c1_14, c0_8, c1_8}, wc {c0_3, c1_3}; order 2 wa
      * {c0_14, c1_14, c2_14, c0_8}, wb {c1_8, c2_8, c0_3, c1_3}, w1 c2_3 */
     const float4 *wa, *wb;

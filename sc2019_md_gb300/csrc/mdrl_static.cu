@@ -310,8 +310,6 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     tab.f2 = (const float2 *)(b + kLayout.tabf); tab.e2 = (const float2 *)(b + kLayout.tabe);
     tab.f4 = (const float4 *)(b + kLayout.tabf); tab.e4 = (const float4 *)(b + kLayout.tabe);
     tab.fr = nullptr;    /* the rows of the other force kernels */
-    tab.fp2 = nullptr;
-    tab.fc2 = nullptr;
     tab.wa = (const float4 *)(b + kLayout.wa); tab.wb = (const float4 *)(b + kLayout.wb);
     tab.wc = (const float2 *)(b + kLayout.wc); tab.w1 = (const float *)(b + kLayout.wc);
     tab.order = order; tab.nseg = nseg; tab.bins = bins;
