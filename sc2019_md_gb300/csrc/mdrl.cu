@@ -520,7 +520,7 @@ static mdrl_status launch_list(mdrl_ctx *c, int n, const float4 *pos, const int 
     if (items > 0)    /* k_scan has zeroed the item counter */
         fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
             pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n, c->d_F64, c->d_cnt, c->d_unit,
-            ListBatch{}, nullptr, cfg, c->d_err, cell0, c->d_work, items);
+            ListBatch{}, nullptr, cfg, c->d_err, cell0, c->d_work, items, extra ? nullptr : c->d_tot);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
     *slots = items;
@@ -535,7 +535,7 @@ static int force_slots(const mdrl_ctx *c, int units) {
 
 /* The force launch over units [unit0, unit0 + units) (units < 0: every unit). */
 static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra,
-                                     unsigned long long *F64, float *F32, int unit0 = 0, int units = -1) {
+                                     unsigned long long *F64, float *F32, DevTotals *tot, int unit0 = 0, int units = -1) {
     if (units < 0) units = c->ncells * kHalfShellCells;
     if (c->tile.warps_per_cta == 1) {
         /* one warp per (unit, i-tile group); fixed point only (set_tile checks) */
@@ -555,7 +555,7 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
         if (items > 0)
             fn<<<grid, 32, smem, c->stream>>>(
                 pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n, F64, F32, c->d_cnt,
-                c->d_unit, nullptr, nullptr, c->tile.steps_per_piece, c->d_err, unit0, c->d_work, items);
+                c->d_unit, nullptr, nullptr, c->tile.steps_per_piece, c->d_err, unit0, c->d_work, items, tot);
         MDRL_CUDA(cudaGetLastError());
         MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
         return MDRL_OK;
@@ -571,18 +571,26 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
         fn<<<units, fw * 32, smem, c->stream>>>(pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef,
                                                  c->p.ntypes, c->ke, n, F64, F32, c->d_cnt, c->d_unit, nullptr,
                                                  nullptr, tile_word(c->tile.steps_per_piece, c->tile.prune_steps),
-                                                 c->d_err, unit0);
+                                                 c->d_err, unit0, tot);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
     return MDRL_OK;
 }
 
-static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra) {
-    return launch_force_into(c, n, pos, type, extra, c->d_F64, c->d_F32);
+/* tot (without energies): the totals that take the pair count */
+static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, DevTotals *tot) {
+    return launch_force_into(c, n, pos, type, extra, c->d_F64, c->d_F32, tot);
 }
 
 
 
+
+/* Whether the one-CTA binning takes the system.  Its ranking costs n times the mean occupancy on one
+ * SM: 1,728 atoms at 64 per cell take 15 us in all, as against 19 us and four more launches; at 4,096
+ * atoms with 150 per cell it would take longer than the general path. */
+static bool small_system(const mdrl_ctx *c, int n) {
+    return n > 0 && n <= kSmallN && c->ncells <= kSmallCells && (long long)n * n <= 160000LL * c->ncells;
+}
 
 /* Bin user-order arrays (already on the device) into the sorted buffers of slot `buf`.  With
  * `spatial` the cells are ordered by Morton key (the force path's order), otherwise by index
@@ -593,6 +601,15 @@ static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int
 static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, const float *z,
                             const float *q, const int *type, int buf, bool spatial, bool stage = false,
                             bool inv = false, bool hilbert = false) {
+    if (spatial && small_system(c, n)) {
+        MDRL_TRY(prepare_force_kernel((force_fn)k_small_user, c->p.device));
+        k_small_user<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
+            n, x, y, z, q, type, c->g, c->ncells, hilbert ? 1 : 0, c->d_pos[buf], c->d_type[buf], c->d_id[buf],
+            inv ? c->d_inv : nullptr, c->d_F64, c->d_F32, c->d_cnt, c->p.ntypes, c->d_start, c->d_tot, c->d_work,
+            c->d_err);
+        MDRL_CUDA(cudaGetLastError());
+        return MDRL_OK;
+    }
     MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * c->ncells, c->stream));
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     if (n > 0) {
@@ -700,11 +717,11 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     int slots = force_slots(c, force_items(c->ncells));
     MDRL_TRY(bin_user(c, n, x, y, z, q, type, 0, true, stage, true, list));
     if (list) MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], extra, 0, c->ncells, &slots));
-    else MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra));
+    else MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra, extra ? nullptr : c->d_tot));
     const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
     MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, energy));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, energy));
-    launch_totals(c, slots, 0, extra);
+    if (extra) launch_totals(c, slots, 0, true);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
     if (energy) MDRL_TRY(bonded_add_energy(c, n));
     if (out) populate(out->ptr, out->count, 4 * (size_t)n);
@@ -924,9 +941,8 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     if (list_eval(c))
         MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], false, hx0 * layer, cells, &slots));
     else
-        MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr,
+        MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr, c->d_tot,
                                    hx0 * layer * kHalfShellCells, cells * kHalfShellCells));
-    launch_totals(c, slots, 0, false);
     if (dF && pageable) populate((void *const *)&F, 1, 3 * sizeof(int64_t) * (size_t)n);
     if (n > 0) k_unsort_fixed<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_inv, c->d_F64, Fout);
     MDRL_CUDA(cudaGetLastError());
@@ -1144,6 +1160,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_CUDA(cudaSetDevice(c->p.device));
     MDRL_TRY(ensure_capacity(c, n));
     MDRL_TRY(bonded_check_atoms(c, n));
+    if (small_system(c, n)) MDRL_TRY(prepare_force_kernel((force_fn)k_small_state, c->p.device));
     const void *src[8] = {x, y, z, q, type, vx, vy, vz};
     void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 8, src, dst, false));
@@ -1153,7 +1170,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     k_gather_vel<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], vx ? c->d_ovx : nullptr, c->d_ovy,
                                                       c->d_ovz, c->d_vel[0]);
     const bool extra = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
-    MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra));
+    MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra, nullptr));
     MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, extra));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, extra));
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, c->d_F32, c->d_mt, 0,
@@ -1176,26 +1193,32 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
     const bool vv = c->p.integrator == MDRL_INT_VELOCITY_VERLET;
     const MassTab *mt = vv ? c->d_mt : c->d_mt + 1;
     const float dt = (float)c->p.dt_fs;
-    MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * c->ncells, c->stream));
-    k_kick_drift_bin<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_pos[a], c->d_vel[a], c->d_type[a], c->d_F64,
-                                                          c->d_F32, mt, dt, c->g, c->d_cell_of, c->d_slot,
-                                                          c->d_count, c->d_key);
-    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot);
-    k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
-    k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted, c->d_key, c->d_sortkey,
-                                                   c->d_err);
-    k_gather_state<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_sorted, c->d_pos[a], c->d_vel[a], c->d_type[a],
-                                                        c->d_id[a], c->d_pos[b], c->d_vel[b], c->d_type[b],
-                                                        c->d_id[b], c->d_F64, c->d_F32);
-    if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
-    MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra));
+    if (small_system(c, n)) {
+        k_small_state<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
+            n, c->d_pos[a], c->d_vel[a], c->d_type[a], c->d_id[a], mt, dt, c->g, c->ncells, c->d_pos[b], c->d_vel[b],
+            c->d_type[b], c->d_id[b], c->d_F64, c->d_F32, extra ? c->d_cnt : nullptr, c->d_start, c->d_tot, c->d_work);
+    } else {
+        MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * c->ncells, c->stream));
+        k_kick_drift_bin<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_pos[a], c->d_vel[a], c->d_type[a], c->d_F64,
+                                                              c->d_F32, mt, dt, c->g, c->d_cell_of, c->d_slot,
+                                                              c->d_count, c->d_key);
+        k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot);
+        k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
+        k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted, c->d_key, c->d_sortkey,
+                                                       c->d_err);
+        k_gather_state<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_sorted, c->d_pos[a], c->d_vel[a], c->d_type[a],
+                                                            c->d_id[a], c->d_pos[b], c->d_vel[b], c->d_type[b],
+                                                            c->d_id[b], c->d_F64, c->d_F32);
+        if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
+    }
+    MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra, extra ? nullptr : c->d_tot));
     MDRL_TRY(pme_enqueue(c, n, c->d_pos[b], c->d_F64, c->d_F32, extra));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[b], c->d_id[b], c->d_F64, c->d_F32, extra));
     /* kinetic energy only when energies are requested */
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[b], c->d_type[b], c->d_F64, c->d_F32, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    launch_totals(c, force_slots(c, force_items(c->ncells)), extra ? nblk(n, 256) : 0, extra);
+    if (extra) launch_totals(c, force_slots(c, force_items(c->ncells)), nblk(n, 256), true);
     if (extra) MDRL_TRY(pme_add_energy(c, n));
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());
@@ -1253,7 +1276,7 @@ extern "C" mdrl_status mdrl_time_force(mdrl_ctx *c, float *ms) {
     if (!fp32 && !c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
     if (fp32) MDRL_CUDA(cudaMemsetAsync(c->d_Fscr32, 0, sizeof(float) * 6 * (size_t)n, c->stream));
     else MDRL_CUDA(cudaMemsetAsync(c->d_Fscr64, 0, sizeof(unsigned long long) * 3 * (size_t)n, c->stream));
-    MDRL_TRY(launch_force_into(c, n, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, c->d_Fscr32));
+    MDRL_TRY(launch_force_into(c, n, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, c->d_Fscr32, nullptr));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_CUDA(cudaEventElapsedTime(ms, c->evf0, c->evf1));
     return MDRL_OK;

@@ -479,7 +479,7 @@ static int batch_slots(const mdrl_batch *b) {
 }
 
 static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const int *type, bool extra,
-                                      unsigned long long *F64) {
+                                      unsigned long long *F64, DevTotals *tot) {
     mdrl_ctx *c = b->c;
     if (c->tile.warps_per_cta == 1) {
         /* the replicas with an edge of at most 2 rc in the CTA kernel (every periodic image,
@@ -498,16 +498,16 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
         if (b->n_ot)
             fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
                 pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, F64, nullptr,
-                c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0);
+                c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0, tot);
         if (b->n_cp)
             fp<<<b->n_cp * G, 32, wsm, c->stream>>>(
                 pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, F64, nullptr,
-                c->d_cnt, c->d_unit + b->n_ot, b->d_items_hs, b->d_reps, G, c->d_err, 0, nullptr, 0);
+                c->d_cnt, c->d_unit + b->n_ot, b->d_items_hs, b->d_reps, G, c->d_err, 0, nullptr, 0, tot);
         if (b->n_hs)
             fw<<<b->n_hs * G, 32, wsm, c->stream>>>(
                 pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, F64, nullptr,
                 c->d_cnt, c->d_unit + b->n_ot + (size_t)b->n_cp * G, b->d_items_hs + b->n_cp, b->d_reps, G, c->d_err, 0,
-                nullptr, 0);
+                nullptr, 0, tot);
         MDRL_CUDA(cudaGetLastError());
         MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
         return MDRL_OK;
@@ -518,7 +518,7 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
     MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
     fn<<<b->nitems, kBatchFT, smem, c->stream>>>(pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef,
                                                   c->p.ntypes, c->ke, b->ntot, F64, nullptr, c->d_cnt, c->d_unit,
-                                                  b->d_items, b->d_reps, tile_word(c->tile.steps_per_piece, c->tile.prune_steps), c->d_err, 0);
+                                                  b->d_items, b->d_reps, tile_word(c->tile.steps_per_piece, c->tile.prune_steps), c->d_err, 0, tot);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
     return MDRL_OK;
@@ -538,13 +538,14 @@ static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int
     const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
     const int G = c->tile_set ? c->tile.steps_per_piece : 1;
     const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
+    DevTotals *tot = extra ? nullptr : c->d_tot;
     force_fn fo = pick_force_batch(eff_order(c), sep, extra, false);
     MDRL_TRY(prepare_force_kernel(fo, c->p.device));
     MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
     if (b->n_ot)
         fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
             pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, nullptr,
-            c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0);
+            c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0, tot);
     *slots = b->n_ot;
     for (int k = 0; k < 2; ++k) {
         bool fine;
@@ -559,7 +560,7 @@ static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int
         MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
         fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
             pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, c->d_cnt,
-            c->d_unit + *slots, b->lists[k].dev, b->d_reps, G, c->d_err, 0, c->d_work + k, items);
+            c->d_unit + *slots, b->lists[k].dev, b->d_reps, G, c->d_err, 0, c->d_work + k, items, tot);
         *slots += items;
     }
     MDRL_CUDA(cudaGetLastError());
@@ -637,9 +638,9 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     int slots = batch_slots(b);
     MDRL_TRY(batch_bin_user(b, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0, list));
     if (list) MDRL_TRY(batch_launch_list(b, c->d_pos[0], c->d_type[0], extra, &slots));
-    else MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
+    else MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64, extra ? nullptr : c->d_tot));
     b->list_slots = list;
-    launch_totals(c, slots, 0, extra);
+    if (extra) launch_totals(c, slots, 0, true);
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], c->d_F64, nullptr, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, counts ? c->d_ocnt : nullptr);
     MDRL_CUDA(cudaGetLastError());
@@ -673,7 +674,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     k_gather_vel<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], vx ? c->d_ovx : nullptr, c->d_ovy, c->d_ovz,
                                                       c->d_vel[0]);
     const bool extra = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
-    MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64));
+    MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64, nullptr));
     b->list_slots = false;
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, nullptr, c->d_mt, 0,
                                                 c->d_kepart);
@@ -706,11 +707,11 @@ static mdrl_status batch_enqueue_step(mdrl_batch *b, bool extra) {
                                                         c->d_id[a], c->d_pos[d], c->d_vel[d], c->d_type[d],
                                                         c->d_id[d], c->d_F64, nullptr);
     if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
-    MDRL_TRY(batch_launch_force(b, c->d_pos[d], c->d_type[d], extra, c->d_F64));
+    MDRL_TRY(batch_launch_force(b, c->d_pos[d], c->d_type[d], extra, c->d_F64, extra ? nullptr : c->d_tot));
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[d], c->d_type[d], c->d_F64, nullptr, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    launch_totals(c, batch_slots(b), extra ? nblk(n, 256) : 0, extra);
+    if (extra) launch_totals(c, batch_slots(b), nblk(n, 256), true);
     MDRL_CUDA(cudaGetLastError());
     return MDRL_OK;
 }
@@ -837,7 +838,7 @@ extern "C" mdrl_status mdrl_batch_time_force(mdrl_batch *b, float *ms) {
     const int a = c->cur;
     if (!c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
     MDRL_CUDA(cudaMemsetAsync(c->d_Fscr64, 0, sizeof(unsigned long long) * 3 * (size_t)b->ntot, c->stream));
-    MDRL_TRY(batch_launch_force(b, c->d_pos[a], c->d_type[a], false, c->d_Fscr64));
+    MDRL_TRY(batch_launch_force(b, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, nullptr));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_CUDA(cudaEventElapsedTime(ms, c->evf0, c->evf1));
     return MDRL_OK;

@@ -66,7 +66,7 @@ struct BatchRep;
 struct BatchItem;
 typedef void (*force_fn)(const float4 *, const int *, const int *, Geom, TableDev, const float4 *,
                          int, float, int, unsigned long long *, float *, int *, UnitOut *,
-                         const BatchItem *, const BatchRep *, int, unsigned *, int);
+                         const BatchItem *, const BatchRep *, int, unsigned *, int, DevTotals *);
 
 /* Work items (one per unit): the result slots k_totals sums. */
 inline int force_items(int ncells) { return ncells * kHalfShellCells; }
@@ -344,6 +344,15 @@ __device__ __forceinline__ void all_images_body(const float4 *__restrict__ pos, 
     }
 }
 
+/* A launch without energies has no sums to order: its pair count goes straight to the totals (tot not
+ * null; zeroed by the binning), and no k_totals follows (5.7 us of a 92k step, 21 us of the 512-replica
+ * batch's). */
+__device__ __forceinline__ void add_pairs(DevTotals *tot, unsigned long long pairs) {
+    if (!tot || !pairs) return;
+    atomicAdd(&tot->pairs, pairs);
+    atomicAdd(&tot->pairs_total, pairs);
+}
+
 /* One unit: home-cell particles [hs, hs + ni_all) against neighbour-cell particles
  * [cs, cs + nj_all) (the same cell when self), with the pair-difference rule MODE (kDiff*); writes the unit's totals to uout[blockIdx.x]. */
 template <int ORDER, bool SEP, bool EXTRA, int ACC, int MODE, int FW, bool PRUNE>
@@ -355,7 +364,7 @@ __device__ __forceinline__ void force_unit(const float4 *__restrict__ pos, const
                                            int *__restrict__ counts, UnitOut *__restrict__ uout, float4 *sIp,
                                            float4 *sJp, float4 *sCoef, int *sIt, int *sJt, float *sF, int *sC,
                                            double (*s_red)[3], unsigned long long (*s_cnt)[2], int tilecfg,
-                                           unsigned *err) {
+                                           unsigned *err, DevTotals *tot) {
     const int spp = tilecfg & 0xff;               /* j-steps per piece */
     constexpr bool prune = PRUNE;                 /* survivor lists (below) */
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -677,6 +686,7 @@ __device__ __forceinline__ void force_unit(const float4 *__restrict__ pos, const
             u.pairs += s_cnt[w][0]; u.below += s_cnt[w][1];
         }
         uout[blockIdx.x] = u;
+        add_pairs(tot, u.pairs);
     }
 }
 
@@ -689,7 +699,7 @@ k_force(const float4 *__restrict__ pos, const int *__restrict__ ptype,
         int ntypes, float ke, int n, unsigned long long *__restrict__ F64,
         float *__restrict__ F32, int *__restrict__ counts, UnitOut *__restrict__ uout,
         const BatchItem *__restrict__ items, const BatchRep *__restrict__ reps, int tilecfg,
-        unsigned *__restrict__ err, int unit0) {
+        unsigned *__restrict__ err, int unit0, DevTotals *tot) {
     extern __shared__ float4 smem[];
     float4 *sIp = smem;
     float4 *sJp = sIp + kChunk;
@@ -740,6 +750,7 @@ k_force(const float4 *__restrict__ pos, const int *__restrict__ ptype,
                     u.pairs += s_cnt[w][0]; u.below += s_cnt[w][1];
                 }
                 uout[blockIdx.x] = u;
+                add_pairs(tot, u.pairs);
             }
             return;
         }
@@ -790,7 +801,7 @@ k_force(const float4 *__restrict__ pos, const int *__restrict__ ptype,
         return;
     }
 #define MDRL_UNIT_ARGS pos, ptype, hs, ni_all, cs, nj_all, self, g, sx, sy, sz, tab, pcoef, ntypes, ke, n, F64, F32, \
-                       counts, uout, sIp, sJp, sCoef, sIt, sJt, sF, sC, s_red, s_cnt, tilecfg, err
+                       counts, uout, sIp, sJp, sCoef, sIt, sJt, sF, sC, s_red, s_cnt, tilecfg, err, tot
     /* one unit body per kernel where the rule is fixed (a second body cost more in instruction
      * fetch than a skipped add saves); the batch picks per item */
     if (BATCH && use_wrap)

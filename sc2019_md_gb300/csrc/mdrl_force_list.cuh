@@ -211,7 +211,7 @@ struct ListBatch {
  * system).  work: the item counter, zero at launch. */
 typedef void (*list_fn)(const float4 *, const int *, const int *, Geom, TableDev, const float4 *, int, float, int,
                         unsigned long long *, int *, UnitOut *, ListBatch, const BatchRep *, int, unsigned *, int,
-                        int *, int);
+                        int *, int, DevTotals *);
 
 /* Warp-wide minimum and maximum of floats. */
 __device__ __forceinline__ float warp_min(float v) {
@@ -264,7 +264,7 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
              Geom gparam, TableDev tab, const float4 *__restrict__ pcoef, int ntypes, float ke, int n,
              unsigned long long *__restrict__ F64, int *__restrict__ counts, UnitOut *__restrict__ uout,
              ListBatch lb, const BatchRep *__restrict__ reps, int cfg, unsigned *__restrict__ err, int cell0,
-             int *__restrict__ work, int nitems) {
+             int *__restrict__ work, int nitems, DevTotals *tot) {
     constexpr bool kCellPair = BATCH && MODE == kDiffWrap;
     const int t2 = (ntypes * ntypes + 1) & ~1;
     extern __shared__ float4 wsm[];
@@ -283,6 +283,7 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
     const float far = 1.0e18f;
     const unsigned below = (1u << lane) - 1u;
 
+    unsigned long long pairs_sum = 0;    /* lane 0: the warp's items' */
     for (;;) {
         int b = 0;
         if (FINE) {
@@ -736,8 +737,10 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
             u.e_lj = e1; u.e_coul = e2; u.virial = e3;
             u.pairs = c1; u.below = c2;
             uout[b] = u;
+            pairs_sum += c1;
         }
     }
+    if (lane == 0) add_pairs(tot, pairs_sum);
 }
 
 /* One set: every order x extra x Coulomb x fine (x arithmetic mode for the reference's difference

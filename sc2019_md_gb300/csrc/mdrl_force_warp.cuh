@@ -103,7 +103,7 @@ inline size_t force_warp_smem_bytes(int ntypes, bool extra) {
  * launch) and item count (work == nullptr: one item per CTA, blockIdx.x). */
 typedef void (*warp_fn)(const float4 *, const int *, const int *, Geom, TableDev, const float4 *, int, float,
                         int, unsigned long long *, float *, int *, UnitOut *, const BatchItem *,
-                        const BatchRep *, int, unsigned *, int, int *, int);
+                        const BatchRep *, int, unsigned *, int, int *, int, DevTotals *);
 
 /* BATCH: the items are the half-shell units of a batch's replicas, items[b / G] (replica geometry
  * and cell offset from reps); otherwise every unit of one system, in launch order. */
@@ -113,7 +113,7 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
              Geom gparam, TableDev tab, const float4 *__restrict__ pcoef, int ntypes, float ke, int n,
              unsigned long long *__restrict__ F64, float *__restrict__ F32, int *__restrict__ counts,
              UnitOut *__restrict__ uout, const BatchItem *__restrict__ items, const BatchRep *__restrict__ reps,
-             int tilecfg, unsigned *__restrict__ err, int unit0, int *__restrict__ work, int nitems) {
+             int tilecfg, unsigned *__restrict__ err, int unit0, int *__restrict__ work, int nitems, DevTotals *tot) {
     constexpr int nst = kWarpJChunk / 8;                        /* steps per chunk */
     const int t2 = (ntypes * ntypes + 1) & ~1;
     extern __shared__ float4 wsm[];
@@ -405,6 +405,7 @@ k_force_warp(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         u.e_lj = e1; u.e_coul = e2; u.virial = e3;
         u.pairs = c1; u.below = c2;
         uout[b] = u;
+        add_pairs(tot, c1);
     }
     if (!work) break;
     __syncwarp();   /* this item's shared-memory reads are done before the next item writes */

@@ -346,8 +346,8 @@ static __global__ void k_bin_user(int n, const float *__restrict__ x, const floa
     slot[i] = cell_slot(count, c);
 }
 
-/* Exclusive scan of the cell counts (one CTA), plus the largest occupancy; zeroes the force launches'
- * item counters work[0..1] on the way (a memset less per evaluation).  Latency-bound: 4 counts per
+/* Exclusive scan of the cell counts (one CTA), plus the largest occupancy; zeroes the totals' counts and
+ * the force launches' item counters work[0..1] on the way (a memset less per evaluation).  Latency-bound: 4 counts per
  * thread and pass in one 16-byte load, warp scans by shuffles, one barrier per pass of 4,096 cells.
  * (A strided run of cells per thread and a 20-barrier scan: 486 cells 3.8 us, 10,648 cells 9.9 us, 28k
  * cells 53 us; now 2.2, 3.3 and 6.) */
@@ -356,6 +356,7 @@ static __global__ void __launch_bounds__(1024) k_scan(int ncells, const int *__r
     __shared__ int s_sum[2][32], s_max[32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (work && t < 2) work[t] = 0;
+    if (t == 0) tot->pairs = tot->below = 0ull;
     int carry = 0, mx = 0, pass = 0;
     for (int base = 0; base < ncells; base += 4096, pass ^= 1) {
         const int k = base + 4 * t;
@@ -529,7 +530,7 @@ struct TotScratch {
     unsigned done;                   /* CTAs finished; 0 between launches */
 };
 inline int tot_blocks(int nunits, int nke) {
-    const int b = ((nunits > nke ? nunits : nke) + kTotThreads - 1) / kTotThreads;
+    const int b = ((nunits > nke ? nunits : nke) + 4 * kTotThreads - 1) / (4 * kTotThreads);
     return b < 1 ? 1 : (b > kTotBlocks ? kTotBlocks : b);
 }
 
@@ -711,6 +712,196 @@ static __global__ void k_gather_state(int n, const int *__restrict__ sorted,
     if (F32) {
 #pragma unroll
         for (int d = 0; d < 6; ++d) F32[(size_t)d * n + k] = 0.0f;   /* hi planes 0-2, lo planes 3-5 */
+    }
+}
+
+/* ---- small systems ----------------------------------------------------------------------------
+ * Binning in one launch for systems of at most kSmallN particles and kSmallCells cells: one CTA bins,
+ * scans, sorts and gathers, with the counts and keys in shared memory, where the general path takes
+ * five launches of ~3.5 us each that do almost nothing (1,728 atoms: 18 -> 8 us per step).  The order
+ * is the general path's: by (key, index) inside a cell.  Larger systems need more than one SM. */
+constexpr int kSmallN = 4096, kSmallCells = 4096, kSmallThreads = 1024, kSmallPer = kSmallN / kSmallThreads;
+
+struct SmallShared {
+    int count[kSmallCells];                  /* occupancy, then the cell's start */
+    unsigned long long key[kSmallN];         /* (key, index), cell by cell */
+    unsigned short cell[kSmallN];            /* the cell of each entry */
+    unsigned short at[kSmallN];              /* cell-order position by index */
+    int warp_sum[kSmallThreads / 32], warp_max[kSmallThreads / 32];
+};
+
+/* Cell-order position of each of the thread's particles (index threadIdx.x + p * kSmallThreads, cell[p],
+ * key[p]); fills start[] and tot->max_occ. */
+__device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, const int (&cell)[kSmallPer],
+                                           const unsigned (&key)[kSmallPer], int (&at)[kSmallPer],
+                                           int *__restrict__ start, DevTotals *tot) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int k = t; k < ncells; k += kSmallThreads) s.count[k] = 0;
+    __syncthreads();
+    int slot[kSmallPer];
+#pragma unroll
+    for (int p = 0; p < kSmallPer; ++p)
+        if (t + p * kSmallThreads < n) slot[p] = atomicAdd(&s.count[cell[p]], 1);
+    __syncthreads();
+    /* exclusive scan, 4 cells per thread */
+    int c[4], own = 0, mx = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        c[k] = 4 * t + k < ncells ? s.count[4 * t + k] : 0;
+        own += c[k];
+        mx = max(mx, c[k]);
+    }
+    int sum = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 31) { s.warp_sum[warp] = sum; s.warp_max[warp] = mx; }
+    __syncthreads();
+    int ws = s.warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += v;
+    }
+    const int before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
+    int first = (warp ? before : 0) + sum - own;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if (4 * t + k < ncells) { s.count[4 * t + k] = first; start[4 * t + k] = first; }
+        first += c[k];
+    }
+    mx = __reduce_max_sync(0xffffffffu, s.warp_max[lane]);
+    if (t == 0) { start[ncells] = n; tot->max_occ = mx; tot->pairs = tot->below = 0ull; }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < kSmallPer; ++p) {
+        const int i = t + p * kSmallThreads;
+        if (i < n) {
+            const int e = s.count[cell[p]] + slot[p];
+            s.key[e] = ((unsigned long long)key[p] << 32) | (unsigned)i;
+            s.cell[e] = (unsigned short)cell[p];
+        }
+    }
+    __syncthreads();
+    /* rank of an entry = the smaller ones of its cell.  By entry, not by particle: neighbouring lanes
+     * then walk the same cell, and a load serves them all (by particle, 64 per cell: 52 us) */
+#pragma unroll
+    for (int p = 0; p < kSmallPer; ++p) {
+        const int e = t + p * kSmallThreads;
+        if (e >= n) continue;
+        const unsigned long long me = s.key[e];
+        const int cl = s.cell[e], a = s.count[cl], b = cl + 1 < ncells ? s.count[cl + 1] : n;
+        int rank = 0;
+#pragma unroll 4
+        for (int q = a; q < b; ++q) rank += s.key[q] < me;
+        s.at[(unsigned)me] = (unsigned short)(a + rank);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < kSmallPer; ++p)
+        if (t + p * kSmallThreads < n) at[p] = s.at[t + p * kSmallThreads];
+}
+
+__device__ __forceinline__ void clear_force(int n, int k, unsigned long long *F64, float *F32, int *counts) {
+    if (F64) { F64[k] = 0ull; F64[n + k] = 0ull; F64[2 * n + k] = 0ull; }
+    if (F32) {
+#pragma unroll
+        for (int d = 0; d < 6; ++d) F32[(size_t)d * n + k] = 0.0f;   /* hi planes 0-2, lo planes 3-5 */
+    }
+    if (counts) counts[k] = 0;
+}
+
+/* User-order inputs (device memory, or host memory the device reads) into cell order: k_bin_user, k_scan,
+ * k_scatter, k_cell_sort and k_gather_user in one.  Also clears the error word and the item counters. */
+static __global__ void __launch_bounds__(kSmallThreads)
+k_small_user(int n, const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+             const float *__restrict__ q, const int *__restrict__ type, Geom g, int ncells, int hilbert,
+             float4 *__restrict__ pos, int *__restrict__ ptype, int *__restrict__ pid, int *__restrict__ inv,
+             unsigned long long *__restrict__ F64, float *__restrict__ F32, int *__restrict__ counts, int ntypes,
+             int *__restrict__ start, DevTotals *tot, int *__restrict__ work, unsigned *__restrict__ err) {
+    extern __shared__ float4 small_sm[];
+    SmallShared &s = *reinterpret_cast<SmallShared *>(small_sm);
+    __shared__ unsigned s_err;
+    if (threadIdx.x == 0) s_err = 0u;
+    if (threadIdx.x < 2) work[threadIdx.x] = 0;
+    __syncthreads();
+    float4 p[kSmallPer];
+    int ty[kSmallPer], cell[kSmallPer], at[kSmallPer];
+    unsigned key[kSmallPer];
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+        const int i = threadIdx.x + k * kSmallThreads;
+        if (i >= n) continue;
+        p[k] = make_float4(x[i], y[i], z[i], q ? q[i] : 0.0f);
+        ty[k] = type ? type[i] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+        const int i = threadIdx.x + k * kSmallThreads;
+        if (i >= n) continue;
+        if (!in_box(g, p[k].x, p[k].y, p[k].z)) atomicOr(&s_err, kErrPosition);
+        if (ty[k] < 0 || ty[k] >= ntypes) { atomicOr(&s_err, kErrType); ty[k] = 0; }
+        cell[k] = cell_of_pos(g, p[k].x, p[k].y, p[k].z);
+        key[k] = hilbert ? cell_hilbert(g, p[k].x, p[k].y, p[k].z, cell[k]) : cell_morton(g, p[k].x, p[k].y, p[k].z, cell[k]);
+    }
+    small_sort(s, n, ncells, cell, key, at, start, tot);
+#pragma unroll
+    for (int k = 0; k < kSmallPer; ++k) {
+        const int i = threadIdx.x + k * kSmallThreads;
+        if (i >= n) continue;
+        pos[at[k]] = p[k];
+        ptype[at[k]] = ty[k];
+        pid[at[k]] = i;
+        if (inv) inv[i] = at[k];
+        clear_force(n, i, F64, F32, counts);
+    }
+    if (threadIdx.x == 0) *err = s_err;
+}
+
+/* One step's first kick, drift and re-binning of the state: k_kick_drift_bin, k_scan, k_scatter,
+ * k_cell_sort and k_gather_state in one. */
+static __global__ void __launch_bounds__(kSmallThreads)
+k_small_state(int n, const float4 *__restrict__ pos0, const float4 *__restrict__ vel0, const int *__restrict__ type0,
+              const int *__restrict__ id0, const MassTab *__restrict__ mt, float dt, Geom g, int ncells,
+              float4 *__restrict__ pos1, float4 *__restrict__ vel1, int *__restrict__ type1, int *__restrict__ id1,
+              unsigned long long *F64, float *F32, int *__restrict__ counts, int *__restrict__ start, DevTotals *tot,
+              int *__restrict__ work) {
+    extern __shared__ float4 small_sm[];
+    SmallShared &s = *reinterpret_cast<SmallShared *>(small_sm);
+    if (threadIdx.x < 2) work[threadIdx.x] = 0;
+    float4 p[kSmallPer], v[kSmallPer];
+    int ty[kSmallPer], id[kSmallPer], cell[kSmallPer], at[kSmallPer];
+    unsigned key[kSmallPer];
+#pragma unroll
+    for (int q = 0; q < kSmallPer; ++q) {
+        const int k = threadIdx.x + q * kSmallThreads;
+        if (k >= n) continue;
+        ty[q] = type0[k];
+        id[q] = id0[k];
+        v[q] = vel0[k];
+        p[q] = pos0[k];
+        const float cm = mt->cm[ty[q]];
+        v[q].x = __fmaf_rn(force_of(F64, F32, n, k, 0), cm, v[q].x);
+        v[q].y = __fmaf_rn(force_of(F64, F32, n, k, 1), cm, v[q].y);
+        v[q].z = __fmaf_rn(force_of(F64, F32, n, k, 2), cm, v[q].z);
+        p[q].x = wrap_pos(__fmaf_rn(v[q].x, dt, p[q].x), g.L[0]);
+        p[q].y = wrap_pos(__fmaf_rn(v[q].y, dt, p[q].y), g.L[1]);
+        p[q].z = wrap_pos(__fmaf_rn(v[q].z, dt, p[q].z), g.L[2]);
+        cell[q] = cell_of_pos(g, p[q].x, p[q].y, p[q].z);
+        key[q] = cell_morton(g, p[q].x, p[q].y, p[q].z, cell[q]);
+        clear_force(n, k, F64, F32, counts);     /* the thread's own entries, read above */
+    }
+    small_sort(s, n, ncells, cell, key, at, start, tot);
+#pragma unroll
+    for (int q = 0; q < kSmallPer; ++q) {
+        if ((int)threadIdx.x + q * kSmallThreads >= n) continue;
+        pos1[at[q]] = p[q];
+        vel1[at[q]] = v[q];
+        type1[at[q]] = ty[q];
+        id1[at[q]] = id[q];
     }
 }
 

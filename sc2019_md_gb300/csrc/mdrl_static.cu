@@ -56,7 +56,7 @@ constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 /* Byte offsets of the sub-buffers inside the array. */
 struct Layout {
-    size_t err, tot, scr, count, start, unit, cell_of, slot, tmp, sorted, key, sortkey, pos, type, id, F64, tabf,
+    size_t err, tot, count, start, unit, cell_of, slot, tmp, sorted, key, sortkey, pos, type, id, F64, tabf,
         tabe, wa, wb, wc, pcoef, work, end;
 };
 
@@ -65,7 +65,6 @@ constexpr Layout make_layout() {
     size_t o = 0;
     l.err = o;     o = align256(o + sizeof(unsigned));
     l.tot = o;     o = align256(o + sizeof(DevTotals));
-    l.scr = o;     o = align256(o + sizeof(TotScratch));
     l.count = o;   o = align256(o + sizeof(int) * kStaticMaxCells);
     l.start = o;   o = align256(o + sizeof(int) * (kStaticMaxCells + 1));
     l.unit = o;    o = align256(o + sizeof(UnitOut) * kHalfShellCells * kStaticMaxCells);
@@ -322,7 +321,7 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     /* state that must start at zero; the previous call's contents are otherwise left in place */
     const int nc = (int)ncells;
     ST_CUDA(cudaMemsetAsync(d_err, 0, sizeof(unsigned), st));
-    ST_CUDA(cudaMemsetAsync(d_tot, 0, kLayout.scr + sizeof(TotScratch) - kLayout.tot, st));   /* and k_totals' scratch */
+    ST_CUDA(cudaMemsetAsync(d_tot, 0, sizeof(DevTotals), st));
     ST_CUDA(cudaMemsetAsync(d_count, 0, sizeof(int) * nc, st));
     const int blk = 256, grid = (n + blk - 1) / blk;
     if (n > 0) k_bin_user<<<grid, blk, 0, st>>>(n, x, y, z, g, d_cell_of, d_slot, d_count, d_err, d_key, nullptr,
@@ -351,9 +350,7 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     ctas = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta, std::max(1, per_sm) * std::max(1, sms));
     fn<<<ctas, 32 * kWarpsPerCta, smem, st>>>(d_pos, d_type, d_start, g, tab, d_pcoef, p->ntypes, (float)p->coulomb_k, n,
                                               d_F64, nullptr, d_unit, ListBatch{}, nullptr, cfg, d_err, 0,
-                                              (int *)(b + kLayout.work), items);
-    k_totals<<<tot_blocks(items, 0), kTotThreads, 0, st>>>(items, d_unit, 0, nullptr, d_tot, 0,
-                                                           (TotScratch *)(b + kLayout.scr));
+                                              (int *)(b + kLayout.work), items, d_tot);
     if (n > 0)
         k_unsort<<<grid, blk, 0, st>>>(n, d_id, d_F64, nullptr, nullptr, fx, fy, fz, nullptr);
     ST_CUDA(cudaGetLastError());
