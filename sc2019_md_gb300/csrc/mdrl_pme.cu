@@ -94,59 +94,77 @@ struct PmeGeom {
 
 __device__ __forceinline__ int wrapk(int k, int K) { return k < 0 ? k + K : (k >= K ? k - K : k); }
 
+/* Spreading, P^2 lanes (16 or 36, the latter as a whole warp twice over) per particle: lane (j1, j2) adds
+ * the P grid points (j0, j1, j2) of its column.  Bound by the atomics: a thread per particle makes every
+ * instruction touch 32 unrelated sectors, P^3 of them per particle; here the P lanes of a j1 row write
+ * consecutive points, so an instruction's atomics fall into 1 or 2 sectors per row (92k particles,
+ * order 4: 28 us before).  The weights of an axis are computed by the lanes of one row and handed out
+ * by shuffles; each product is formed in the order q th0 th1 th2 as before, and the integer sums are
+ * exact, so the grid is the same bit for bit. */
 template <int P>
-__global__ void k_pme_spread(int n, const float4 *__restrict__ pos, PmeGeom pg,
-                             unsigned long long *__restrict__ qfix, double *__restrict__ qpart) {
+__global__ void __launch_bounds__(256) k_pme_spread(int n, const float4 *__restrict__ pos, PmeGeom pg,
+                                                    unsigned long long *__restrict__ qfix) {
+    constexpr int L = P == 4 ? 16 : 32;            /* lanes per particle */
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / L, l = threadIdx.x % L;
+    const unsigned mask = L == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);
+    if (i >= n) return;                            /* uniform over a particle's lanes */
+    const float4 r = pos[i];
+    const float q = r.w;
+    if (q == 0.0f) return;
+    /* lane a P + j (a < 3): the weight th_a[j] and its grid index */
+    float w = 0.0f;
+    int k = 0;
+    {
+        const int a = l / P, j = l % P;
+        const float x = a == 0 ? r.x : (a == 1 ? r.y : r.z), sc = a == 0 ? pg.scale[0] : (a == 1 ? pg.scale[1] : pg.scale[2]);
+        const int K = a == 0 ? pg.K[0] : (a == 1 ? pg.K[1] : pg.K[2]);
+        float th[P], dth[P];
+        const float u = x * sc;
+        const float fl = floorf(u);
+        /* positions outside [0, L) are reported by the binning; keep the grid index in range whatever
+         * the input (k0 - j stays in [-P, K]) */
+        const int k0 = min(max((int)fl, 0), K);
+        bspline<P>(fminf(fmaxf(u - fl, 0.0f), 1.0f), th, dth);
+#pragma unroll
+        for (int m = 0; m < P; ++m)
+            if (j == m) w = th[m];
+        k = wrapk(k0 - j, K);
+    }
+    float w0[P];
+    int g0[P];
+#pragma unroll
+    for (int j0 = 0; j0 < P; ++j0) {
+        w0[j0] = q * __shfl_sync(mask, w, j0, L);
+        g0[j0] = __shfl_sync(mask, k, j0, L) * pg.K[1];
+    }
+    for (int c = l; c < ((P * P + L - 1) / L) * L; c += L) {      /* columns (j1, j2) */
+        const int j1 = (c / P) % P, j2 = c % P;
+        const float w1 = __shfl_sync(mask, w, P + j1, L), w2 = __shfl_sync(mask, w, 2 * P + j2, L);
+        const int k1 = __shfl_sync(mask, k, P + j1, L), k2 = __shfl_sync(mask, k, 2 * P + j2, L);
+        if (c >= P * P) continue;
+#pragma unroll
+        for (int j0 = 0; j0 < P; ++j0) {
+            const float v = (w0[j0] * w1) * w2;
+            /* v 2^40 is exact in FP32 (a power-of-two scale), so rounding it to an integer gives the
+             * same value as the same product in FP64 would, without FP64 arithmetic (slow on this part) */
+            atomicAdd(qfix + (size_t)(g0[j0] + k1) * pg.K[2] + k2, (unsigned long long)__float2ll_rn(v * kPmeFix));
+        }
+    }
+}
+
+/* Sums of q and q^2 per CTA, in a fixed order (energies only). */
+__global__ void __launch_bounds__(256) k_pme_charge(int n, const float4 *__restrict__ pos, double *__restrict__ qpart) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float q = 0.0f;
-    if (i < n) {
-        const float4 r = pos[i];
-        q = r.w;
-        if (q != 0.0f) {
-            float th[3][P], dth[P];
-            int k0[3];
-            const float rr[3] = {r.x, r.y, r.z};
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float u = rr[a] * pg.scale[a];
-                const float fl = floorf(u);
-                /* positions outside [0, L) are reported by the binning; keep the grid index in
-                 * range whatever the input (k0 - j stays in [-P, K]) */
-                k0[a] = min(max((int)fl, 0), pg.K[a]);
-                bspline<P>(fminf(fmaxf(u - fl, 0.0f), 1.0f), th[a], dth);
-            }
-#pragma unroll
-            for (int j0 = 0; j0 < P; ++j0) {
-                const int g0 = wrapk(k0[0] - j0, pg.K[0]) * pg.K[1];
-                const float q0 = q * th[0][j0];
-#pragma unroll
-                for (int j1 = 0; j1 < P; ++j1) {
-                    const int g1 = (g0 + wrapk(k0[1] - j1, pg.K[1])) * pg.K[2];
-                    const float q1 = q0 * th[1][j1];
-#pragma unroll
-                    for (int j2 = 0; j2 < P; ++j2) {
-                        const float v = q1 * th[2][j2];
-                        /* v 2^40 is exact in FP32 (a power-of-two scale), so rounding it to an
-                         * integer gives the same value as the same product in FP64 would, without
-                         * FP64 arithmetic (slow on this part) */
-                        atomicAdd(qfix + g1 + wrapk(k0[2] - j2, pg.K[2]),
-                                  (unsigned long long)__float2ll_rn(v * kPmeFix));
-                    }
-                }
-            }
-        }
-    }
-    if (qpart) {   /* sum q and sum q^2 of the block, fixed order */
-        __shared__ double s[2][256];
-        s[0][threadIdx.x] = q;
-        s[1][threadIdx.x] = (double)q * (double)q;
+    const float q = i < n ? pos[i].w : 0.0f;
+    __shared__ double s[2][256];
+    s[0][threadIdx.x] = q;
+    s[1][threadIdx.x] = (double)q * (double)q;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) { s[0][threadIdx.x] += s[0][threadIdx.x + o]; s[1][threadIdx.x] += s[1][threadIdx.x + o]; }
         __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) { s[0][threadIdx.x] += s[0][threadIdx.x + o]; s[1][threadIdx.x] += s[1][threadIdx.x + o]; }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) { qpart[2 * blockIdx.x] = s[0][0]; qpart[2 * blockIdx.x + 1] = s[1][0]; }
     }
+    if (threadIdx.x == 0) { qpart[2 * blockIdx.x] = s[0][0]; qpart[2 * blockIdx.x + 1] = s[1][0]; }
 }
 
 __global__ void k_pme_unfix(int nreal, const unsigned long long *__restrict__ qfix, float *__restrict__ real) {
@@ -409,9 +427,9 @@ mdrl_status pme_enqueue(mdrl_ctx *c, int n, const float4 *pos, unsigned long lon
         s->qblocks = qb;
     }
     MDRL_CUDA(cudaMemsetAsync(s->d_qfix, 0, sizeof(unsigned long long) * s->nreal, c->stream));
-    double *qpart = energy ? s->d_qpart : nullptr;
-    if (s->p.order == 6) k_pme_spread<6><<<qb, 256, 0, c->stream>>>(n, pos, pg, s->d_qfix, qpart);
-    else k_pme_spread<4><<<qb, 256, 0, c->stream>>>(n, pos, pg, s->d_qfix, qpart);
+    if (s->p.order == 6) k_pme_spread<6><<<nblk(n, 8), 256, 0, c->stream>>>(n, pos, pg, s->d_qfix);
+    else k_pme_spread<4><<<nblk(n, 16), 256, 0, c->stream>>>(n, pos, pg, s->d_qfix);
+    if (energy) k_pme_charge<<<qb, 256, 0, c->stream>>>(n, pos, s->d_qpart);
     const int gb = std::min(nblk(s->nreal, 256), 4 * std::max(1, c->num_sms));
     k_pme_unfix<<<gb, 256, 0, c->stream>>>(s->nreal, s->d_qfix, s->d_real);
     MDRL_CUDA(cudaGetLastError());
