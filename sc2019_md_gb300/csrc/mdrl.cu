@@ -716,10 +716,11 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     const bool list = list_eval(c);
     int slots = force_slots(c, force_items(c->ncells));
     MDRL_TRY(bin_user(c, n, x, y, z, q, type, 0, true, stage, true, list));
+    const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
+    MDRL_TRY(pme_begin(c, n, c->d_pos[0], energy));
     if (list) MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], extra, 0, c->ncells, &slots));
     else MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra, extra ? nullptr : c->d_tot));
-    const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
-    MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, energy));
+    MDRL_TRY(pme_finish(c, n, c->d_pos[0], c->d_F64, c->d_F32));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, energy));
     if (extra) launch_totals(c, slots, 0, true);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
@@ -1170,8 +1171,9 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     k_gather_vel<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], vx ? c->d_ovx : nullptr, c->d_ovy,
                                                       c->d_ovz, c->d_vel[0]);
     const bool extra = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
+    MDRL_TRY(pme_begin(c, n, c->d_pos[0], extra));
     MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra, nullptr));
-    MDRL_TRY(pme_enqueue(c, n, c->d_pos[0], c->d_F64, c->d_F32, extra));
+    MDRL_TRY(pme_finish(c, n, c->d_pos[0], c->d_F64, c->d_F32));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, extra));
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, c->d_F32, c->d_mt, 0,
                                                 c->d_kepart);
@@ -1211,8 +1213,9 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
                                                             c->d_id[b], c->d_F64, c->d_F32);
         if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
     }
+    MDRL_TRY(pme_begin(c, n, c->d_pos[b], extra));
     MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra, extra ? nullptr : c->d_tot));
-    MDRL_TRY(pme_enqueue(c, n, c->d_pos[b], c->d_F64, c->d_F32, extra));
+    MDRL_TRY(pme_finish(c, n, c->d_pos[b], c->d_F64, c->d_F32));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[b], c->d_id[b], c->d_F64, c->d_F32, extra));
     /* kinetic energy only when energies are requested */
     if (vv || extra)
@@ -1245,6 +1248,8 @@ extern "C" mdrl_status mdrl_step(mdrl_ctx *c, int nsteps, mdrl_stats *st) {
             cudaGraph_t g = nullptr;
             const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
             c->cur = saved;
+            /* a step that failed between PME's two halves ends the capture unjoined: not the next call's error */
+            if (e != cudaSuccess) (void)cudaGetLastError();
             if (s != MDRL_OK) { if (g) cudaGraphDestroy(g); return s; }
             if (e != cudaSuccess) { set_error(std::string("graph capture: ") + cudaGetErrorString(e)); return MDRL_ERR_CUDA; }
             c->graph[k] = g;

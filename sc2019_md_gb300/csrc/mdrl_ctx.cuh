@@ -156,7 +156,8 @@ inline int nblk(int n, int b) { return (n + b - 1) / b; }
 /* PME (mdrl_pme.cu): setup, teardown, the reciprocal part of a force evaluation, its energies. */
 mdrl_status pme_setup(mdrl_ctx *c, const mdrl_pme_params *p);
 void pme_free(mdrl_ctx *c);
-mdrl_status pme_enqueue(mdrl_ctx *c, int n, const float4 *pos, unsigned long long *F64, float *F32, bool energy);
+mdrl_status pme_begin(mdrl_ctx *c, int n, const float4 *pos, bool energy);    /* before the pair kernel's launch */
+mdrl_status pme_finish(mdrl_ctx *c, int n, const float4 *pos, unsigned long long *F64, float *F32);   /* after it */
 mdrl_status pme_add_energy(mdrl_ctx *c, int n);
 /* Bonded terms (mdrl_bonded.cu): forces into the accumulators of cell-order buffer pos / pid
  * (after the pair kernel), energies into the totals (after k_totals). */

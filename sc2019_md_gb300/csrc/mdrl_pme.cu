@@ -15,7 +15,7 @@
  *             G(m) = ke exp(-pi^2 m^2 / beta^2) / (pi V m^2) * |b1(m1) b2(m2) b3(m3)|^2, G(0) = 0,
  *             E_rec = 1/2 sum_m G(m) |X(m)|^2;
  *   gather    F_i = -q_i sum_k grad_i(prod_a M_p) phi(k), added to the particle's accumulator
- *             (one thread per particle, after the pair kernel's atomics in stream order);
+ *             (one thread per particle, after the pair kernel's atomics and the solve);
  *   constants E_self = -ke beta / sqrt(pi) sum q^2, E_background = -ke pi Q^2 / (2 V beta^2).
  *
  * The 3-D transforms are cuFFT (a plain library transform, as cuBLAS would be for a plain GEMM);
@@ -54,6 +54,9 @@ struct PmeState {
     double *d_qpart = nullptr;              /* [2 * blocks] sum q, sum q^2 partials */
     int qblocks = 0;
     double volume = 0.0;
+    /* the reciprocal part runs beside the pair kernel, on a stream of its own between two events */
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 /* theta[j] = M_p(w + j), dtheta[j] = M_p'(w + j) for j < p (grid point floor(u) - j), w in [0, 1):
@@ -320,6 +323,10 @@ static double beta_for(double rc, double tol) {
 void pme_free(mdrl_ctx *c) {
     PmeState *s = c->pme;
     if (!s) return;
+    if (s->stream) cudaStreamSynchronize(s->stream);
+    if (s->stream) cudaStreamDestroy(s->stream);
+    if (s->fork) cudaEventDestroy(s->fork);
+    if (s->join) cudaEventDestroy(s->join);
     if (s->fwd) cufftDestroy(s->fwd);
     if (s->bwd) cufftDestroy(s->bwd);
     dfree(&s->d_qfix); dfree(&s->d_real); dfree(&s->d_cplx); dfree(&s->d_green);
@@ -396,18 +403,28 @@ mdrl_status pme_setup(mdrl_ctx *c, const mdrl_pme_params *in) {
             }
     cudaError_t e = cudaMemcpy(s->d_green, G.data(), sizeof(float) * G.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { set_error(std::string("PME: ") + cudaGetErrorString(e)); return fail(MDRL_ERR_CUDA); }
+    int low = 0, high = 0;
+    e = cudaDeviceGetStreamPriorityRange(&low, &high);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&s->stream, cudaStreamNonBlocking, high);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming);
+    if (e != cudaSuccess) { set_error(std::string("PME: ") + cudaGetErrorString(e)); return fail(MDRL_ERR_CUDA); }
     if (cufftPlan3d(&s->fwd, s->K[0], s->K[1], s->K[2], CUFFT_R2C) != CUFFT_SUCCESS ||
         cufftPlan3d(&s->bwd, s->K[0], s->K[1], s->K[2], CUFFT_C2R) != CUFFT_SUCCESS ||
-        cufftSetStream(s->fwd, c->stream) != CUFFT_SUCCESS || cufftSetStream(s->bwd, c->stream) != CUFFT_SUCCESS) {
+        cufftSetStream(s->fwd, s->stream) != CUFFT_SUCCESS || cufftSetStream(s->bwd, s->stream) != CUFFT_SUCCESS) {
         set_error("PME: cuFFT plan creation failed");
         return fail(MDRL_ERR_CUDA);
     }
     return MDRL_OK;
 }
 
-/* The reciprocal-space part of one force evaluation, enqueued on the context stream after the
- * pair kernel (pos: the cell-sorted particles the pair kernel used; forces added in place). */
-mdrl_status pme_enqueue(mdrl_ctx *c, int n, const float4 *pos, unsigned long long *F64, float *F32, bool energy) {
+/* The reciprocal-space part of one force evaluation, enqueued beside what the context stream holds
+ * next, the pair kernel (pos: the cell-sorted particles the pair kernel uses).  Its eight kernels are
+ * bound by atomics, launches and the L2, the pair kernel by the L1 and its own latency, and the pair
+ * kernel's last CTAs leave SMs idle: 92k step 429 us one after the other, 414 us so.  Giving the
+ * chain room by leaving CTA slots free in the pair kernel's persistent grid costs more than it hides
+ * (15 of 16 CTAs per SM 422 us, 12 501 us), and so does one CTA per item (421 us). */
+mdrl_status pme_begin(mdrl_ctx *c, int n, const float4 *pos, bool energy) {
     PmeState *s = c->pme;
     if (!s || n <= 0) return MDRL_OK;
     PmeGeom pg;
@@ -426,18 +443,35 @@ mdrl_status pme_enqueue(mdrl_ctx *c, int n, const float4 *pos, unsigned long lon
         MDRL_TRY(dalloc(&s->d_qpart, 2 * (size_t)qb));
         s->qblocks = qb;
     }
-    MDRL_CUDA(cudaMemsetAsync(s->d_qfix, 0, sizeof(unsigned long long) * s->nreal, c->stream));
-    if (s->p.order == 6) k_pme_spread<6><<<nblk(n, 8), 256, 0, c->stream>>>(n, pos, pg, s->d_qfix);
-    else k_pme_spread<4><<<nblk(n, 16), 256, 0, c->stream>>>(n, pos, pg, s->d_qfix);
-    if (energy) k_pme_charge<<<qb, 256, 0, c->stream>>>(n, pos, s->d_qpart);
+    MDRL_CUDA(cudaEventRecord(s->fork, c->stream));
+    MDRL_CUDA(cudaStreamWaitEvent(s->stream, s->fork, 0));
+    MDRL_CUDA(cudaMemsetAsync(s->d_qfix, 0, sizeof(unsigned long long) * s->nreal, s->stream));
+    if (s->p.order == 6) k_pme_spread<6><<<nblk(n, 8), 256, 0, s->stream>>>(n, pos, pg, s->d_qfix);
+    else k_pme_spread<4><<<nblk(n, 16), 256, 0, s->stream>>>(n, pos, pg, s->d_qfix);
+    if (energy) k_pme_charge<<<qb, 256, 0, s->stream>>>(n, pos, s->d_qpart);
     const int gb = std::min(nblk(s->nreal, 256), 4 * std::max(1, c->num_sms));
-    k_pme_unfix<<<gb, 256, 0, c->stream>>>(s->nreal, s->d_qfix, s->d_real);
+    k_pme_unfix<<<gb, 256, 0, s->stream>>>(s->nreal, s->d_qfix, s->d_real);
     MDRL_CUDA(cudaGetLastError());
     PME_FFT(cufftExecR2C(s->fwd, s->d_real, s->d_cplx));
-    k_pme_convolve<<<kPmeEnergyBlocks, 256, 0, c->stream>>>(s->ncplx, s->K[2] / 2 + 1, s->K[2], s->d_cplx,
+    k_pme_convolve<<<kPmeEnergyBlocks, 256, 0, s->stream>>>(s->ncplx, s->K[2] / 2 + 1, s->K[2], s->d_cplx,
                                                             s->d_green, energy ? s->d_epart : nullptr);
     MDRL_CUDA(cudaGetLastError());
     PME_FFT(cufftExecC2R(s->bwd, s->d_cplx, s->d_real));
+    MDRL_CUDA(cudaEventRecord(s->join, s->stream));
+    return MDRL_OK;
+}
+
+/* The rest, after the pair kernel: the reciprocal forces added in place. */
+mdrl_status pme_finish(mdrl_ctx *c, int n, const float4 *pos, unsigned long long *F64, float *F32) {
+    PmeState *s = c->pme;
+    if (!s || n <= 0) return MDRL_OK;
+    PmeGeom pg;
+    for (int d = 0; d < 3; ++d) {
+        pg.K[d] = s->K[d];
+        pg.scale[d] = (float)((double)s->K[d] / c->p.box[d]);
+    }
+    const int qb = nblk(n, 256);
+    MDRL_CUDA(cudaStreamWaitEvent(c->stream, s->join, 0));
     const int acc = c->p.accum;
     if (s->p.order == 6) {
         if (acc == MDRL_ACC_FIXED64) k_pme_gather<6, MDRL_ACC_FIXED64><<<qb, 256, 0, c->stream>>>(n, pos, pg, s->d_real, F64, F32, c->d_err);
