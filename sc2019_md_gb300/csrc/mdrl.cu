@@ -20,6 +20,7 @@
 
 #include "mdrl_ctx.cuh"
 #include "mdrl_force_warp.cuh"
+#include "mdrl_force_narrow.cuh"
 #include "mdrl_hostio.cuh"
 
 using namespace mdrl;
@@ -379,7 +380,7 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     free_particles(c);
     dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     dfree(&c->d_pcoef);
-    dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work);
+    dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work); dfree(&c->d_narrow);
     dfree(&c->d_tot); dfree(&c->d_totscr); dfree(&c->d_err); dfree(&c->d_mt);
     if (c->h_tot) cudaFreeHost(c->h_tot);
     if (c->h_err) cudaFreeHost(c->h_err);
@@ -533,9 +534,35 @@ static int force_slots(const mdrl_ctx *c, int units) {
     return c->tile.warps_per_cta == 1 ? units * c->tile.steps_per_piece : units;
 }
 
-/* The force launch over units [unit0, unit0 + units) (units < 0: every unit). */
+/* Whether dynamics runs the default tile's units one warp each (mdrl_force_narrow.cuh; the same bits).
+ * c->narrow says that the state's cells fit its accumulators and the units fill the chip. */
+static bool narrow_force(const mdrl_ctx *c) {
+    return c->narrow && c->p.accum == MDRL_ACC_FIXED64 && c->tile.warps_per_cta == kNarrowWarps && !c->tile.prune_steps;
+}
+
+/* Sets c->narrow for a new state, whose largest cell holds max_occ.  Above the accumulators' 96 particles
+ * a unit works in global memory: 24,000 atoms with 192 per cell 298 us a launch, 144 by CTAs.  Below, a
+ * unit of up to 64 x 64 takes a warp no longer than the CTA, whose barriers it saves (27 cells of 64 16.0
+ * against 20.1 us); a longer one only pays where the warps run out of units late (90,000 atoms with 68 per
+ * cell 227 against 329 us, 5,000 with 78 53 against 34).  Allocates the scratch that cells crowded by later
+ * steps use; where it can't be had, the CTA kernel stays. */
+static void plan_narrow(mdrl_ctx *c, int n, int max_occ) {
+    const bool was = c->narrow;
+    const long long slots = (long long)kNarrowCtas * std::max(1, c->num_sms);
+    c->narrow = n > 0 && max_occ <= kNarrowCell && c->p.accum == MDRL_ACC_FIXED64 &&
+                (n <= 64LL * c->ncells || (long long)c->ncells * kHalfShellCells >= 4 * slots);
+    if (c->narrow && !c->d_narrow && dalloc(&c->d_narrow, kNarrowScratch * (size_t)slots) != MDRL_OK) {
+        (void)cudaGetLastError();
+        c->narrow = false;
+    }
+    if (c->narrow != was) c->graph_n = -1;
+}
+
+/* The force launch over units [unit0, unit0 + units) (units < 0: every unit).  steps: of the state that
+ * set_state planned for. */
 static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra,
-                                     unsigned long long *F64, float *F32, DevTotals *tot, int unit0 = 0, int units = -1) {
+                                     unsigned long long *F64, float *F32, DevTotals *tot, int unit0 = 0, int units = -1,
+                                     bool steps = false) {
     if (units < 0) units = c->ncells * kHalfShellCells;
     if (c->tile.warps_per_cta == 1) {
         /* one warp per (unit, i-tile group); fixed point only (set_tile checks) */
@@ -562,6 +589,25 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
     }
     const int fw = c->p.accum == MDRL_ACC_FIXED64 ? c->tile.warps_per_cta : kFW;
     const bool prune = c->p.accum == MDRL_ACC_FIXED64 && c->tile.prune_steps;
+    if (steps && narrow_force(c)) {
+        const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
+        narrow_fn fn = (c->p.flags & MDRL_FLAG_EXACT_DIFF) ? pick_force_narrow<kDiffExact>(eff_order(c), false, extra, coul)
+                                                           : pick_force_narrow<kDiffShift>(eff_order(c), sep, extra, coul);
+        MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
+        const size_t smem = force_narrow_smem_bytes(c->p.ntypes, extra);
+        int per_sm = 0;
+        MDRL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32, smem));
+        const int grid = std::min(units, std::min(std::max(1, per_sm), kNarrowCtas) * std::max(1, c->num_sms));
+        MDRL_CUDA(cudaMemsetAsync(c->d_work, 0, sizeof(int), c->stream));
+        MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
+        if (units > 0)
+            fn<<<grid, 32, smem, c->stream>>>(pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n,
+                                              F64, c->d_cnt, c->d_unit, c->tile.steps_per_piece, c->d_err, unit0,
+                                              c->d_work, units, c->d_narrow, tot);
+        MDRL_CUDA(cudaGetLastError());
+        MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
+        return MDRL_OK;
+    }
     force_fn fn = pick_force(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE, extra, c->p.accum, fw, prune,
                              (c->p.flags & MDRL_FLAG_EXACT_DIFF) != 0);
     const size_t smem = force_smem_bytes(c->p.ntypes, extra, fw);
@@ -578,12 +624,10 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
 }
 
 /* tot (without energies): the totals that take the pair count */
-static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, DevTotals *tot) {
-    return launch_force_into(c, n, pos, type, extra, c->d_F64, c->d_F32, tot);
+static mdrl_status launch_force(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, DevTotals *tot,
+                                bool steps = false) {
+    return launch_force_into(c, n, pos, type, extra, c->d_F64, c->d_F32, tot, 0, -1, steps);
 }
-
-
-
 
 /* Whether the one-CTA binning takes the system.  Its ranking costs n times the mean occupancy on one
  * SM: 1,728 atoms at 64 per cell take 15 us in all, as against 19 us and four more launches; at 4,096
@@ -1183,6 +1227,9 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_TRY(check_device_errors(c));
+    int max_occ = 0;
+    MDRL_CUDA(cudaMemcpy(&max_occ, &c->d_tot->max_occ, sizeof(int), cudaMemcpyDeviceToHost));
+    plan_narrow(c, n, max_occ);
     c->n = n;
     c->have_state = true;
     return MDRL_OK;
@@ -1214,7 +1261,7 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
         if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
     }
     MDRL_TRY(pme_begin(c, n, c->d_pos[b], extra));
-    MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra, extra ? nullptr : c->d_tot));
+    MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra, extra ? nullptr : c->d_tot, true));
     MDRL_TRY(pme_finish(c, n, c->d_pos[b], c->d_F64, c->d_F32));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[b], c->d_id[b], c->d_F64, c->d_F32, extra));
     /* kinetic energy only when energies are requested */
@@ -1281,7 +1328,7 @@ extern "C" mdrl_status mdrl_time_force(mdrl_ctx *c, float *ms) {
     if (!fp32 && !c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
     if (fp32) MDRL_CUDA(cudaMemsetAsync(c->d_Fscr32, 0, sizeof(float) * 6 * (size_t)n, c->stream));
     else MDRL_CUDA(cudaMemsetAsync(c->d_Fscr64, 0, sizeof(unsigned long long) * 3 * (size_t)n, c->stream));
-    MDRL_TRY(launch_force_into(c, n, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, c->d_Fscr32, nullptr));
+    MDRL_TRY(launch_force_into(c, n, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, c->d_Fscr32, nullptr, 0, -1, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_CUDA(cudaEventElapsedTime(ms, c->evf0, c->evf1));
     return MDRL_OK;

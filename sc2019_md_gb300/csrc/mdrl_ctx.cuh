@@ -94,6 +94,8 @@ struct mdrl_ctx {
     int *d_cell_of = nullptr, *d_slot = nullptr, *d_tmp = nullptr, *d_sorted = nullptr;
     int *d_count = nullptr, *d_start = nullptr;
     int *d_work = nullptr;      /* the persistent force kernels' item counters [2] */
+    float *d_narrow = nullptr;  /* the narrow kernel's accumulators for crowded cells */
+    bool narrow = false;        /* the state's steps take the narrow kernel (plan_narrow) */
     unsigned *d_key = nullptr;   /* in-cell sort key (Morton code inside the cell) */
     unsigned long long *d_sortkey = nullptr;   /* sorted chunks of cells above kSortSmall */
     unsigned long long *d_F64 = nullptr;
