@@ -559,7 +559,7 @@ static void plan_narrow(mdrl_ctx *c, int n, int max_occ) {
 }
 
 /* The force launch over units [unit0, unit0 + units) (units < 0: every unit).  steps: of the state that
- * set_state planned for. */
+ * set_state planned for.  The item counter d_work is zero: the scan before it has seen to that. */
 static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra,
                                      unsigned long long *F64, float *F32, DevTotals *tot, int unit0 = 0, int units = -1,
                                      bool steps = false) {
@@ -577,7 +577,6 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
         int per_sm = 0;
         MDRL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32, smem));
         const int grid = std::min(items, std::max(1, per_sm) * std::max(1, c->num_sms));
-        if (items > 0) MDRL_CUDA(cudaMemsetAsync(c->d_work, 0, sizeof(int), c->stream));
         MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
         if (items > 0)
             fn<<<grid, 32, smem, c->stream>>>(
@@ -598,7 +597,6 @@ static mdrl_status launch_force_into(mdrl_ctx *c, int n, const float4 *pos, cons
         int per_sm = 0;
         MDRL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32, smem));
         const int grid = std::min(units, std::min(std::max(1, per_sm), kNarrowCtas) * std::max(1, c->num_sms));
-        MDRL_CUDA(cudaMemsetAsync(c->d_work, 0, sizeof(int), c->stream));
         MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
         if (units > 0)
             fn<<<grid, 32, smem, c->stream>>>(pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n,
@@ -667,7 +665,7 @@ static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, 
             if (type) type = c->d_ut;
         }
     }
-    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work);
+    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work, spatial);
     if (n > 0) {
         k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
         k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted,
@@ -1247,18 +1245,17 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
             n, c->d_pos[a], c->d_vel[a], c->d_type[a], c->d_id[a], mt, dt, c->g, c->ncells, c->d_pos[b], c->d_vel[b],
             c->d_type[b], c->d_id[b], c->d_F64, c->d_F32, extra ? c->d_cnt : nullptr, c->d_start, c->d_tot, c->d_work);
     } else {
-        MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * c->ncells, c->stream));
+        /* the scan of set_state or of the last step has zeroed the counts */
         k_kick_drift_bin<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_pos[a], c->d_vel[a], c->d_type[a], c->d_F64,
                                                               c->d_F32, mt, dt, c->g, c->d_cell_of, c->d_slot,
                                                               c->d_count, c->d_key);
-        k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot);
+        k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work, true);
         k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
         k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted, c->d_key, c->d_sortkey,
                                                        c->d_err);
         k_gather_state<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_sorted, c->d_pos[a], c->d_vel[a], c->d_type[a],
                                                             c->d_id[a], c->d_pos[b], c->d_vel[b], c->d_type[b],
-                                                            c->d_id[b], c->d_F64, c->d_F32);
-        if (extra) MDRL_CUDA(cudaMemsetAsync(c->d_cnt, 0, sizeof(int) * (size_t)n, c->stream));
+                                                            c->d_id[b], c->d_F64, c->d_F32, extra ? c->d_cnt : nullptr);
     }
     MDRL_TRY(pme_begin(c, n, c->d_pos[b], extra));
     MDRL_TRY(launch_force(c, n, c->d_pos[b], c->d_type[b], extra, extra ? nullptr : c->d_tot, true));
@@ -1328,6 +1325,7 @@ extern "C" mdrl_status mdrl_time_force(mdrl_ctx *c, float *ms) {
     if (!fp32 && !c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
     if (fp32) MDRL_CUDA(cudaMemsetAsync(c->d_Fscr32, 0, sizeof(float) * 6 * (size_t)n, c->stream));
     else MDRL_CUDA(cudaMemsetAsync(c->d_Fscr64, 0, sizeof(unsigned long long) * 3 * (size_t)n, c->stream));
+    MDRL_CUDA(cudaMemsetAsync(c->d_work, 0, 2 * sizeof(int), c->stream));    /* no scan precedes this launch */
     MDRL_TRY(launch_force_into(c, n, c->d_pos[a], c->d_type[a], false, c->d_Fscr64, c->d_Fscr32, nullptr, 0, -1, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     MDRL_CUDA(cudaEventElapsedTime(ms, c->evf0, c->evf1));

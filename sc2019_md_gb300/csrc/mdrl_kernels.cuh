@@ -347,12 +347,13 @@ static __global__ void k_bin_user(int n, const float *__restrict__ x, const floa
 }
 
 /* Exclusive scan of the cell counts (one CTA), plus the largest occupancy; zeroes the totals' counts and
- * the force launches' item counters work[0..1] on the way (a memset less per evaluation).  Latency-bound: 4 counts per
+ * the force launches' item counters work[0..1] on the way (a memset less per launch), and with clear the
+ * counts it has read, for the next step's binning.  Latency-bound: 4 counts per
  * thread and pass in one 16-byte load, warp scans by shuffles, one barrier per pass of 4,096 cells.
  * (A strided run of cells per thread and a 20-barrier scan: 486 cells 3.8 us, 10,648 cells 9.9 us, 28k
  * cells 53 us; now 2.2, 3.3 and 6.) */
-static __global__ void __launch_bounds__(1024) k_scan(int ncells, const int *__restrict__ count,
-                                               int *__restrict__ start, DevTotals *tot, int *work = nullptr) {
+static __global__ void __launch_bounds__(1024) k_scan(int ncells, int *__restrict__ count, int *__restrict__ start,
+                                               DevTotals *tot, int *work = nullptr, bool clear = false) {
     __shared__ int s_sum[2][32], s_max[32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     if (work && t < 2) work[t] = 0;
@@ -366,6 +367,11 @@ static __global__ void __launch_bounds__(1024) k_scan(int ncells, const int *__r
             if (k < ncells) c.x = count[k];
             if (k + 1 < ncells) c.y = count[k + 1];
             if (k + 2 < ncells) c.z = count[k + 2];
+        }
+        if (clear) {
+            if (k + 3 < ncells) *reinterpret_cast<int4 *>(count + k) = make_int4(0, 0, 0, 0);
+            else
+                for (int u = k; u < ncells; ++u) count[u] = 0;
         }
         mx = max(mx, max(max(c.x, c.y), max(c.z, c.w)));
         const int own = c.x + c.y + c.z + c.w;
@@ -700,9 +706,11 @@ static __global__ void k_gather_state(int n, const int *__restrict__ sorted,
                                const int *__restrict__ type0, const int *__restrict__ id0,
                                float4 *__restrict__ pos1, float4 *__restrict__ vel1,
                                int *__restrict__ type1, int *__restrict__ id1,
-                               unsigned long long *__restrict__ F64, float *__restrict__ F32) {
+                               unsigned long long *__restrict__ F64, float *__restrict__ F32,
+                               int *__restrict__ counts = nullptr) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
+    if (counts) counts[k] = 0;
     const int o = sorted[k];
     pos1[k] = pos0[o];
     vel1[k] = vel0[o];
