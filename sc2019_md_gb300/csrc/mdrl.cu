@@ -367,14 +367,19 @@ static void free_particles(mdrl_ctx *c) {
     c->cap = 0;
 }
 
+static void drop_graphs(mdrl_ctx *c) {
+    for (int k = 0; k < 4; ++k) {
+        if (c->graph_exec[k]) { cudaGraphExecDestroy(c->graph_exec[k]); c->graph_exec[k] = nullptr; }
+        if (c->graph[k]) { cudaGraphDestroy(c->graph[k]); c->graph[k] = nullptr; }
+    }
+    c->graph_n = -1;
+}
+
 extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     if (!c) return MDRL_OK;
     cudaSetDevice(c->p.device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (int k = 0; k < 2; ++k) {
-        if (c->graph_exec[k]) cudaGraphExecDestroy(c->graph_exec[k]);
-        if (c->graph[k]) cudaGraphDestroy(c->graph[k]);
-    }
+    drop_graphs(c);
     pme_free(c);
     bonded_free(c);
     free_particles(c);
@@ -1052,11 +1057,7 @@ extern "C" mdrl_status mdrl_set_tables(mdrl_ctx *c, int order, int nseg, int bin
     c->local = (flags & MDRL_TABLE_BIN_LOCAL) != 0;
     c->tab.assign((size_t)kNumFunc * nc * nidx, 0.0f);
     memcpy(c->tab.data(), coef, sizeof(float) * (size_t)nfunc * nc * nidx);
-    for (int k = 0; k < 2; ++k) {
-        if (c->graph_exec[k]) { cudaGraphExecDestroy(c->graph_exec[k]); c->graph_exec[k] = nullptr; }
-        if (c->graph[k]) { cudaGraphDestroy(c->graph[k]); c->graph[k] = nullptr; }
-    }
-    c->graph_n = -1;
+    drop_graphs(c);
     return upload_tables(c);
 }
 
@@ -1272,6 +1273,32 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
     return MDRL_OK;
 }
 
+/* Captures and instantiates graph k of the context, unless it is there: one step from buffer slot k, or
+ * two from slot k - 2.  Between two graphs the GPU waits longer than between two of a graph's nodes;
+ * graphs of two steps halve those waits and cost no more to make than the two of one step that an even
+ * number of steps would need. */
+static mdrl_status capture_steps(mdrl_ctx *c, bool extra, int k) {
+    if (c->graph_exec[k]) return MDRL_OK;
+    const int saved = c->cur;
+    MDRL_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    mdrl_status s = MDRL_OK;
+    for (int t = 0; t < (k < 2 ? 1 : 2) && s == MDRL_OK; ++t) {
+        c->cur = (k & 1) ^ t;
+        s = enqueue_step(c, extra);
+    }
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    c->cur = saved;
+    /* a step that failed between PME's two halves ends the capture unjoined: not the next call's error */
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    if (s != MDRL_OK) { if (g) cudaGraphDestroy(g); return s; }
+    if (e != cudaSuccess) { set_error(std::string("graph capture: ") + cudaGetErrorString(e)); return MDRL_ERR_CUDA; }
+    if (c->graph[k]) cudaGraphDestroy(c->graph[k]);
+    c->graph[k] = g;
+    MDRL_CUDA(cudaGraphInstantiate(&c->graph_exec[k], g, 0));
+    return MDRL_OK;
+}
+
 extern "C" mdrl_status mdrl_step(mdrl_ctx *c, int nsteps, mdrl_stats *st) {
     if (!c || nsteps < 0) { set_error("mdrl_step: invalid argument"); return MDRL_ERR_INVALID_ARG; }
     if (!c->have_state) { set_error("mdrl_step: call mdrl_set_state first"); return MDRL_ERR_STATE; }
@@ -1281,29 +1308,16 @@ extern "C" mdrl_status mdrl_step(mdrl_ctx *c, int nsteps, mdrl_stats *st) {
     MDRL_CUDA(cudaMemsetAsync(&c->d_tot->pairs_total, 0, sizeof(unsigned long long), c->stream));
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     if (c->graph_n != c->n || c->graph_extra != extra) {
-        /* Capture one step per buffer parity (slot 0 -> 1 and slot 1 -> 0). */
-        const int saved = c->cur;
-        for (int k = 0; k < 2; ++k) {
-            if (c->graph_exec[k]) { cudaGraphExecDestroy(c->graph_exec[k]); c->graph_exec[k] = nullptr; }
-            if (c->graph[k]) { cudaGraphDestroy(c->graph[k]); c->graph[k] = nullptr; }
-            c->cur = k;
-            MDRL_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            const mdrl_status s = enqueue_step(c, extra);
-            cudaGraph_t g = nullptr;
-            const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
-            c->cur = saved;
-            /* a step that failed between PME's two halves ends the capture unjoined: not the next call's error */
-            if (e != cudaSuccess) (void)cudaGetLastError();
-            if (s != MDRL_OK) { if (g) cudaGraphDestroy(g); return s; }
-            if (e != cudaSuccess) { set_error(std::string("graph capture: ") + cudaGetErrorString(e)); return MDRL_ERR_CUDA; }
-            c->graph[k] = g;
-            MDRL_CUDA(cudaGraphInstantiate(&c->graph_exec[k], g, 0));
-        }
+        drop_graphs(c);
         c->graph_n = c->n;
         c->graph_extra = extra;
     }
+    /* pairs of steps, and an odd one after them: the slot they start from is the same */
+    if (nsteps >= 2) MDRL_TRY(capture_steps(c, extra, 2 + c->cur));
+    if (nsteps & 1) MDRL_TRY(capture_steps(c, extra, c->cur));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
-    for (int k = 0; k < nsteps; ++k) {
+    for (int k = 0; k + 2 <= nsteps; k += 2) MDRL_CUDA(cudaGraphLaunch(c->graph_exec[2 + c->cur], c->stream));
+    if (nsteps & 1) {
         MDRL_CUDA(cudaGraphLaunch(c->graph_exec[c->cur], c->stream));
         c->cur ^= 1;
     }
@@ -1379,14 +1393,6 @@ static mdrl_status check_tile(const mdrl_tile *t, bool allow8, bool allow_prune,
         return MDRL_ERR_INVALID_ARG;
     }
     return MDRL_OK;
-}
-
-static void drop_graphs(mdrl_ctx *c) {
-    for (int k = 0; k < 2; ++k) {
-        if (c->graph_exec[k]) { cudaGraphExecDestroy(c->graph_exec[k]); c->graph_exec[k] = nullptr; }
-        if (c->graph[k]) { cudaGraphDestroy(c->graph[k]); c->graph[k] = nullptr; }
-    }
-    c->graph_n = -1;
 }
 
 namespace mdrl {

@@ -125,8 +125,9 @@ struct mdrl_ctx {
 
     /* state */
     bool have_state = false;
-    cudaGraph_t graph[2] = {nullptr, nullptr};          /* one step from buffer slot k to 1-k */
-    cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
+    /* [k]: one step from buffer slot k to 1-k; [2 + k]: two steps from slot k back to it */
+    cudaGraph_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaGraphExec_t graph_exec[4] = {nullptr, nullptr, nullptr, nullptr};
     int graph_n = -1;
     bool graph_extra = false;
 
