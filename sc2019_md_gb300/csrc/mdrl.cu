@@ -546,16 +546,19 @@ static bool narrow_force(const mdrl_ctx *c) {
 }
 
 /* Sets c->narrow for a new state, whose largest cell holds max_occ.  Above the accumulators' 96 particles
- * a unit works in global memory: 24,000 atoms with 192 per cell 298 us a launch, 144 by CTAs.  Below, a
- * unit of up to 64 x 64 takes a warp no longer than the CTA, whose barriers it saves (27 cells of 64 16.0
- * against 20.1 us); a longer one only pays where the warps run out of units late (90,000 atoms with 68 per
- * cell 227 against 329 us, 5,000 with 78 53 against 34).  Allocates the scratch that cells crowded by later
- * steps use; where it can't be had, the CTA kernel stays. */
+ * a unit works in global memory: 24,000 atoms with 192 per cell 298 us a launch, 144 by CTAs.  Below, units
+ * of one 32-particle tile are always faster (64 cells of 27 particles 16 against 20 us).  Larger ones take a
+ * warp longer than a CTA and pay once they fill a wave: chains of up to 70 per cell take 45 against 25 us in
+ * 64 cells, 43 against 45 in 196, 47 against 71 in 392; up to 60 argon atoms in 216 cells 43 against 53.
+ * Above 64 on average they pay where the last wave counts for little: 90,000 atoms with 68 per cell (7.7
+ * waves) 227 against 329 us, 5,000 with 78 53 against 34.  Allocates the scratch that cells crowded by
+ * later steps use; where it can't be had, the CTA kernel stays. */
 static void plan_narrow(mdrl_ctx *c, int n, int max_occ) {
     const bool was = c->narrow;
     const long long slots = (long long)kNarrowCtas * std::max(1, c->num_sms);
+    const long long units = (long long)c->ncells * kHalfShellCells;
     c->narrow = n > 0 && max_occ <= kNarrowCell && c->p.accum == MDRL_ACC_FIXED64 &&
-                (n <= 64LL * c->ncells || (long long)c->ncells * kHalfShellCells >= 4 * slots);
+                (max_occ <= 32 || units >= (n <= 64LL * c->ncells ? 1 : 4) * slots);
     if (c->narrow && !c->d_narrow && dalloc(&c->d_narrow, kNarrowScratch * (size_t)slots) != MDRL_OK) {
         (void)cudaGetLastError();
         c->narrow = false;

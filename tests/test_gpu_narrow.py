@@ -1,14 +1,15 @@
-"""Dynamics that runs the default tile's units one warp each (no cell above 96 particles at set_state)
-against the CTA kernel: the same forces and velocities bit for bit.  The second run holds a crowded cell
-beyond everyone's reach, so it takes the CTA kernel.  The step moves the particles into cells from empty
-to 300: on both sides of a tile, of the shared accumulators (96) and of a chunk (256)."""
+"""Dynamics that runs the default tile's units one warp each (no cell above 96 particles at set_state,
+2,646 units: more than one for each resident warp) against the CTA kernel: the same forces and velocities
+bit for bit.  The second run holds a crowded cell beyond everyone's reach, so it takes the CTA kernel.
+The step moves the particles into cells from empty to 300: on both sides of a tile, of the shared
+accumulators (96) and of a chunk (256)."""
 import numpy as np
 import pytest
 
 import sc2019_md_gb300 as m
 
 pytestmark = pytest.mark.gpu
-BOX, RC, DT = (37.5, 37.5, 150.0), 12.0, 2.0
+BOX, RC, DT = (37.5, 37.5, 262.5), 12.0, 2.0
 
 
 def _grid(rng, lo, hi, n, jitter):
@@ -49,7 +50,7 @@ def arrays():
 
 def _occupancy(p):
     c = np.floor(p / 12.5).astype(int)
-    return np.bincount((c[:, 0] * 3 + c[:, 1]) * 12 + c[:, 2], minlength=108)
+    return np.bincount((c[:, 0] * 3 + c[:, 1]) * 21 + c[:, 2], minlength=189)
 
 
 @pytest.mark.parametrize("order", [0, 1, 2, 3])
