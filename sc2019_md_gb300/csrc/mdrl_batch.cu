@@ -202,6 +202,9 @@ struct mdrl_batch {
     int *d_rep_pos = nullptr;
     bool list_slots = false; /* the result slots are those of a list launch: */
     int list_first[2] = {0, 0}, list_per_item[2] = {1, 1};   /* its first slots and slots per item */
+    /* an evaluation's list launches run beside its all-image launch, on a stream of their own */
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     RepTotals *d_reptot = nullptr;
     bool have_eval = false;  /* the unit outputs hold a force evaluation */
 };
@@ -251,7 +254,11 @@ extern "C" mdrl_status mdrl_batch_destroy(mdrl_batch *b) {
     if (b->c) {
         cudaSetDevice(b->c->p.device);
         if (b->c->stream) cudaStreamSynchronize(b->c->stream);
+        if (b->side) cudaStreamSynchronize(b->side);
     }
+    if (b->side) cudaStreamDestroy(b->side);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
     dfree(&b->d_reps); dfree(&b->d_items); dfree(&b->d_rep_of); dfree(&b->d_item_begin);
     dfree(&b->d_rep_items); dfree(&b->d_reptot);
     dfree(&b->d_items_hs); dfree(&b->d_items_ot); dfree(&b->d_begin_hs); dfree(&b->d_list_hs);
@@ -414,6 +421,13 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     /* the context's cell buffers sized for the whole batch (ensure_capacity keeps them) */
     c->ncells = bt->ncells;
     c->batch = true;
+    cudaError_t se = cudaStreamCreateWithFlags(&bt->side, cudaStreamNonBlocking);
+    if (se == cudaSuccess) se = cudaEventCreateWithFlags(&bt->fork, cudaEventDisableTiming);
+    if (se == cudaSuccess) se = cudaEventCreateWithFlags(&bt->join, cudaEventDisableTiming);
+    if (se != cudaSuccess) {
+        set_error(std::string("mdrl_batch_create: ") + cudaGetErrorString(se));
+        return fail(MDRL_ERR_CUDA);
+    }
     if ((s = dalloc(&c->d_work, 2)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_count, (size_t)bt->ncells)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_start, (size_t)bt->ncells + 1)) != MDRL_OK) return fail(s);
@@ -535,22 +549,15 @@ static int list_items(const mdrl_batch *b, int k, bool *fine) {
     return *fine ? items * kRuns : items;
 }
 
-/* A force evaluation's launches (list_eval): the all-image replicas in the CTA kernel, then the list
- * kernel over the min-image and the half-shell replicas; *slots: their result slots, in that order. */
-static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int *type, bool extra, int *slots) {
+/* The list kernel over the min-image and the half-shell replicas on stream st; *slots: the result slots
+ * so far. */
+static mdrl_status launch_lists(mdrl_batch *b, cudaStream_t st, const float4 *pos, const int *type, bool extra,
+                                int *slots) {
     mdrl_ctx *c = b->c;
     const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
     const int G = c->tile_set ? c->tile.steps_per_piece : 1;
     const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
     DevTotals *tot = extra ? nullptr : c->d_tot;
-    force_fn fo = pick_force_batch(eff_order(c), sep, extra, false);
-    MDRL_TRY(prepare_force_kernel(fo, c->p.device));
-    MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
-    if (b->n_ot)
-        fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
-            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, nullptr,
-            c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0, tot);
-    *slots = b->n_ot;
     for (int k = 0; k < 2; ++k) {
         bool fine;
         int grid = 0;
@@ -562,12 +569,45 @@ static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int
                        : pick_force_list<kDiffWrap, true>(eff_order(c), sep, extra, coul, fine);
         MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
         MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
-        fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
+        fn<<<grid, 32 * kWarpsPerCta, smem, st>>>(
             pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, c->d_cnt,
             c->d_unit + *slots, b->lists[k].dev, b->d_reps, G, c->d_err, 0, c->d_work + k, items, tot);
         *slots += items;
     }
     MDRL_CUDA(cudaGetLastError());
+    return MDRL_OK;
+}
+
+/* A force evaluation's launches (list_eval): the all-image replicas in the CTA kernel and, beside it on
+ * the side stream, the list kernel; *slots: their result slots, in that order.  The launches write
+ * different replicas' particles and slots; the counts they share are atomic sums of integers.  The
+ * all-image launch is a few long CTAs (15 replicas of 500 to 4,000 atoms: 309 us on a fraction of the
+ * SMs, with the lists' 93 + 82 us after it); it is first in its stream, so its CTAs are placed before the
+ * lists' persistent grids take the rest. */
+static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int *type, bool extra, int *slots) {
+    mdrl_ctx *c = b->c;
+    force_fn fo = pick_force_batch(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE, extra, false);
+    MDRL_TRY(prepare_force_kernel(fo, c->p.device));
+    MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
+    *slots = b->n_ot;
+    const bool both = b->n_ot && (b->lists[0].items || b->lists[1].items);
+    if (both) MDRL_CUDA(cudaEventRecord(b->fork, c->stream));
+    if (b->n_ot)
+        fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
+            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, nullptr,
+            c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0,
+            extra ? nullptr : c->d_tot);
+    if (!both) {
+        MDRL_TRY(launch_lists(b, c->stream, pos, type, extra, slots));
+    } else {
+        MDRL_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
+        const mdrl_status s = launch_lists(b, b->side, pos, type, extra, slots);
+        cudaError_t e = cudaEventRecord(b->join, b->side);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, b->join, 0);
+        if (e != cudaSuccess) cudaStreamSynchronize(b->side);    /* nothing of this call runs into the next */
+        MDRL_TRY(s);
+        MDRL_CUDA(e);
+    }
     MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
     return MDRL_OK;
 }
