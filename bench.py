@@ -39,6 +39,9 @@ sys.path.insert(0, str(ROOT))
 
 FLOPS_PER_PAIR = 28            # algorithmic flops per in-cutoff pair, force only
 BYTES_PER_PARTICLE = 16 + 4 + 24   # pos+q and type read, int64 x3 force atomics, per force launch
+# kernels of a step without energies: kick+drift+bin, scan, scatter, sort, gather, force, kick; systems of
+# up to 4,096 particles bin, sort and gather in one
+STEP_LAUNCHES, SMALL_STEP_LAUNCHES = 7, 3
 L2_FLUSH_BYTES = 256 << 20     # > 129 MB L2
 METRIC = "pair-evals/s & ns/day, 92k-atom RL LJ+Coulomb, tuned vs plain @1e-5 force err"
 CAPTURES = ROOT / "profiles" / "ncu_captures.json"   # per-capture ncu figures (workload, tile, datapath)
@@ -430,7 +433,7 @@ def sub_workload_single(m, sysm, args, local, flush, props):
                 "d2h_bytes_per_step": sysm.n * 12, "calls": e2e["calls"],
                 "ms_per_call": e2e["secs"] / e2e["calls"] * 1e3},
         "pairs_per_step": tuned["pairs_per_step"],
-        "gpu_launches": 8 * k,
+        "gpu_launches": STEP_LAUNCHES * k,
     }
 
 
@@ -610,7 +613,7 @@ def run_ours(args, rank, world, local, dist):
                 "host_link": "pinned buffers read and written in place by the binning and unsort kernels"},
         "with_pme": pme_out,
         "bonded": bonded_out,
-        "gpu_launches": 8 * args.steps,
+        "gpu_launches": (SMALL_STEP_LAUNCHES if sysm.n <= 4096 else STEP_LAUNCHES) * args.steps,
         "clocks": clk,
         "wall_s": res["wall_s"],
     }
