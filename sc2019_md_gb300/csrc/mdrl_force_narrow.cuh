@@ -16,7 +16,7 @@
  *
  * Latency-bound, as the CTA kernel, with 16 working warps per SM instead of 4 to 8.  A launch by CTAs
  * and here: 24,000 atoms at 14 per cell 172 -> 73 us, at 33 120 -> 61; 90,000 at 33 421 -> 192, at 68
- * 329 -> 227; 1,728 at 64 20 -> 16.  Accumulators of 64 particles run 33 per cell 3 to 7 % faster and
+ * 329 -> 227; 1,728 at 27 20 -> 16.  Accumulators of 64 particles run 33 per cell 3 to 7 % faster and
  * 68 per cell 1.6 times slower, of 128 10 % slower and 4 % faster; 12 CTAs per SM instead of 16
  * 13 % slower at 33, 20 and 24 never faster.
  */
