@@ -175,6 +175,10 @@ mdrl_status mdrl_fit_tables_bin_local(int order, int nseg, int bins, int min_log
 mdrl_status mdrl_create(const mdrl_params *p, mdrl_ctx **out);
 mdrl_status mdrl_destroy(mdrl_ctx *ctx);
 
+/* *pending: 1 while a stream of the context holds unfinished work, else 0.  Every call that takes the
+ * caller's arrays returns with 0, whatever its status, so the arrays may be freed or reused at once. */
+mdrl_status mdrl_pending(mdrl_ctx *ctx, int *pending);
+
 /* Replace the generated tables, e.g. with the reference's ROM images.  coef holds nfunc
  * functions (2: r^-14, r^-8; 3: + r^-3; 6: + r^-12, r^-6, r^-1), each as (order+1) planes of
  * nseg*bins coefficients, plane k holding the coefficient of r2^k.  flags (MDRL_TABLE_*):
@@ -349,6 +353,7 @@ enum { MDRL_PATH_HALF_SHELL = 0, MDRL_PATH_MIN_IMAGE = 1, MDRL_PATH_ALL_IMAGES =
 mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const mdrl_replica *reps,
                               mdrl_batch **out);
 mdrl_status mdrl_batch_destroy(mdrl_batch *batch);
+mdrl_status mdrl_batch_pending(mdrl_batch *batch, int *pending);   /* see mdrl_pending */
 /* Per replica (arrays of nrep, any may be NULL): the path, cells per axis [3*nrep], and work
  * items of the force launch; *total_items the launch's grid. */
 mdrl_status mdrl_batch_layout(mdrl_batch *batch, int *path, int *ncell, int *items, int *total_items);

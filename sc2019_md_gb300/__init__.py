@@ -157,6 +157,8 @@ def lib() -> C.CDLL:
     L.mdrl_force_eval_fixed.argtypes = [vp, st, _F, _F, _F, _F, _I, st, st, C.POINTER(C.c_int64), C.POINTER(Stats)]
     L.mdrl_create.argtypes = [C.POINTER(Params), C.POINTER(vp)]
     L.mdrl_destroy.argtypes = [vp]
+    L.mdrl_pending.argtypes = [vp, _I]
+    L.mdrl_batch_pending.argtypes = [vp, _I]
     L.mdrl_set_tables.argtypes = [vp, st, st, st, st, st, _F, st]
     L.mdrl_get_tables.argtypes = [vp, _I, _I, _I, _I, _F]
     L.mdrl_get_pair_coefficients.argtypes = [vp, _F]
@@ -198,7 +200,7 @@ def lib() -> C.CDLL:
     for name in ("mdrl_set_pme", "mdrl_get_pme", "mdrl_set_pair_coefficients", "mdrl_batch_set_pair_coefficients", "mdrl_set_tile", "mdrl_get_tile", "mdrl_autotune", "mdrl_batch_set_tile", "mdrl_batch_autotune",
                  "mdrl_batch_create", "mdrl_batch_destroy", "mdrl_batch_layout", "mdrl_batch_force_eval",
                  "mdrl_batch_set_state", "mdrl_batch_step", "mdrl_batch_get_state",
-                 "mdrl_batch_replica_stats", "mdrl_batch_time_force"):
+                 "mdrl_batch_replica_stats", "mdrl_batch_time_force", "mdrl_pending", "mdrl_batch_pending"):
         getattr(L, name).restype = st
     for name in ("mdrl_fit_tables", "mdrl_fit_tables_bin_local", "mdrl_get_table_form", "mdrl_slab_plan",
                  "mdrl_slab_select", "mdrl_force_eval_fixed", "mdrl_create", "mdrl_destroy", "mdrl_set_tables",
@@ -285,6 +287,12 @@ class Context:
         if self._h:
             lib().mdrl_destroy(self._h)
             self._h = C.c_void_p()
+
+    def pending(self) -> bool:
+        """Whether a stream of the context holds unfinished work."""
+        v = C.c_int()
+        _check(lib().mdrl_pending(self._h, C.byref(v)))
+        return bool(v.value)
 
     def __enter__(self):
         return self
@@ -527,6 +535,11 @@ class Batch:
             self.close()
         except Exception:
             pass
+
+    def pending(self) -> bool:
+        v = C.c_int()
+        _check(lib().mdrl_batch_pending(self._h, C.byref(v)))
+        return bool(v.value)
 
     def layout(self) -> dict:
         path = np.zeros(self.nrep, np.int32)

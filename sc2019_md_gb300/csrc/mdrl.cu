@@ -399,6 +399,23 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     return MDRL_OK;
 }
 
+int mdrl::streams_pending(const mdrl_ctx *c, cudaStream_t side) {
+    int pending = 0;
+    for (cudaStream_t s : {c->stream, side, pme_stream(c)})
+        if (s && cudaStreamQuery(s) == cudaErrorNotReady) {
+            (void)cudaGetLastError();
+            pending = 1;
+        }
+    return pending;
+}
+
+extern "C" mdrl_status mdrl_pending(mdrl_ctx *c, int *pending) {
+    if (!c || !pending) { set_error("mdrl_pending: null argument"); return MDRL_ERR_INVALID_ARG; }
+    MDRL_CUDA(cudaSetDevice(c->p.device));
+    *pending = streams_pending(c);
+    return MDRL_OK;
+}
+
 static mdrl_status ensure_cells(mdrl_ctx *c) {
     if (c->ncells) return MDRL_OK;
     MDRL_TRY(check_cells(c));
@@ -818,8 +835,10 @@ static mdrl_status force_eval_finish(mdrl_ctx *c, mdrl_stats *st) {
 static mdrl_status force_eval_dev(mdrl_ctx *c, int n, const float *x, const float *y, const float *z,
                                   const float *q, const int *type, float *fx, float *fy, float *fz,
                                   int *counts, mdrl_stats *st) {
+    CallGuard guard(c);
     MDRL_TRY(force_eval_enqueue(c, n, x, y, z, q, type, fx, fy, fz, counts));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     return force_eval_finish(c, st);
 }
 
@@ -844,6 +863,8 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
     }
     MDRL_CUDA(cudaSetDevice(c->p.device));
     MDRL_TRY(ensure_capacity(c, n));
+    MDRL_TRY(bonded_check_atoms(c, n));    /* refused calls enqueue nothing */
+    CallGuard guard(c);
     /* Pinned (page-locked) host buffers, or this device's memory: the kernels read the inputs and
      * write the forces in place, coalesced, over the host link; no staging copies. */
     if (n > 0) {
@@ -856,6 +877,7 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
                                         (const float *)dq, (const int *)dt, (float *)dfx, (float *)dfy,
                                         (float *)dfz, (int *)dc, true));
             MDRL_CUDA(cudaStreamSynchronize(c->stream));   /* the one synchronisation of the call */
+            guard.done();
             return force_eval_finish(c, st);
         }
     }
@@ -881,6 +903,7 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
                                 direct ? &out : nullptr));
     if (!direct) MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, dev, host, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));   /* the one synchronisation of the call */
+    guard.done();
     return force_eval_finish(c, st);
 }
 
@@ -973,6 +996,8 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     bool pageable = false;
     void *dF = n ? device_view(c, F, 8, &pageable) : nullptr;
     const bool direct = n > 0 && dx && dy && dz && (!q || dq) && (!type || dt);
+    if (!dF && n > 0 && !c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
+    CallGuard guard(c);
     if (n > 0 && !direct) {
         const void *src[5] = {x, y, z, q, type};
         void *dst[5] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut};
@@ -981,7 +1006,6 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
         dq = q ? c->d_uq : nullptr;
         dt = type ? c->d_ut : nullptr;
     }
-    if (!dF && n > 0 && !c->d_Fscr64) MDRL_TRY(dalloc(&c->d_Fscr64, 3 * (size_t)c->cap));
     long long *Fout = dF ? (long long *)dF : (long long *)c->d_Fscr64;
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
@@ -1001,6 +1025,7 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     if (n > 0 && !dF)
         MDRL_CUDA(cudaMemcpyAsync(F, c->d_Fscr64, 3 * sizeof(long long) * (size_t)n, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     MDRL_TRY(check_device_errors(c));
     c->have_state = false;
     float ms = 0.0f;
@@ -1016,6 +1041,7 @@ extern "C" mdrl_status mdrl_bin(mdrl_ctx *c, int n, const float *x, const float 
     }
     MDRL_CUDA(cudaSetDevice(c->p.device));
     MDRL_TRY(ensure_capacity(c, n));
+    CallGuard guard(c);
     const void *src[3] = {x, y, z};
     void *dst[3] = {c->d_ux, c->d_uy, c->d_uz};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 3, src, dst, false));
@@ -1025,6 +1051,7 @@ extern "C" mdrl_status mdrl_bin(mdrl_ctx *c, int n, const float *x, const float 
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 2, bsrc, bdst, true));
     if (cell_count) MDRL_CUDA(cudaMemcpyAsync(cell_count, c->d_count, sizeof(int) * c->ncells, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     MDRL_TRY(check_device_errors(c));
     c->have_state = false;
     return MDRL_OK;
@@ -1164,6 +1191,7 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
     }
     /* the types are read and the results written in place where the device can; the positions are
      * copied (4 n elements: two launches' worth of 2^31 at most) */
+    CallGuard guard(c);
     const bool small = n <= 0x7fffffff / 4;
     const void *src[2] = {ref, nbr};
     void *dst[2] = {c->d_pr, c->d_pn};
@@ -1192,6 +1220,7 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
     if (!vout) MDRL_CUDA(cudaMemcpyAsync(out, c->d_pout, sizeof(float4) * n, cudaMemcpyDeviceToHost, c->stream));
     if (aux && !vaux) MDRL_CUDA(cudaMemcpyAsync(aux, c->d_paux, sizeof(float2) * n, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     return MDRL_OK;
 }
 
@@ -1208,6 +1237,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_TRY(ensure_capacity(c, n));
     MDRL_TRY(bonded_check_atoms(c, n));
     if (small_system(c, n)) MDRL_TRY(prepare_force_kernel((force_fn)k_small_state, c->p.device));
+    CallGuard guard(c);
     const void *src[8] = {x, y, z, q, type, vx, vy, vz};
     void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 8, src, dst, false));
@@ -1228,6 +1258,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     MDRL_TRY(check_device_errors(c));
     int max_occ = 0;
     MDRL_CUDA(cudaMemcpy(&max_occ, &c->d_tot->max_occ, sizeof(int), cudaMemcpyDeviceToHost));
@@ -1354,6 +1385,7 @@ extern "C" mdrl_status mdrl_get_state(mdrl_ctx *c, float *x, float *y, float *z,
     if (!c) { set_error("null context"); return MDRL_ERR_INVALID_ARG; }
     if (!c->have_state) { set_error("mdrl_get_state: no state"); return MDRL_ERR_STATE; }
     MDRL_CUDA(cudaSetDevice(c->p.device));
+    CallGuard guard(c);
     const int n = c->n, a = c->cur;
     k_unsort_state<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[a], c->d_pos[a], c->d_vel[a], c->d_ux, c->d_uy,
                                                         c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz);
@@ -1364,6 +1396,7 @@ extern "C" mdrl_status mdrl_get_state(mdrl_ctx *c, float *x, float *y, float *z,
     const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     return MDRL_OK;
 }
 

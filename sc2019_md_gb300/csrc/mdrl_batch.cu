@@ -675,6 +675,7 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     MDRL_CUDA(cudaSetDevice(c->p.device));
     const int n = b->ntot;
     const bool extra = counts != nullptr || (c->p.flags & MDRL_FLAG_ENERGY);
+    CallGuard guard(c, b->side);
     MDRL_TRY(upload_user(b, x, y, z, q, type));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
@@ -693,6 +694,7 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     void *dst[4] = {fx, fy, fz, counts};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     float ms = 0.0f;
     MDRL_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     MDRL_TRY(check_device_errors(c));
@@ -711,6 +713,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     mdrl_ctx *c = b->c;
     MDRL_CUDA(cudaSetDevice(c->p.device));
     const int n = b->ntot;
+    CallGuard guard(c, b->side);
     MDRL_TRY(upload_user(b, x, y, z, q, type, vx, vy, vz));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     c->cur = 0;
@@ -725,6 +728,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     launch_totals(c, batch_slots(b), nblk(n, 256), extra);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     MDRL_TRY(check_device_errors(c));
     c->n = n;
     c->have_state = true;
@@ -807,6 +811,7 @@ extern "C" mdrl_status mdrl_batch_get_state(mdrl_batch *b, float *x, float *y, f
     mdrl_ctx *c = b->c;
     if (!c->have_state) { set_error("mdrl_batch_get_state: no state"); return MDRL_ERR_STATE; }
     MDRL_CUDA(cudaSetDevice(c->p.device));
+    CallGuard guard(c, b->side);
     const int n = b->ntot, a = c->cur;
     k_unsort_state<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[a], c->d_pos[a], c->d_vel[a], c->d_ux, c->d_uy,
                                                         c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz);
@@ -817,6 +822,7 @@ extern "C" mdrl_status mdrl_batch_get_state(mdrl_batch *b, float *x, float *y, f
     const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
     MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
+    guard.done();
     return MDRL_OK;
 }
 
@@ -860,6 +866,13 @@ extern "C" mdrl_status mdrl_batch_replica_stats(mdrl_batch *b, mdrl_stats *out) 
         s.virial = h[r].virial;
         s.kinetic = h[r].kinetic;
     }
+    return MDRL_OK;
+}
+
+extern "C" mdrl_status mdrl_batch_pending(mdrl_batch *b, int *pending) {
+    if (!b || !pending) { set_error("mdrl_batch_pending: null argument"); return MDRL_ERR_INVALID_ARG; }
+    MDRL_CUDA(cudaSetDevice(b->c->p.device));
+    *pending = streams_pending(b->c, b->side);
     return MDRL_OK;
 }
 

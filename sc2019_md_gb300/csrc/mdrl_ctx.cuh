@@ -156,6 +156,28 @@ bool list_eval(const mdrl_ctx *c);
 void launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy);
 mdrl_status list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid);
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
+
+cudaStream_t pme_stream(const mdrl_ctx *c);    /* PME's own stream, or null without PME */
+
+/* A call that hands the caller's arrays to kernels or copies: on every return before done() it waits for
+ * the call's streams, so that the caller may free or reuse the arrays whatever the status.  (Direct
+ * calls: an injected failure does not reach them.) */
+struct CallGuard {
+    mdrl_ctx *c;
+    cudaStream_t side;
+    bool open = true;
+    explicit CallGuard(mdrl_ctx *ctx, cudaStream_t side_stream = nullptr) : c(ctx), side(side_stream) {}
+    CallGuard(const CallGuard &) = delete;
+    void done() { open = false; }              /* the streams have been joined and waited for */
+    ~CallGuard() {
+        if (!open) return;
+        if (side) (void)cudaStreamSynchronize(side);
+        if (cudaStream_t s = pme_stream(c)) (void)cudaStreamSynchronize(s);
+        if (c->stream) (void)cudaStreamSynchronize(c->stream);
+    }
+};
+/* 1 while a stream of the context (or `side`) holds work that has not finished. */
+int streams_pending(const mdrl_ctx *c, cudaStream_t side = nullptr);
 /* PME (mdrl_pme.cu): setup, teardown, the reciprocal part of a force evaluation, its energies. */
 mdrl_status pme_setup(mdrl_ctx *c, const mdrl_pme_params *p);
 void pme_free(mdrl_ctx *c);

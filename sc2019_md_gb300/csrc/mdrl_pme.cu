@@ -320,6 +320,8 @@ static double beta_for(double rc, double tol) {
     return 0.5 * (lo + hi);
 }
 
+cudaStream_t pme_stream(const mdrl_ctx *c) { return c->pme ? c->pme->stream : nullptr; }
+
 void pme_free(mdrl_ctx *c) {
     PmeState *s = c->pme;
     if (!s) return;
