@@ -258,7 +258,9 @@ mdrl_status mdrl_force_eval_device(mdrl_ctx *ctx, int n, const float *x, const f
 mdrl_status mdrl_pair_eval(mdrl_ctx *ctx, int n, const float *ref, const float *nbr,
                            const int *type_ref, const int *type_nbr, float *out, float *aux);
 
-/* Molecular dynamics on device-resident state.  set_state copies n particles in (velocities
+/* Molecular dynamics on device-resident state.  (Force evaluations and mdrl_bin work in the same
+ * buffers: after one that got as far as binning, also one that failed then, set_state comes first.)
+ * set_state copies n particles in (velocities
  * may be NULL: zero); step advances nsteps with the configured integrator, rebinning every
  * step; get_state copies positions, velocities and the last forces out in the original particle
  * order (any pointer may be NULL). */

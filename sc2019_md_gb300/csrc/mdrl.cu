@@ -659,15 +659,17 @@ static bool small_system(const mdrl_ctx *c, int n) {
     return n > 0 && n <= kSmallN && c->ncells <= kSmallCells && (long long)n * n <= 160000LL * c->ncells;
 }
 
-/* Bin user-order arrays (already on the device) into the sorted buffers of slot `buf`.  With
- * `spatial` the cells are ordered by Morton key (the force path's order), otherwise by index
- * (the reference's in-cell order). */
-/* Bin user-order inputs into cell order (buffer buf).  stage: the inputs may be host memory the
+/* Bin user-order inputs into cell order (buffer buf): with `spatial` each cell by Morton or Hilbert key
+ * (the force paths' orders), otherwise by index (the reference's in-cell order).  From here on the
+ * buffers hold these particles, whatever becomes of the call: a state that steps could go on from is
+ * gone (its forces are cleared, and a binning that is not spatial leaves counts behind that a step
+ * would take for zeros).  stage: the inputs may be host memory the
  * device reads directly; the binning pass copies them to the device staging buffers on the way
  * and the gather reads those.  inv: also record each user index's cell-order position. */
 static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, const float *z,
                             const float *q, const int *type, int buf, bool spatial, bool stage = false,
                             bool inv = false, bool hilbert = false) {
+    c->have_state = false;
     if (spatial && small_system(c, n)) {
         MDRL_TRY(prepare_force_kernel((force_fn)k_small_user, c->p.device));
         k_small_user<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
@@ -802,7 +804,6 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
         MDRL_CUDA(cudaMemcpyAsync(c->h_tot, c->d_tot, sizeof(DevTotals), cudaMemcpyDeviceToHost, c->stream));
         MDRL_CUDA(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     }
-    c->have_state = false; /* the sorted buffers now hold this evaluation */
     return MDRL_OK;
 }
 
@@ -1027,7 +1028,6 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
     MDRL_TRY(check_device_errors(c));
-    c->have_state = false;
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) != cudaSuccess) cudaGetLastError();
     return read_stats(c, st, ms);
@@ -1053,7 +1053,6 @@ extern "C" mdrl_status mdrl_bin(mdrl_ctx *c, int n, const float *x, const float 
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
     MDRL_TRY(check_device_errors(c));
-    c->have_state = false;
     return MDRL_OK;
 }
 

@@ -612,10 +612,12 @@ static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int
     return MDRL_OK;
 }
 
-/* Bin the user-order arrays already on the device into slot `buf` and clear the accumulators. */
+/* Bin the user-order arrays already on the device into slot `buf` and clear the accumulators.  A state
+ * and the last evaluation's results are gone from here on, whatever becomes of the call. */
 static mdrl_status batch_bin_user(mdrl_batch *b, const float *q, const int *type, int buf, bool hilbert = false) {
     mdrl_ctx *c = b->c;
     const int n = b->ntot;
+    c->have_state = b->have_eval = false;
     MDRL_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(int) * (size_t)b->ncells, c->stream));
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     k_bbin_user<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_ux, c->d_uy, c->d_uz, b->d_rep_of, b->d_reps,
@@ -698,7 +700,6 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     float ms = 0.0f;
     MDRL_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
     MDRL_TRY(check_device_errors(c));
-    c->have_state = false;
     b->have_eval = true;
     return batch_read_totals(b, st, ms);
 }
