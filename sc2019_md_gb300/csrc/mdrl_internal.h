@@ -68,6 +68,12 @@ void mix_pair_coefficients(const mdrl_params &p, std::vector<float> *pc, std::ve
 
 void set_error(const std::string &msg);
 
+/* The particle of a thread in a launch of CTAs of `threads` with `lanes` lanes per particle.  Formed from
+ * the CTA's first particle: the thread's index in the grid passes 2^31 from 2^31 / lanes particles on. */
+constexpr unsigned lane_particle(unsigned block, unsigned threads, unsigned thread, unsigned lanes) {
+    return block * (threads / lanes) + thread / lanes;
+}
+
 /* Host validation of a parameter block (box, cutoff, types, tables, modes, time step); sets the
  * error text and returns INVALID_ARG on the first failure. */
 mdrl_status validate_params(const mdrl_params *p);

@@ -108,9 +108,10 @@ template <int P>
 __global__ void __launch_bounds__(256) k_pme_spread(int n, const float4 *__restrict__ pos, PmeGeom pg,
                                                     unsigned long long *__restrict__ qfix) {
     constexpr int L = P == 4 ? 16 : 32;            /* lanes per particle */
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / L, l = threadIdx.x % L;
+    const int l = threadIdx.x % L;
+    const unsigned i = lane_particle(blockIdx.x, blockDim.x, threadIdx.x, L);
     const unsigned mask = L == 32 ? 0xffffffffu : 0xffffu << (threadIdx.x & 16);
-    if (i >= n) return;                            /* uniform over a particle's lanes */
+    if (i >= (unsigned)n) return;                  /* uniform over a particle's lanes */
     const float4 r = pos[i];
     const float q = r.w;
     if (q == 0.0f) return;
