@@ -155,7 +155,6 @@ bool list_eval(const mdrl_ctx *c);
 /* The totals of the last force launch (nunits result slots, nke kinetic-energy partials) into d_tot. */
 void launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy);
 mdrl_status list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid);
-inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 cudaStream_t pme_stream(const mdrl_ctx *c);    /* PME's own stream, or null without PME */
 

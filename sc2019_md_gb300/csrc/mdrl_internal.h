@@ -68,6 +68,9 @@ void mix_pair_coefficients(const mdrl_params &p, std::vector<float> *pc, std::ve
 
 void set_error(const std::string &msg);
 
+/* CTAs of b threads for n elements, for every n an int holds (n + b - 1 does not). */
+constexpr int nblk(int n, int b) { return n / b + (n % b != 0 ? 1 : 0); }
+
 /* The particle of a thread in a launch of CTAs of `threads` with `lanes` lanes per particle.  Formed from
  * the CTA's first particle: the thread's index in the grid passes 2^31 from 2^31 / lanes particles on. */
 constexpr unsigned lane_particle(unsigned block, unsigned threads, unsigned thread, unsigned lanes) {

@@ -31,3 +31,12 @@ def test_lanes_of_a_particle(tmp_path, lanes):
             for (unsigned t = 0; t < T; ++t)
                 CHECK((long long)lane_particle((unsigned)b, T, t, L) == b * per + t / L);
     """)
+
+
+def test_blocks_of_a_launch(tmp_path):
+    """Up to the largest int: mdrl_pair_eval copies 4 n elements for n up to 2^29 - 1."""
+    _run(tmp_path, """
+    for (long long n : {0LL, 1LL, 255LL, 256LL, 257LL, 4 * 536870848LL, 4 * 536870849LL, 4 * 536870911LL, (1LL << 31) - 1})
+        for (int b : {8, 16, 256})
+            CHECK(nblk((int)n, b) == (n + b - 1) / b);
+    """)
