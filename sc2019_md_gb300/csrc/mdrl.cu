@@ -1201,8 +1201,8 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
     }
     bool pg_out = false, pg_aux = false;
     const int *vtr = tref ? (const int *)device_view(c, tref, 4) : nullptr, *vtn = tnbr ? (const int *)device_view(c, tnbr, 4) : nullptr;
-    float4 *vout = (uintptr_t)out % 16 ? nullptr : (float4 *)device_view(c, out, 16, &pg_out);
-    float2 *vaux = !aux || (uintptr_t)aux % 8 ? nullptr : (float2 *)device_view(c, aux, 8, &pg_aux);
+    float4 *vout = (float4 *)device_view(c, out, 16, &pg_out);
+    float2 *vaux = aux ? (float2 *)device_view(c, aux, 8, &pg_aux) : nullptr;
     if (tref && !vtr) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptr, tref, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtr = c->d_ptr; }
     if (tnbr && !vtn) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptn, tnbr, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtn = c->d_ptn; }
     void *po = out, *pa = aux;

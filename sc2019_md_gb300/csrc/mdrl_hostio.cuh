@@ -29,9 +29,10 @@ constexpr size_t kPopulateChunk = size_t(8) << 20;   /* bytes per populating thr
 /* The device address of p when the context's device can read and write it in place: page-locked
  * host memory (cudaHostAlloc / cudaHostRegister, mapped), managed memory, memory of this device, or
  * pageable memory where the device walks the host's page tables (*pageable is then set); nullptr
- * otherwise (the caller stages through copies).  Kernels access whole elements, so a pageable address
- * that is not a multiple of `align` is left to the copies, which take any. */
+ * otherwise (the caller stages through copies).  Kernels access whole elements, so an address that is
+ * not a multiple of `align`, in whatever memory, is left to the copies, which take any. */
 inline void *device_view(const mdrl_ctx *c, const void *p, size_t align, bool *pageable = nullptr) {
+    if ((uintptr_t)p % align) return nullptr;
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
@@ -39,7 +40,7 @@ inline void *device_view(const mdrl_ctx *c, const void *p, size_t align, bool *p
     }
     if (a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged) return a.devicePointer;
     if (a.type == cudaMemoryTypeDevice && a.device == c->p.device) return a.devicePointer;
-    if (a.type != cudaMemoryTypeUnregistered || !c->host_tables || (uintptr_t)p % align) return nullptr;
+    if (a.type != cudaMemoryTypeUnregistered || !c->host_tables) return nullptr;
     if (pageable) *pageable = true;
     return const_cast<void *>(p);
 }
