@@ -893,7 +893,7 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
     for (int k = 0; k < 4 && direct; ++k) {
         if (!host[k]) continue;
         bool pageable = false;
-        view[k] = device_view(c, host[k], 4, &pageable);
+        view[k] = overlaps_another(host, 4, k, 4 * (size_t)n) ? nullptr : device_view(c, host[k], 4, &pageable);
         if (!view[k]) direct = false;
         else if (pageable) out.ptr[out.count++] = host[k];
     }
@@ -1200,9 +1200,14 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
         MDRL_CUDA(cudaMemcpyAsync(c->d_pn, nbr, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
     }
     bool pg_out = false, pg_aux = false;
-    const int *vtr = tref ? (const int *)device_view(c, tref, 4) : nullptr, *vtn = tnbr ? (const int *)device_view(c, tnbr, 4) : nullptr;
-    float4 *vout = (float4 *)device_view(c, out, 16, &pg_out);
-    float2 *vaux = aux ? (float2 *)device_view(c, aux, 8, &pg_aux) : nullptr;
+    const size_t bo = sizeof(float4) * (size_t)n, ba = sizeof(float2) * (size_t)n, bt = sizeof(int) * (size_t)n;
+    auto types = [&](const int *t) {    /* types in the results' storage are read before it is written */
+        return !t || overlap(t, bt, out, bo) || overlap(t, bt, aux, ba) ? nullptr : (const int *)device_view(c, t, 4);
+    };
+    const int *vtr = types(tref), *vtn = types(tnbr);
+    const bool apart = !overlap(out, bo, aux, ba);
+    float4 *vout = apart ? (float4 *)device_view(c, out, 16, &pg_out) : nullptr;
+    float2 *vaux = aux && apart ? (float2 *)device_view(c, aux, 8, &pg_aux) : nullptr;
     if (tref && !vtr) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptr, tref, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtr = c->d_ptr; }
     if (tnbr && !vtn) { MDRL_CUDA(cudaMemcpyAsync(c->d_ptn, tnbr, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream)); vtn = c->d_ptn; }
     void *po = out, *pa = aux;

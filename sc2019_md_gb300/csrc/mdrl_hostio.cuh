@@ -45,6 +45,19 @@ inline void *device_view(const mdrl_ctx *c, const void *p, size_t align, bool *p
     return const_cast<void *>(p);
 }
 
+/* Whether [a, a + na) and [b, b + nb) share a byte (null: no array). */
+inline bool overlap(const void *a, size_t na, const void *b, size_t nb) {
+    const uintptr_t pa = (uintptr_t)a, pb = (uintptr_t)b;
+    return a && b && pa < pb + nb && pb < pa + na;
+}
+
+/* Whether array k of `arrays` (equal sizes) shares storage with another one. */
+inline bool overlaps_another(const void *const *ptr, int arrays, int k, size_t bytes) {
+    for (int m = 0; m < arrays; ++m)
+        if (m != k && overlap(ptr[k], bytes, ptr[m], bytes)) return true;
+    return false;
+}
+
 /* Populate the pages of [p, p + bytes) for writing, contents kept: MADV_POPULATE_WRITE, or an atomic
  * OR of 0 into every page where the kernel has no such advice. */
 inline void populate_range(char *p, size_t bytes) {
@@ -98,7 +111,8 @@ static __global__ void k_copy_arrays(int n, Arrays a) {
 }
 
 /* Enqueue the copies of n 4-byte elements src[k] -> dst[k] (null entries are skipped) between host and
- * device: one kernel for the arrays the device can use in place, cudaMemcpyAsync for the others.  The
+ * device: one kernel for the arrays the device can use in place, cudaMemcpyAsync for the others, and for
+ * host arrays that share storage (written one after the other, so that the later one's values stay).  The
  * caller synchronises the stream before it returns.  (Named for what it replaces: an injected failure
  * of cudaMemcpyAsync, which goes by the text of the call, is one of this too.) */
 inline cudaError_t cudaMemcpyAsyncArrays(mdrl_ctx *c, int n, int arrays, const void *const *src, void *const *dst,
@@ -109,7 +123,8 @@ inline cudaError_t cudaMemcpyAsyncArrays(mdrl_ctx *c, int n, int arrays, const v
     for (int k = 0; k < arrays && n > 0; ++k) {
         if (!src[k] || !dst[k]) continue;
         bool pageable = false;
-        void *v = device_view(c, to_host ? dst[k] : src[k], 4, &pageable);
+        void *v = to_host && overlaps_another(dst, arrays, k, 4 * (size_t)n)
+                      ? nullptr : device_view(c, to_host ? dst[k] : src[k], 4, &pageable);
         if (!v) {
             const cudaError_t e = cudaMemcpyAsync(dst[k], src[k], 4 * (size_t)n,
                                                   to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, c->stream);
