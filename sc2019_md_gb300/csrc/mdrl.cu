@@ -884,7 +884,7 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
     }
     const void *src[5] = {x, y, z, q, type};
     void *dst[5] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 5, src, dst, false));
+    MDRL_TRY(copy_arrays(c, n, 5, src, dst, false));
     /* the forces go to the caller's arrays in place when the device can write them all */
     void *host[4] = {fx, fy, fz, counts}, *view[4] = {nullptr, nullptr, nullptr, nullptr};
     const void *dev[4] = {c->d_ox, c->d_oy, c->d_oz, c->d_ocnt};
@@ -902,7 +902,7 @@ extern "C" mdrl_status mdrl_force_eval(mdrl_ctx *c, int n, const float *x, const
     MDRL_TRY(force_eval_enqueue(c, n, c->d_ux, c->d_uy, c->d_uz, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr,
                                 (float *)view[0], (float *)view[1], (float *)view[2], (int *)view[3], false,
                                 direct ? &out : nullptr));
-    if (!direct) MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, dev, host, true));
+    if (!direct) MDRL_TRY(copy_arrays(c, n, 4, dev, host, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));   /* the one synchronisation of the call */
     guard.done();
     return force_eval_finish(c, st);
@@ -1002,7 +1002,7 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     if (n > 0 && !direct) {
         const void *src[5] = {x, y, z, q, type};
         void *dst[5] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut};
-        MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 5, src, dst, false));
+        MDRL_TRY(copy_arrays(c, n, 5, src, dst, false));
         dx = c->d_ux; dy = c->d_uy; dz = c->d_uz;
         dq = q ? c->d_uq : nullptr;
         dt = type ? c->d_ut : nullptr;
@@ -1044,11 +1044,11 @@ extern "C" mdrl_status mdrl_bin(mdrl_ctx *c, int n, const float *x, const float 
     CallGuard guard(c);
     const void *src[3] = {x, y, z};
     void *dst[3] = {c->d_ux, c->d_uy, c->d_uz};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 3, src, dst, false));
+    MDRL_TRY(copy_arrays(c, n, 3, src, dst, false));
     MDRL_TRY(bin_user(c, n, c->d_ux, c->d_uy, c->d_uz, nullptr, nullptr, 0, false));
     const void *bsrc[2] = {c->d_cell_of, c->d_sorted};
     void *bdst[2] = {cell_of, order};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 2, bsrc, bdst, true));
+    MDRL_TRY(copy_arrays(c, n, 2, bsrc, bdst, true));
     if (cell_count) MDRL_CUDA(cudaMemcpyAsync(cell_count, c->d_count, sizeof(int) * c->ncells, cudaMemcpyDeviceToHost, c->stream));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
@@ -1194,7 +1194,7 @@ extern "C" mdrl_status mdrl_pair_eval(mdrl_ctx *c, int n, const float *ref, cons
     const bool small = n <= 0x7fffffff / 4;
     const void *src[2] = {ref, nbr};
     void *dst[2] = {c->d_pr, c->d_pn};
-    if (small) MDRL_CUDA(cudaMemcpyAsyncArrays(c, 4 * n, 2, src, dst, false));
+    if (small) MDRL_TRY(copy_arrays(c, 4 * n, 2, src, dst, false));
     else {
         MDRL_CUDA(cudaMemcpyAsync(c->d_pr, ref, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
         MDRL_CUDA(cudaMemcpyAsync(c->d_pn, nbr, sizeof(float4) * n, cudaMemcpyHostToDevice, c->stream));
@@ -1244,7 +1244,7 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     CallGuard guard(c);
     const void *src[8] = {x, y, z, q, type, vx, vy, vz};
     void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 8, src, dst, false));
+    MDRL_TRY(copy_arrays(c, n, 8, src, dst, false));
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     c->cur = 0;
     MDRL_TRY(bin_user(c, n, c->d_ux, c->d_uy, c->d_uz, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0, true));
@@ -1398,7 +1398,7 @@ extern "C" mdrl_status mdrl_get_state(mdrl_ctx *c, float *x, float *y, float *z,
     MDRL_CUDA(cudaGetLastError());
     void *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
     const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
+    MDRL_TRY(copy_arrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
     return MDRL_OK;

@@ -639,7 +639,7 @@ static mdrl_status upload_user(mdrl_batch *b, const float *x, const float *y, co
     mdrl_ctx *c = b->c;
     const void *src[8] = {x, y, z, q, type, vx, vy, vz};
     void *dst[8] = {c->d_ux, c->d_uy, c->d_uz, c->d_uq, c->d_ut, c->d_ovx, c->d_ovy, c->d_ovz};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, b->ntot, 8, src, dst, false));
+    MDRL_TRY(copy_arrays(c, b->ntot, 8, src, dst, false));
     return MDRL_OK;
 }
 
@@ -694,7 +694,7 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     MDRL_CUDA(cudaEventRecord(c->ev1, c->stream));
     const void *src[4] = {c->d_ox, c->d_oy, c->d_oz, c->d_ocnt};
     void *dst[4] = {fx, fy, fz, counts};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 4, src, dst, true));
+    MDRL_TRY(copy_arrays(c, n, 4, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
     float ms = 0.0f;
@@ -821,7 +821,7 @@ extern "C" mdrl_status mdrl_batch_get_state(mdrl_batch *b, float *x, float *y, f
     MDRL_CUDA(cudaGetLastError());
     void *dst[9] = {x, y, z, vx, vy, vz, fx, fy, fz};
     const void *src[9] = {c->d_ux, c->d_uy, c->d_uz, c->d_ovx, c->d_ovy, c->d_ovz, c->d_ox, c->d_oy, c->d_oz};
-    MDRL_CUDA(cudaMemcpyAsyncArrays(c, n, 9, src, dst, true));
+    MDRL_TRY(copy_arrays(c, n, 9, src, dst, true));
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
     return MDRL_OK;

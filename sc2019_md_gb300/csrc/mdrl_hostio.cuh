@@ -113,10 +113,13 @@ static __global__ void k_copy_arrays(int n, Arrays a) {
 /* Enqueue the copies of n 4-byte elements src[k] -> dst[k] (null entries are skipped) between host and
  * device: one kernel for the arrays the device can use in place, cudaMemcpyAsync for the others, and for
  * host arrays that share storage (written one after the other, so that the later one's values stay).  The
- * caller synchronises the stream before it returns.  (Named for what it replaces: an injected failure
- * of cudaMemcpyAsync, which goes by the text of the call, is one of this too.) */
-inline cudaError_t cudaMemcpyAsyncArrays(mdrl_ctx *c, int n, int arrays, const void *const *src, void *const *dst,
-                                         bool to_host) {
+ * caller synchronises the stream before it returns.  An injected failure of cudaMemcpyAsync (fault_hit)
+ * is one of this too, whichever way the arrays go. */
+inline mdrl_status copy_arrays(mdrl_ctx *c, int n, int arrays, const void *const *src, void *const *dst, bool to_host) {
+    if (fault_hit("cudaMemcpyAsync")) {
+        set_error("cudaMemcpyAsync of the call's arrays: injected failure (MDRL_FAULT)");
+        return MDRL_ERR_CUDA;
+    }
     Arrays a;
     void *fresh[kMaxArrays];
     int nfresh = 0;
@@ -126,9 +129,8 @@ inline cudaError_t cudaMemcpyAsyncArrays(mdrl_ctx *c, int n, int arrays, const v
         void *v = to_host && overlaps_another(dst, arrays, k, 4 * (size_t)n)
                       ? nullptr : device_view(c, to_host ? dst[k] : src[k], 4, &pageable);
         if (!v) {
-            const cudaError_t e = cudaMemcpyAsync(dst[k], src[k], 4 * (size_t)n,
-                                                  to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, c->stream);
-            if (e != cudaSuccess) return e;
+            MDRL_CUDA(cudaMemcpyAsync(dst[k], src[k], 4 * (size_t)n, to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice,
+                                      c->stream));
             continue;
         }
         a.src[a.count] = (const uint32_t *)(to_host ? src[k] : v);
@@ -137,7 +139,8 @@ inline cudaError_t cudaMemcpyAsyncArrays(mdrl_ctx *c, int n, int arrays, const v
     }
     populate(fresh, nfresh, 4 * (size_t)n);
     if (a.count) k_copy_arrays<<<nblk(n, 256), 256, 0, c->stream>>>(n, a);
-    return cudaGetLastError();
+    MDRL_CUDA(cudaGetLastError());
+    return MDRL_OK;
 }
 
 }  // namespace mdrl
