@@ -132,7 +132,8 @@ typedef struct mdrl_ctx mdrl_ctx;
  * groups each unit is split into, and prune_steps must be 1 (the kernel always prunes).
  * Default {4, 6, 0}; mdrl_autotune picks among both kinds.
  * Force evaluations (mdrl_force_eval*, mdrl_batch_force_eval; MDRL_ACC_FIXED64) run a third kernel,
- * over particle lists, until a CTA tile is asked for; under {1, groups, 1} groups splits its items,
+ * over particle lists, until a CTA tile is asked for by mdrl_set_tile / mdrl_batch_set_tile (the
+ * tuner's choice is for dynamics, and ends an earlier call's); under {1, groups, 1} groups splits its items,
  * without effect on the result. */
 typedef struct {
     int warps_per_cta;
@@ -415,7 +416,11 @@ mdrl_status mdrl_get_pme(mdrl_ctx *ctx, mdrl_pme_params *p, int *enabled);
 mdrl_status mdrl_set_tile(mdrl_ctx *ctx, const mdrl_tile *tile);
 mdrl_status mdrl_get_tile(mdrl_ctx *ctx, mdrl_tile *tile);
 mdrl_status mdrl_autotune(mdrl_ctx *ctx, int flags, mdrl_tile *best, float *best_ms, float *default_ms);
-/* The same for a batch (4 warps per CTA; steps per piece and pruning tuned), after
+/* Which force kernel (MDRL_KERNEL_*) an evaluation and a step of the context take now, and the kernels
+ * that one step launches (0 before the first step, which builds the graph).  Any pointer may be NULL. */
+enum { MDRL_KERNEL_CTA = 0, MDRL_KERNEL_WARP = 1, MDRL_KERNEL_LIST = 2, MDRL_KERNEL_NARROW = 3 };
+mdrl_status mdrl_get_kernels(mdrl_ctx *ctx, int *eval_kernel, int *step_kernel, int *step_launches);
+/* Tiles and the tuner for a batch (4 warps per CTA; steps per piece and pruning tuned), after
  * mdrl_batch_set_state. */
 mdrl_status mdrl_batch_set_tile(mdrl_batch *batch, const mdrl_tile *tile);
 mdrl_status mdrl_batch_autotune(mdrl_batch *batch, int flags, mdrl_tile *best, float *best_ms,

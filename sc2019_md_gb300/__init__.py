@@ -194,13 +194,15 @@ def lib() -> C.CDLL:
     L.mdrl_batch_set_pair_coefficients.argtypes = [vp, _D]
     L.mdrl_set_tile.argtypes = [vp, C.POINTER(Tile)]
     L.mdrl_get_tile.argtypes = [vp, C.POINTER(Tile)]
+    L.mdrl_get_kernels.argtypes = [vp, _I, _I, _I]
     L.mdrl_autotune.argtypes = [vp, st, C.POINTER(Tile), _F, _F]
     L.mdrl_batch_set_tile.argtypes = [vp, C.POINTER(Tile)]
     L.mdrl_batch_autotune.argtypes = [vp, st, C.POINTER(Tile), _F, _F]
     for name in ("mdrl_set_pme", "mdrl_get_pme", "mdrl_set_pair_coefficients", "mdrl_batch_set_pair_coefficients", "mdrl_set_tile", "mdrl_get_tile", "mdrl_autotune", "mdrl_batch_set_tile", "mdrl_batch_autotune",
                  "mdrl_batch_create", "mdrl_batch_destroy", "mdrl_batch_layout", "mdrl_batch_force_eval",
                  "mdrl_batch_set_state", "mdrl_batch_step", "mdrl_batch_get_state",
-                 "mdrl_batch_replica_stats", "mdrl_batch_time_force", "mdrl_pending", "mdrl_batch_pending"):
+                 "mdrl_batch_replica_stats", "mdrl_batch_time_force", "mdrl_pending", "mdrl_batch_pending",
+                 "mdrl_get_kernels"):
         getattr(L, name).restype = st
     for name in ("mdrl_fit_tables", "mdrl_fit_tables_bin_local", "mdrl_get_table_form", "mdrl_slab_plan",
                  "mdrl_slab_select", "mdrl_force_eval_fixed", "mdrl_create", "mdrl_destroy", "mdrl_set_tables",
@@ -487,6 +489,14 @@ class Context:
         t = Tile()
         _check(lib().mdrl_get_tile(self._h, C.byref(t)))
         return t.as_tuple()
+
+    def kernels(self) -> dict:
+        """The force kernels that an evaluation and a step take now ("cta", "warp", "list" or "narrow"), and
+        the launches of one step (0 before the first)."""
+        e, s, n = C.c_int(), C.c_int(), C.c_int()
+        _check(lib().mdrl_get_kernels(self._h, C.byref(e), C.byref(s), C.byref(n)))
+        names = ("cta", "warp", "list", "narrow")
+        return {"eval": names[e.value], "step": names[s.value], "step_launches": n.value}
 
     def autotune(self, retime: bool = False) -> dict:
         """Time every candidate tile on the current state and keep the fastest."""

@@ -487,13 +487,14 @@ force_fn pick_force_batch(int order, bool sep, bool extra, bool prune) {
 }
 }  // namespace mdrl
 
-/* Force evaluations take the list kernel unless a CTA tile was asked for: it is the faster one at
+/* Force evaluations take the list kernel unless a caller asked for a CTA tile (the tuner times dynamics'
+ * kernels, so its choice says nothing here): it is the faster one at
  * every size measured (92k system, order 1: 250 us against 577 us for the default CTA tile and 374 us
  * for {1, 1, 1}; 1M system, order 2: 1.71 ms against 4.06 and 2.61; 1,728 atoms: within 2 us of the
  * CTA kernel's 18 us).  Dynamics keeps the kernels of its tile: its FP32 partial sums, and so every
  * bit of a trajectory, stay those of runs made before. */
 bool mdrl::list_eval(const mdrl_ctx *c) {
-    return c->p.accum == MDRL_ACC_FIXED64 && (!c->tile_set || c->tile.warps_per_cta == 1);
+    return c->p.accum == MDRL_ACC_FIXED64 && (!c->tile_asked || c->tile.warps_per_cta == 1);
 }
 
 mdrl_status mdrl::list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid) {
@@ -529,7 +530,7 @@ int mdrl::eff_order(const mdrl_ctx *c) { return c->p.eval == MDRL_EVAL_DIRECT ? 
  * slots, one per item. */
 static mdrl_status launch_list(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, int cell0, int cells,
                                int *slots) {
-    const int G = c->tile_set ? c->tile.steps_per_piece : 1;
+    const int G = c->tile_asked ? c->tile.steps_per_piece : 1;
     bool fine;
     int items = 0, grid = 0;
     const int cfg = list_cfg(n, c->ncells, cells, G, c->num_sms, &fine, &items);
@@ -1436,9 +1437,9 @@ static mdrl_status check_tile(const mdrl_tile *t, bool allow8, bool allow_prune,
 }
 
 namespace mdrl {
-mdrl_status set_tile(mdrl_ctx *c, const mdrl_tile *t, bool allow8, bool allow_warp) {
+mdrl_status set_tile(mdrl_ctx *c, const mdrl_tile *t, bool allow8, bool allow_warp, bool asked) {
     MDRL_TRY(check_tile(t, allow8, c->p.accum == MDRL_ACC_FIXED64, allow_warp));
-    c->tile_set = true;
+    c->tile_asked = asked;
     if (t->warps_per_cta != c->tile.warps_per_cta || t->steps_per_piece != c->tile.steps_per_piece ||
         t->prune_steps != c->tile.prune_steps) {
         MDRL_CUDA(cudaSetDevice(c->p.device));
@@ -1504,12 +1505,35 @@ static const int kTuneSpp[] = {3, 4, 6, 8, 12};
 
 extern "C" mdrl_status mdrl_set_tile(mdrl_ctx *c, const mdrl_tile *t) {
     if (!c || !t) { set_error("mdrl_set_tile: null argument"); return MDRL_ERR_INVALID_ARG; }
-    return set_tile(c, t, c->p.accum == MDRL_ACC_FIXED64, c->p.accum == MDRL_ACC_FIXED64);
+    return set_tile(c, t, c->p.accum == MDRL_ACC_FIXED64, c->p.accum == MDRL_ACC_FIXED64, true);
 }
 
 extern "C" mdrl_status mdrl_get_tile(mdrl_ctx *c, mdrl_tile *t) {
     if (!c || !t) { set_error("mdrl_get_tile: null argument"); return MDRL_ERR_INVALID_ARG; }
     *t = c->tile;
+    return MDRL_OK;
+}
+
+extern "C" mdrl_status mdrl_get_kernels(mdrl_ctx *c, int *eval_kernel, int *step_kernel, int *step_launches) {
+    if (!c) { set_error("mdrl_get_kernels: null context"); return MDRL_ERR_INVALID_ARG; }
+    const int of_tile = c->tile.warps_per_cta == 1 ? MDRL_KERNEL_WARP : MDRL_KERNEL_CTA;
+    if (eval_kernel) *eval_kernel = list_eval(c) ? MDRL_KERNEL_LIST : of_tile;
+    if (step_kernel) *step_kernel = narrow_force(c) ? MDRL_KERNEL_NARROW : of_tile;
+    if (!step_launches) return MDRL_OK;
+    *step_launches = 0;
+    for (int k = 0; k < 4 && !*step_launches; ++k) {
+        if (!c->graph_exec[k]) continue;
+        size_t n = 0;
+        MDRL_CUDA(cudaGraphGetNodes(c->graph[k], nullptr, &n));
+        std::vector<cudaGraphNode_t> node(n);
+        MDRL_CUDA(cudaGraphGetNodes(c->graph[k], node.data(), &n));
+        for (cudaGraphNode_t v : node) {
+            cudaGraphNodeType type;
+            MDRL_CUDA(cudaGraphNodeGetType(v, &type));
+            *step_launches += type == cudaGraphNodeTypeKernel;
+        }
+        if (k >= 2) *step_launches /= 2;
+    }
     return MDRL_OK;
 }
 
@@ -1522,7 +1546,7 @@ extern "C" mdrl_status mdrl_autotune(mdrl_ctx *c, int flags, mdrl_tile *best, fl
     snprintf(buf, sizeof buf, "ctx-%dx%dx%d-p%d-", c->g.nc[0], c->g.nc[1], c->g.nc[2], ppc8);
     const std::string key = std::string(buf) + tune_key_common(c);
     auto time_tile = [&](const mdrl_tile &t, float *ms) -> mdrl_status {
-        MDRL_TRY(set_tile(c, &t, true, true));
+        MDRL_TRY(set_tile(c, &t, true, true, false));
         float v[5];
         for (int r = 0; r < 5; ++r) MDRL_TRY(mdrl_time_force(c, &v[r]));
         std::sort(v, v + 5);
@@ -1559,7 +1583,7 @@ extern "C" mdrl_status mdrl_autotune(mdrl_ctx *c, int flags, mdrl_tile *best, fl
             }
         tune_store(key, pick, pick_ms);
     }
-    MDRL_TRY(set_tile(c, &pick, true, true));
+    MDRL_TRY(set_tile(c, &pick, true, true, false));
     if (best) *best = pick;
     if (best_ms) *best_ms = pick_ms;
     if (default_ms) *default_ms = def_ms;

@@ -544,7 +544,7 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
 
 /* The list kernel's items of list k (0 min-image, 1 half-shell) and whether they are fine ones. */
 static int list_items(const mdrl_batch *b, int k, bool *fine) {
-    const int items = b->lists[k].items * (b->c->tile_set ? b->c->tile.steps_per_piece : 1);
+    const int items = b->lists[k].items * (b->c->tile_asked ? b->c->tile.steps_per_piece : 1);
     *fine = fine_items(b->lists[k].tile_groups, items, b->c->num_sms);
     return *fine ? items * kRuns : items;
 }
@@ -555,7 +555,7 @@ static mdrl_status launch_lists(mdrl_batch *b, cudaStream_t st, const float4 *po
                                 int *slots) {
     mdrl_ctx *c = b->c;
     const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
-    const int G = c->tile_set ? c->tile.steps_per_piece : 1;
+    const int G = c->tile_asked ? c->tile.steps_per_piece : 1;
     const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
     DevTotals *tot = extra ? nullptr : c->d_tot;
     for (int k = 0; k < 2; ++k) {
@@ -905,7 +905,7 @@ extern "C" mdrl_status mdrl_batch_time_force(mdrl_batch *b, float *ms) {
 extern "C" mdrl_status mdrl_batch_set_tile(mdrl_batch *b, const mdrl_tile *t) {
     if (!b || !t) { set_error("mdrl_batch_set_tile: null argument"); return MDRL_ERR_INVALID_ARG; }
     const mdrl_tile before = b->c->tile;
-    MDRL_TRY(set_tile(b->c, t, false, true));
+    MDRL_TRY(set_tile(b->c, t, false, true, true));
     /* another tile lays the result slots out differently: the last evaluation's no longer apply */
     if (before.warps_per_cta != t->warps_per_cta || before.steps_per_piece != t->steps_per_piece ||
         before.prune_steps != t->prune_steps)
@@ -923,7 +923,7 @@ extern "C" mdrl_status mdrl_batch_autotune(mdrl_batch *b, int flags, mdrl_tile *
     snprintf(buf, sizeof buf, "batch-r%d-n%d-c%d-i%d-", b->nrep, b->ntot, b->ncells, b->nitems);
     const std::string key = std::string(buf) + tune_key_common(c);
     auto time_tile = [&](const mdrl_tile &t, float *ms) -> mdrl_status {
-        MDRL_TRY(set_tile(c, &t, false, true));
+        MDRL_TRY(set_tile(c, &t, false, true, false));
         float v[5];
         for (int r = 0; r < 5; ++r) MDRL_TRY(mdrl_batch_time_force(b, &v[r]));
         std::sort(v, v + 5);
@@ -956,7 +956,7 @@ extern "C" mdrl_status mdrl_batch_autotune(mdrl_batch *b, int flags, mdrl_tile *
         }
         tune_store(key, pick, pick_ms);
     }
-    MDRL_TRY(set_tile(c, &pick, false, true));
+    MDRL_TRY(set_tile(c, &pick, false, true, false));
     b->have_eval = false;   /* the timings overwrote the result slots */
     if (best) *best = pick;
     if (best_ms) *best_ms = pick_ms;

@@ -137,7 +137,7 @@ struct mdrl_ctx {
 
     /* force-kernel tile (mdrl_set_tile / mdrl_autotune) */
     mdrl_tile tile = {mdrl::kFW, mdrl::kStepsPerPiece, 0};
-    bool tile_set = false;       /* by a caller or the tuner */
+    bool tile_asked = false;     /* by a caller (the tuner's choice is for dynamics alone) */
     bool batch = false;          /* the buffers of an mdrl_batch (which sizes d_unit itself) */
 };
 
@@ -194,7 +194,7 @@ mdrl_status upload_tables(mdrl_ctx *c);
 /* Tiles: change (re-capturing graphs), and the autotuner's process-wide cache. */
 /* allow8: 8-warp CTAs and pruning (fixed point, one system); allow_warp: one warp per item
  * (fixed point) */
-mdrl_status set_tile(mdrl_ctx *c, const mdrl_tile *t, bool allow8, bool allow_warp);
+mdrl_status set_tile(mdrl_ctx *c, const mdrl_tile *t, bool allow8, bool allow_warp, bool asked);
 bool tune_lookup(const std::string &key, mdrl_tile *t);
 void tune_store(const std::string &key, const mdrl_tile &t, float ms);
 std::string tune_key_common(const mdrl_ctx *c);
