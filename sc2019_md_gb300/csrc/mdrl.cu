@@ -570,14 +570,20 @@ static bool narrow_force(const mdrl_ctx *c) {
  * 64 cells, 43 against 45 in 196, 47 against 71 in 392; up to 60 argon atoms in 216 cells 43 against 53.
  * Above 64 on average they pay where the last wave counts for little: 90,000 atoms with 68 per cell (7.7
  * waves) 227 against 329 us, 5,000 with 78 53 against 34.  Allocates the scratch that cells crowded by
- * later steps use; where it can't be had, the CTA kernel stays. */
+ * later steps use, 24 KB for each warp of the launch (at most one per unit: 9 MB for 27 cells, 60 MB from
+ * 174 cells on), and gives it back with a state that has no use for it; where it can't be had, the CTA
+ * kernel stays.  (One accumulator at a time in shared memory needs no scratch, but takes the crowded
+ * units 1.3 to 2.1 times as long, and its registers cost every launch 7 %: 23,558-atom chains, where some
+ * cells pass 96 within a few hundred steps, 1,194 -> 1,253 us per 10 steps.) */
 static void plan_narrow(mdrl_ctx *c, int n, int max_occ) {
     const bool was = c->narrow;
     const long long slots = (long long)kNarrowCtas * std::max(1, c->num_sms);
     const long long units = (long long)c->ncells * kHalfShellCells;
     c->narrow = n > 0 && max_occ <= kNarrowCell && c->p.accum == MDRL_ACC_FIXED64 &&
                 (max_occ <= 32 || units >= (n <= 64LL * c->ncells ? 1 : 4) * slots);
-    if (c->narrow && !c->d_narrow && dalloc(&c->d_narrow, kNarrowScratch * (size_t)slots) != MDRL_OK) {
+    if (!c->narrow) {
+        dfree(&c->d_narrow);
+    } else if (!c->d_narrow && dalloc(&c->d_narrow, kNarrowScratch * (size_t)std::min(units, slots)) != MDRL_OK) {
         (void)cudaGetLastError();
         c->narrow = false;
     }
