@@ -1,12 +1,30 @@
-"""The narrow kernel's scratch is sized by the system."""
+"""The two runs that tests/test_gpu_narrow.py compares take different kernels, and the narrow one's
+scratch is sized by the system."""
 import numpy as np
 import pytest
 import torch
 
 import sc2019_md_gb300 as m
-from test_gpu_narrow import RC
+from test_gpu_narrow import BOX, DT, RC, arrays  # noqa: F401
 
 pytestmark = pytest.mark.gpu
+
+
+def _context():
+    return m.Context(m.default_params(box=BOX, cutoff=RC, ntypes=3, sigma=[1.2, 1.5, 1.8], epsilon=[0.05, 0.1, 0.2],
+                                      mass=[12.0, 14.0, 16.0], coulomb_k=332.06371, dt_fs=DT))
+
+
+def test_each_run_takes_its_kernel(arrays):  # noqa: F811
+    pos, vel, q, ty, nb = arrays
+    for n, want in ((nb, "narrow"), (len(pos), "cta")):
+        with _context() as ctx:
+            ctx.set_state(pos[:n, 0], pos[:n, 1], pos[:n, 2], vel[:n], q[:n], ty[:n])
+            assert ctx.kernels()["step"] == want
+            ctx.step(1)
+            assert ctx.kernels()["step"] == want
+            ctx.set_tile(1, 1, 1)
+            assert ctx.kernels()["step"] == "warp"
 
 
 def test_scratch_of_a_small_system():
