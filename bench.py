@@ -39,9 +39,6 @@ sys.path.insert(0, str(ROOT))
 
 FLOPS_PER_PAIR = 28            # algorithmic flops per in-cutoff pair, force only
 BYTES_PER_PARTICLE = 16 + 4 + 24   # pos+q and type read, int64 x3 force atomics, per force launch
-# kernels of a step without energies: kick+drift+bin, scan, scatter, sort, gather, force, kick; systems of
-# up to 4,096 particles bin, sort and gather in one
-STEP_LAUNCHES, SMALL_STEP_LAUNCHES = 7, 3
 L2_FLUSH_BYTES = 256 << 20     # > 129 MB L2
 METRIC = "pair-evals/s & ns/day, 92k-atom RL LJ+Coulomb, tuned vs plain @1e-5 force err"
 CAPTURES = ROOT / "profiles" / "ncu_captures.json"   # per-capture ncu figures (workload, tile, datapath)
@@ -233,7 +230,8 @@ def md_leg(m, obj, steps: int, warmup: int, flush, nkernel: int = 12):
         flush()
         fms.append(obj.time_force())
     return {"dev_ms": dev_ms, "pairs": pairs, "pairs_per_step": float(np.mean(pstep)) if pstep else 0.0,
-            "force_ms": float(np.median(fms)), "steps": steps}
+            "force_ms": float(np.median(fms)), "steps": steps,
+            "step_launches": obj.kernels()["step_launches"] if hasattr(obj, "kernels") else None}
 
 
 def force_eval_pinned(m, ctx, bufs, n):
@@ -261,7 +259,8 @@ def e2e_leg(m, params, sysm, tile, warmup: int, calls: int, flush):
                  ("t", sysm.type)):
         bufs[k][:] = v
     with m.Context(params) as ctx:
-        ctx.set_tile(*tile)
+        if tile:                       # a tuned tile is for dynamics; evaluations take one that is asked for
+            ctx.set_tile(*tile)
         for _ in range(warmup):
             force_eval_pinned(m, ctx, bufs, n)
         secs, pairs, dev = 0.0, 0, 0.0
@@ -394,7 +393,7 @@ def single_system(m, sysm, args, local, flush, clocks=None, barrier=lambda: None
         out["reference_datapath"] = md_leg(m, ctx, kp, args.warmup, flush, nkernel=5)
         out["reference_datapath"]["tile"] = rtune["tile"]
 
-    out["e2e"] = e2e_leg(m, p_tuned, sysm, tune["tile"], args.warmup, max(3, min(args.steps, 30)), flush)
+    out["e2e"] = e2e_leg(m, p_tuned, sysm, args.tile, args.warmup, max(3, min(args.steps, 30)), flush)
     return out
 
 
@@ -414,7 +413,7 @@ def sub_workload_single(m, sysm, args, local, flush, props):
     with m.Context(p_p) as ctx:
         ctx.set_state(*st_args)
         plain = md_leg(m, ctx, k, args.warmup, flush, nkernel=5)
-    e2e = e2e_leg(m, p_t, sysm, tune["tile"], 2, 3, flush)
+    e2e = e2e_leg(m, p_t, sysm, None, 2, 3, flush)
     mhz = measured_peaks().get("sm_max_mhz") or 2070.0
     ms = tuned["dev_ms"] / k
     return {
@@ -433,7 +432,7 @@ def sub_workload_single(m, sysm, args, local, flush, props):
                 "d2h_bytes_per_step": sysm.n * 12, "calls": e2e["calls"],
                 "ms_per_call": e2e["secs"] / e2e["calls"] * 1e3},
         "pairs_per_step": tuned["pairs_per_step"],
-        "gpu_launches": STEP_LAUNCHES * k,
+        "gpu_launches": tuned["step_launches"] * k,
     }
 
 
@@ -456,7 +455,8 @@ def sub_workload_batch(m, reps, args, local, flush, props):
             tune = b.autotune(retime=True)
         leg = md_leg(m, b, k, args.warmup, flush, nkernel=5)
     with m.Batch(params, spec) as b:       # e2e: host arrays in and out (copies inside the call)
-        b.set_tile(*tune["tile"])
+        if args.tile:
+            b.set_tile(*args.tile)
         b.force(pos[:, 0], pos[:, 1], pos[:, 2], q, t)
         e_secs, e_pairs = 0.0, 0
         for _ in range(3):
@@ -497,7 +497,8 @@ def sub_workload_batch(m, reps, args, local, flush, props):
                 "d2h_bytes_per_step": ntot * 12, "calls": 3, "ms_per_call": e_secs / 3 * 1e3,
                 "call": "mdrl_batch_force_eval (host x,y,z,q,type in; fx,fy,fz out)"},
         "pairs_per_step": leg["pairs_per_step"],
-        "gpu_launches": 9 * k,
+        # binning to gather, kick, and the force launch: one, or with a warp tile one per kind of replica
+        "gpu_launches": (6 + (int((npath > 0).sum()) if tune["tile"][0] == 1 else 1)) * k,
     }
 
 
@@ -613,7 +614,7 @@ def run_ours(args, rank, world, local, dist):
                 "host_link": "pinned buffers read and written in place by the binning and unsort kernels"},
         "with_pme": pme_out,
         "bonded": bonded_out,
-        "gpu_launches": (SMALL_STEP_LAUNCHES if sysm.n <= 4096 else STEP_LAUNCHES) * args.steps,
+        "gpu_launches": tuned["step_launches"] * args.steps,
         "clocks": clk,
         "wall_s": res["wall_s"],
     }
