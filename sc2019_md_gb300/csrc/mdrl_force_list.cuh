@@ -19,13 +19,15 @@
  *      i-particles, which are the same in every lane.  Only the table loads depend on the filter
  *      0 < r2 <= rc2; a rejected candidate's scalar force is selected to 0.  The j force of the 4 is
  *      added to the warp's accumulator in shared memory (a lane owns its j: no shuffles), and the i
- *      forces stay in registers until the group's list ends (one reduce-scatter);
- *   4. adds the list's j forces, and at the end of a run of ranges with one periodic shift the tile's
- *      i forces, to the global accumulators (one atomic per particle and component).
+ *      forces stay in registers until the group's list ends (one reduce-scatter, then to the global
+ *      accumulators: kept in shared memory until a run of lists ends they would be FP32 sums over
+ *      any number of cells);
+ *   4. adds the list's j forces to the global accumulators (one atomic per particle and component).
+ *      So no FP32 sum holds more than one list's 256 j, or one tile's 32 i.
  * The two levels of lists only drop candidates that cannot be pairs: the box test of
  * mdrl_force_warp.cuh (tests/test_cull_bound.py) with one particle for the second box.  So the accepted
  * pairs are those of the plain traversal, bit for bit.  Deterministic: every FP32 partial sum is of one
- * tile, one run and one list, whose order follows from the particles of its cells alone, and the int64
+ * tile and one list, whose order follows from the particles of its cells alone, and the int64
  * global sums are exact; so the result does not depend on scheduling, on S, or on what else a launch
  * holds (other replicas, other slabs), nor on whether the items are fine (below).
  *
@@ -172,7 +174,6 @@ struct ListSmem {
     float4 i[32];                        /* tile: x, y, z (shifted), ke q */
     float4 g[kTileGroups][2];            /* group boxes: centre, half widths + margin (far: empty) */
     float fj[3][kListCap];               /* j accumulator of the tile list */
-    float fi[3][32];                     /* i accumulator of the tile */
     int it[32];                          /* tile: type * ntypes */
     int idx[kListCap];                   /* tile list: particle */
     unsigned char list[kListCap];        /* the current group's list: tile-list entries */
@@ -378,24 +379,11 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         if (EXTRA && lane < kTileGroups)
             for (int d = 0; d < 3; ++d) s.eg[lane][d][0] = s.eg[lane][d][1] = 0.0f;
 
-        /* the i forces of the run that ends (FP32 sums never span two runs, so that a run's item gives
-         * what the whole item's share of it gives) */
-        auto flush_i = [&]() {
-            if (s.i0 + lane < s.i1 && (!FINE || (lane >> 2) == warp)) {
-                const float v0 = s.fi[0][lane], v1 = s.fi[1][lane], v2 = s.fi[2][lane];
-                if (v0 != 0.0f || v1 != 0.0f || v2 != 0.0f) flush_force<0>(F64, nullptr, n, s.i0 + lane, v0, v1, v2, err);
-                if (EXTRA && s.ci[lane]) atomicAdd(counts + s.i0 + lane, s.ci[lane]);
-            }
-            s.fi[0][lane] = s.fi[1][lane] = s.fi[2][lane] = 0.0f;
-            if (EXTRA) s.ci[lane] = 0;
-        };
         for (int ti = first_tile; ti < s.ntile; ti = s.ti + s.S) {
             {
                 const int ng = (s.ni + 3) >> 2, ga = ng * ti / s.ntile, gb = ng * (ti + 1) / s.ntile;
                 const int i0 = s.hs + 4 * ga, i1 = min(s.hs + s.ni, s.hs + 4 * gb);
                 s.it[lane] = i0 + lane < i1 ? __ldg(ptype + i0 + lane) * ntypes : 0;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) s.fi[d][lane] = 0.0f;
                 if (EXTRA) s.ci[lane] = 0;
                 __syncwarp();
                 s.ti = ti; s.i0 = i0; s.i1 = i1; s.ngr = gb - ga;
@@ -456,7 +444,6 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                             je = hi;
                             if (jb + lane < je) pn = __ldg(pos + jb + lane);
                             if (same) continue;
-                            if (!FINE) flush_i();
                             s.self = own;
                             /* the tile under this shift.  Exact rule: the box edge comes off the high
                              * side's coordinates (see pair_diff) */
@@ -656,7 +643,13 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                             }
                         }
                         reduce_scatter12(fi, lane);
-                        if ((lane & 1) == 0 && (lane & 7) < 6) s.fi[(lane & 7) >> 1][4 * gi + (lane >> 3)] += fi[0];
+                        {   /* to the global sums: lane 8 k + 2 c, component c of particle k */
+                            const int k = ig + (lane >> 3), c = (lane & 7) >> 1;
+                            if ((lane & 1) == 0 && c < 3 && k < s.i1 && fi[0] != 0.0f) {
+                                if (!(fabsf(fi[0]) < kFixMax) && err) atomicOr(err, kErrForce);
+                                atomicAdd(F64 + (size_t)c * n + k, to_fixed(fi[0]));
+                            }
+                        }
                         if (EXTRA) {
 #pragma unroll
                             for (int k = 0; k < 4; ++k) {
@@ -706,7 +699,8 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                 if (FINE) __syncthreads();
                 __syncwarp();
             }
-            flush_i();
+            if (EXTRA && s.i0 + lane < s.i1 && (!FINE || (lane >> 2) == warp) && s.ci[lane])
+                atomicAdd(counts + s.i0 + lane, s.ci[lane]);
             __syncwarp();
         }
 

@@ -1,0 +1,77 @@
+"""Partial sums of the list kernel: what is added in FP32, and what in exact integers or with compensation.
+
+Each case plants terms that cancel where the sums have to keep a small one beside them."""
+import numpy as np
+import pytest
+
+import sc2019_md_gb300 as m
+
+pytestmark = pytest.mark.gpu
+
+L, RC, EDGE = 62.5, 12.0, 12.5
+
+
+def _hilbert(pos, cell):
+    """Index along the 24-bit Hilbert curve of the in-cell order (Skilling's transform)."""
+    loc = (pos.astype(np.float64) - np.asarray(cell) * EDGE) * (256.0 / EDGE)
+    x = np.clip(loc.astype(int), 0, 255).T.copy()
+    bit = 128
+    while bit > 1:
+        low = bit - 1
+        for k in range(3):
+            hi = (x[k] & bit) != 0
+            t = np.where(hi, 0, (x[0] ^ x[k]) & low)
+            x[0] ^= np.where(hi, low, t)
+            x[k] ^= t
+        bit >>= 1
+    x[1] ^= x[0]
+    x[2] ^= x[1]
+    t = np.zeros_like(x[0])
+    bit = 128
+    while bit > 1:
+        t ^= np.where(x[2] & bit, bit - 1, 0)
+        bit >>= 1
+    x ^= t
+    h = np.zeros_like(x[0])
+    for b in range(7, -1, -1):
+        for k in range(3):
+            h = (h << 1) | ((x[k] >> b) & 1)
+    return h
+
+
+def _params(**kw):
+    return m.default_params(**{**dict(box=[L] * 3, cutoff=RC, ntypes=3, sigma=[1.0] * 3, epsilon=[0.0] * 3, mass=[1.0] * 3,
+                                      table_bins=256), **kw})
+
+
+def test_forces_of_different_lists_add_exactly():
+    """An atom with two neighbours whose y forces cancel exactly, 1e5 kcal/mol/A each, in different cells, and
+    between them in the cell order more than 512 atoms without forces, a weak neighbour, and 512 more: the
+    three are in different lists, and the weak one's force comes out as if the strong ones were not there."""
+    rng = np.random.default_rng(1)
+    i = np.array([24.5, 24.5, 13.0])
+    lo = np.array([2, 2, 0]) * EDGE
+    f = lo + rng.uniform(0.05, EDGE - 0.05, (6000, 3))
+    f = f[np.linalg.norm(f - i, axis=1) < RC - 0.5].astype(np.float32)
+    f = f[np.argsort(_hilbert(f, (2, 2, 0)), kind="stable")]
+    near = np.linalg.norm(f - i, axis=1) < 7.0
+    at = [k for k in np.flatnonzero(near) if 600 < k < len(f) - 600]
+    c = at[len(at) // 2]
+    pos = np.concatenate([[i, [25.5, 23.5, 13.0], [25.5, 25.5, 13.0]], f]).astype(np.float32)
+    t = np.ones(len(pos), np.int32)
+    t[:3] = 0
+    t[3 + c] = 2
+    coef = np.zeros((3, 3, 4))
+    coef[0, 0, 0] = 1.28e7                     # 2^-7 of it at r2 = 2: 1e5 per component
+    r2 = float(((f[c] - i) ** 2).sum())
+    coef[0, 2, 0] = coef[2, 0, 0] = 1.234567 * r2 ** 7
+    keep = np.arange(len(pos)) > 2
+    keep[0] = True
+    with m.Context(_params()) as ctx:
+        ctx.set_pair_coefficients(coef)
+        assert ctx.kernels()["eval"] == "list"
+        F, st = ctx.force_fixed(*(np.ascontiguousarray(pos[:, k]) for k in range(3)), type=t)
+        W, _ = ctx.force_fixed(*(np.ascontiguousarray(pos[keep, k]) for k in range(3)), type=t[keep])
+    assert abs(F[1, 1]) > 9e4 * 2 ** 24 and abs(F[2, 1]) > 9e4 * 2 ** 24
+    assert abs(W[0, 1]) > 0.1 * 2 ** 24
+    assert F[0, 1] == W[0, 1] and F[0, 2] == W[0, 2]
