@@ -79,13 +79,6 @@ __device__ __forceinline__ float3 bsub(float4 a, float4 b, const Geom &g) {
     return make_float3(bsub1(a.x, b.x, g.L[0], g.h[0]), bsub1(a.y, b.y, g.L[1], g.h[1]),
                        bsub1(a.z, b.z, g.L[2], g.h[2]));
 }
-/* s + e = a + b exactly (Knuth's two-sum) */
-__device__ __forceinline__ float two_sum(float a, float b, float &e) {
-    const float s = __fadd_rn(a, b);
-    const float bb = __fsub_rn(s, a);
-    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    return s;
-}
 /* r^2 of v as an unevaluated sum hi + lo (products split exactly with fma, the sum with two-sum):
  * about twice FP32's precision, so that r^2 - r0^2 of a bond near its rest length keeps its digits */
 __device__ __forceinline__ float norm2_hilo(float3 v, float &lo) {

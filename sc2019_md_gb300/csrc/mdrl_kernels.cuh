@@ -98,6 +98,14 @@ __device__ __forceinline__ float wrap_exact(float xi, float xj, float L, float h
     return d;
 }
 
+/* s + e = a + b exactly (Knuth's two-sum) */
+__device__ __forceinline__ float two_sum(float a, float b, float &e) {
+    const float s = __fadd_rn(a, b);
+    const float bb = __fsub_rn(s, a);
+    e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+
 template <bool SEP>
 __device__ __forceinline__ float madd(float a, float b, float c) {
     return SEP ? __fadd_rn(__fmul_rn(a, b), c) : __fmaf_rn(a, b, c);

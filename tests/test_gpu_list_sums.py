@@ -1,6 +1,8 @@
 """Partial sums of the list kernel: what is added in FP32, and what in exact integers or with compensation.
 
 Each case plants terms that cancel where the sums have to keep a small one beside them."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -75,3 +77,33 @@ def test_forces_of_different_lists_add_exactly():
     assert abs(F[1, 1]) > 9e4 * 2 ** 24 and abs(F[2, 1]) > 9e4 * 2 ** 24
     assert abs(W[0, 1]) > 0.1 * 2 ** 24
     assert F[0, 1] == W[0, 1] and F[0, 2] == W[0, 2]
+
+
+def _planted(types, at, order=1, a12=(), a14=()):
+    pos = np.array([[24.0, 18.0, 18.0]] + at, np.float32)
+    coef = np.zeros((4, 4, 4))
+    for k, (e, f) in enumerate(zip(a12, a14)):
+        coef[0, k + 1, 0] = coef[k + 1, 0, 0] = f
+        coef[0, k + 1, 2] = coef[k + 1, 0, 2] = e
+    with m.Context(_params(ntypes=4, sigma=[1.0] * 4, epsilon=[0.0] * 4, mass=[1.0] * 4, flags=m.FLAG_ENERGY,
+                           table_order=order)) as ctx:
+        ctx.set_pair_coefficients(coef)
+        assert ctx.kernels()["eval"] == "list"
+        return ctx.force(*(np.ascontiguousarray(pos[:, k]) for k in range(3)), type=np.array([0] + types, np.int32))[1]
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
+def test_energies_that_cancel_across_lanes(order):
+    """Two pair energies (and virials) of 6,400 and -6,400 and one of 8e-5 in one list, in every order: the small
+    one is what is left.  Lanes hold one pair each; the sums over lanes keep 2^-46 of the largest term:
+    1e-9 here."""
+    at = [[26.0, 19.0, 18.0], [26.0, 17.0, 18.0], [26.0, 18.0, 19.0]]
+    e, f = (1.0e8, -1.0e8, 1.2345), (1.0e8, -1.0e8, 1.2345)
+    want = _planted([3], at[2:], order, e, f)
+    assert want["e_lj"] > 5e-5
+    for types in itertools.permutations([1, 2, 3]):
+        got = _planted(list(types), at, order, e, f)
+        assert got["pairs"] == 6
+        assert abs(got["e_lj"] - want["e_lj"]) < 1e-9
+        assert abs(got["virial"] - want["virial"]) < 1e-9
+
