@@ -277,6 +277,11 @@ __device__ __forceinline__ float warp_sums(float a, float b, float c, int lane, 
     return hi;
 }
 
+/* hi + lo in FP64; an infinite or NaN hi by itself, whose lo is NaN. */
+__device__ __forceinline__ double hi_lo(const float (&v)[2]) {
+    return isfinite(v[0]) ? (double)v[0] + v[1] : (double)v[0];
+}
+
 /* BATCH: the items are those of a batch's replicas (replica geometry, cell offset and splits from
  * reps); with MODE kDiffWrap they are (cell a, split) of replicas whose edges all exceed 2 rc: a's
  * particles against every later particle of the replica. */
@@ -733,7 +738,7 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         if (EXTRA) {
             if (lane < (FINE ? kWarpsPerCta : kTileGroups)) {
                 const float (*eg)[2] = FINE ? all[lane].eg[lane] : s.eg[lane];
-                e1 = (double)eg[0][0] + eg[0][1]; e2 = (double)eg[1][0] + eg[1][1]; e3 = (double)eg[2][0] + eg[2][1];
+                e1 = hi_lo(eg[0]); e2 = hi_lo(eg[1]); e3 = hi_lo(eg[2]);
             }
 #pragma unroll
             for (int o = kTileGroups / 2; o > 0; o >>= 1) {

@@ -107,3 +107,10 @@ def test_energies_that_cancel_across_lanes(order):
         assert abs(got["e_lj"] - want["e_lj"]) < 1e-9
         assert abs(got["virial"] - want["virial"]) < 1e-9
 
+
+def test_infinite_energies_stay_infinite():
+    """A pair energy that overflows FP32 while its force is finite: the total is infinite, not NaN."""
+    st = _planted([1], [[24.5, 18.0, 18.0]], 1, (3.0e38,), (1.0,))
+    assert st["e_lj"] == np.inf and np.isfinite(st["virial"])
+    st = _planted([1, 2], [[24.5, 18.0, 18.0], [26.0, 17.0, 18.0]], 1, (-3.0e38, 1.0), (1.0, 1.0))
+    assert st["e_lj"] == -np.inf and np.isfinite(st["virial"])
