@@ -361,7 +361,7 @@ static void free_particles(mdrl_ctx *c) {
     dfree(&c->d_ovx); dfree(&c->d_ovy); dfree(&c->d_ovz); dfree(&c->d_ocnt);
     for (int b = 0; b < 2; ++b) { dfree(&c->d_pos[b]); dfree(&c->d_vel[b]); dfree(&c->d_type[b]); dfree(&c->d_id[b]); }
     dfree(&c->d_cell_of); dfree(&c->d_slot); dfree(&c->d_tmp); dfree(&c->d_sorted); dfree(&c->d_key);
-    dfree(&c->d_sortkey);
+    dfree(&c->d_sortkey); dfree(&c->d_tile[0]); dfree(&c->d_tile[1]);
     dfree(&c->d_F64); dfree(&c->d_F32); dfree(&c->d_cnt);
     dfree(&c->d_Fscr64); dfree(&c->d_Fscr32);
     c->cap = 0;
@@ -385,7 +385,7 @@ extern "C" mdrl_status mdrl_destroy(mdrl_ctx *c) {
     free_particles(c);
     dfree(&c->d_f2); dfree(&c->d_e2); dfree(&c->d_f4); dfree(&c->d_e4); dfree(&c->d_fr); dfree(&c->d_wa); dfree(&c->d_wb); dfree(&c->d_wc); dfree(&c->d_w1);
     dfree(&c->d_pcoef);
-    dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work); dfree(&c->d_narrow);
+    dfree(&c->d_count); dfree(&c->d_start); dfree(&c->d_unit); dfree(&c->d_kepart); dfree(&c->d_work); dfree(&c->d_tstart); dfree(&c->d_narrow);
     dfree(&c->d_tot); dfree(&c->d_totscr); dfree(&c->d_err); dfree(&c->d_mt);
     if (c->h_tot) cudaFreeHost(c->h_tot);
     if (c->h_err) cudaFreeHost(c->h_err);
@@ -422,14 +422,16 @@ static mdrl_status ensure_cells(mdrl_ctx *c) {
     c->ncells = c->g.nc[0] * c->g.nc[1] * c->g.nc[2];
     MDRL_TRY(dalloc(&c->d_count, c->ncells));
     MDRL_TRY(dalloc(&c->d_start, c->ncells + 1));
-    MDRL_TRY(dalloc(&c->d_work, 2));
+    MDRL_TRY(dalloc(&c->d_work, 4));
+    MDRL_TRY(dalloc(&c->d_tstart, (size_t)c->ncells + 1));
     return MDRL_OK;
 }
 
 mdrl_status mdrl::ensure_capacity(mdrl_ctx *c, int n) {
     MDRL_TRY(ensure_cells(c));
     /* result slots of any kernel and tile (a batch sizes its own) */
-    const size_t slots = (size_t)c->ncells * std::max(kHalfShellCells * kMaxItemGroups, list_cell_slots(std::max(n, c->cap), c->ncells));
+    const size_t slots = std::max((size_t)c->ncells * kHalfShellCells * kMaxItemGroups,
+                                  (size_t)items_max(std::max(n, c->cap), c->ncells, fine_items(tile_groups(c->ncells), 0, 1)));
     if (!c->batch && slots > c->unit_cap) {
         MDRL_TRY(dalloc(&c->d_unit, slots));
         c->unit_cap = slots;
@@ -450,6 +452,8 @@ mdrl_status mdrl::ensure_capacity(mdrl_ctx *c, int n) {
     MDRL_TRY(dalloc(&c->d_cell_of, m)); MDRL_TRY(dalloc(&c->d_slot, m));
     MDRL_TRY(dalloc(&c->d_tmp, m)); MDRL_TRY(dalloc(&c->d_sorted, m)); MDRL_TRY(dalloc(&c->d_key, m));
     MDRL_TRY(dalloc(&c->d_sortkey, m));
+    if (c->p.accum == MDRL_ACC_FIXED64)
+        for (int2 *&t : c->d_tile) MDRL_TRY(dalloc(&t, (size_t)tiles_max(n, c->ncells, 4)));
     if (c->p.accum == MDRL_ACC_FIXED64) { MDRL_TRY(dalloc(&c->d_F64, 3 * m)); }
     else { MDRL_TRY(dalloc(&c->d_F32, 6 * m)); }   /* high and low planes */
     MDRL_TRY(dalloc(&c->d_cnt, m));
@@ -497,17 +501,17 @@ bool mdrl::list_eval(const mdrl_ctx *c) {
     return c->p.accum == MDRL_ACC_FIXED64 && (!c->tile_asked || c->tile.warps_per_cta == 1);
 }
 
-mdrl_status mdrl::list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid) {
+mdrl_status mdrl::list_grid(list_fn fn, size_t smem, long long items, bool fine, int num_sms, int *grid) {
     int per_sm = 0;
     MDRL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32 * kWarpsPerCta, smem));
-    *grid = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta,
-                     std::max(1, per_sm) * std::max(1, num_sms));
+    *grid = (int)std::min<long long>(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta,
+                                     std::max(1, per_sm) * std::max(1, num_sms));
     return MDRL_OK;
 }
 
-void mdrl::launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy) {
-    k_totals<<<tot_blocks(nunits, nke), kTotThreads, 0, c->stream>>>(nunits, c->d_unit, nke, c->d_kepart, c->d_tot,
-                                                                    energy ? 1 : 0, c->d_totscr);
+void mdrl::launch_totals(mdrl_ctx *c, const TotUnits &units, long long upto, int nke, bool energy) {
+    k_totals<<<tot_blocks((int)upto, nke), kTotThreads, 0, c->stream>>>(units, c->d_unit, nke, c->d_kepart, c->d_tot,
+                                                                       energy ? 1 : 0, c->d_totscr);
 }
 
 /* The smem attribute is set once per kernel and device, on the first (uncaptured) launch. */
@@ -526,28 +530,34 @@ mdrl_status mdrl::prepare_force_kernel(force_fn fn, int device) {
 
 int mdrl::eff_order(const mdrl_ctx *c) { return c->p.eval == MDRL_EVAL_DIRECT ? 0 : c->order; }
 
-/* The list kernel's launch over the units of home cells [cell0, cell0 + cells); *slots: its result
- * slots, one per item. */
+/* The list kernel's launch over the units of home cells [cell0, cell0 + cells), whose tiles the binning
+ * has written; *upto: the most result slots it can fill (their number is left in d_work[2]). */
 static mdrl_status launch_list(mdrl_ctx *c, int n, const float4 *pos, const int *type, bool extra, int cell0, int cells,
-                               int *slots) {
-    const int G = c->tile_asked ? c->tile.steps_per_piece : 1;
-    bool fine;
-    int items = 0, grid = 0;
-    const int cfg = list_cfg(n, c->ncells, cells, G, c->num_sms, &fine, &items);
+                               long long *upto) {
+    int grid = 0;
+    const int tg = tile_groups(c->ncells);
+    const bool fine = fine_items(tg, items_expected(n, c->ncells, cells), c->num_sms);
+    const long long items = items_max(n, c->ncells, fine);
     const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
     list_fn fn = (c->p.flags & MDRL_FLAG_EXACT_DIFF) ? pick_force_list<kDiffExact, false>(eff_order(c), false, extra, coul, fine)
                                                      : pick_force_list<kDiffShift, false>(eff_order(c), sep, extra, coul, fine);
     MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
     const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
     MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
+    ListTiles lt;
+    lt.first = c->d_tstart + cell0;
+    lt.last = lt.first + cells;
+    lt.tile[0] = c->d_tile[0];
+    lt.tile[1] = c->d_tile[1];
+    lt.groups = tg;
     MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
-    if (items > 0)    /* k_scan has zeroed the item counter */
-        fn<<<grid, 32 * kWarpsPerCta, smem, c->stream>>>(
-            pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n, c->d_F64, c->d_cnt, c->d_unit,
-            ListBatch{}, nullptr, cfg, c->d_err, cell0, c->d_work, items, extra ? nullptr : c->d_tot);
+    /* the binning has zeroed the item counter; without particles one CTA finds no tiles */
+    fn<<<std::max(1, grid), 32 * kWarpsPerCta, smem, c->stream>>>(
+        pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, n, c->d_F64, c->d_cnt, c->d_unit, lt,
+        nullptr, c->d_err, c->d_work, c->d_work + 2, extra ? nullptr : c->d_tot);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaEventRecord(c->evf1, c->stream));
-    *slots = items;
+    *upto = items;
     return MDRL_OK;
 }
 
@@ -677,12 +687,19 @@ static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, 
                             const float *q, const int *type, int buf, bool spatial, bool stage = false,
                             bool inv = false, bool hilbert = false) {
     c->have_state = false;
+    Tiles tl;
+    if (hilbert) {      /* the order of the list kernel */
+        tl.groups = tile_groups(c->ncells);
+        tl.start = c->d_tstart;
+        tl.tile[0] = c->d_tile[0];
+        tl.tile[1] = c->d_tile[1];
+    }
     if (spatial && small_system(c, n)) {
         MDRL_TRY(prepare_force_kernel((force_fn)k_small_user, c->p.device));
         k_small_user<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
             n, x, y, z, q, type, c->g, c->ncells, hilbert ? 1 : 0, c->d_pos[buf], c->d_type[buf], c->d_id[buf],
             inv ? c->d_inv : nullptr, c->d_F64, c->d_F32, c->d_cnt, c->p.ntypes, c->d_start, c->d_tot, c->d_work,
-            c->d_err);
+            c->d_err, tl);
         MDRL_CUDA(cudaGetLastError());
         return MDRL_OK;
     }
@@ -699,11 +716,11 @@ static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, 
             if (type) type = c->d_ut;
         }
     }
-    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work, spatial);
+    k_scan<<<1, 1024, 0, c->stream>>>(c->ncells, c->d_count, c->d_start, c->d_tot, c->d_work, spatial, tl);
     if (n > 0) {
         k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
         k_cell_sort<<<c->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted,
-                                                       spatial ? c->d_key : nullptr, c->d_sortkey, c->d_err);
+                                                       spatial ? c->d_key : nullptr, c->d_sortkey, c->d_err, tl);
         k_gather_user<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_sorted, x, y, z, q, type, c->d_pos[buf],
                                                            c->d_type[buf], c->d_id[buf], c->d_F64,
                                                            c->d_F32, c->d_cnt, c->p.ntypes, c->d_err,
@@ -790,15 +807,17 @@ static mdrl_status force_eval_enqueue(mdrl_ctx *c, int n, const float *x, const 
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
     const bool list = list_eval(c);
-    int slots = force_slots(c, force_items(c->ncells));
+    TotUnits units{force_slots(c, force_items(c->ncells))};
+    long long upto = units.n;
     MDRL_TRY(bin_user(c, n, x, y, z, q, type, 0, true, stage, true, list));
     const bool energy = (c->p.flags & MDRL_FLAG_ENERGY) != 0;
     MDRL_TRY(pme_begin(c, n, c->d_pos[0], energy));
-    if (list) MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], extra, 0, c->ncells, &slots));
+    if (list) units = TotUnits{0, c->d_work + 2};
+    if (list) MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], extra, 0, c->ncells, &upto));
     else MDRL_TRY(launch_force(c, n, c->d_pos[0], c->d_type[0], extra, extra ? nullptr : c->d_tot));
     MDRL_TRY(pme_finish(c, n, c->d_pos[0], c->d_F64, c->d_F32));
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, energy));
-    if (extra) launch_totals(c, slots, 0, true);
+    if (extra) launch_totals(c, units, upto, 0, true);
     if (energy) MDRL_TRY(pme_add_energy(c, n));
     if (energy) MDRL_TRY(bonded_add_energy(c, n));
     if (out) populate(out->ptr, out->count, 4 * (size_t)n);
@@ -1020,9 +1039,9 @@ extern "C" mdrl_status mdrl_force_eval_fixed(mdrl_ctx *c, int n, const float *x,
     MDRL_TRY(bin_user(c, n, (const float *)dx, (const float *)dy, (const float *)dz, (const float *)dq,
                       (const int *)dt, 0, true, direct, true, list_eval(c)));
     const int layer = c->g.nc[1] * c->g.nc[2], cells = (hx1 - hx0) * layer;
-    int slots = force_slots(c, cells * kHalfShellCells);
+    long long upto = 0;
     if (list_eval(c))
-        MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], false, hx0 * layer, cells, &slots));
+        MDRL_TRY(launch_list(c, n, c->d_pos[0], c->d_type[0], false, hx0 * layer, cells, &upto));
     else
         MDRL_TRY(launch_force_into(c, n, c->d_pos[0], c->d_type[0], false, c->d_F64, nullptr, c->d_tot,
                                    hx0 * layer * kHalfShellCells, cells * kHalfShellCells));
@@ -1264,7 +1283,8 @@ extern "C" mdrl_status mdrl_set_state(mdrl_ctx *c, int n, const float *x, const 
     MDRL_TRY(bonded_enqueue(c, n, c->d_pos[0], c->d_id[0], c->d_F64, c->d_F32, extra));
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, c->d_F32, c->d_mt, 0,
                                                 c->d_kepart);
-    launch_totals(c, force_slots(c, force_items(c->ncells)), nblk(n, 256), extra);
+    const int slots = force_slots(c, force_items(c->ncells));
+    launch_totals(c, TotUnits{slots}, slots, nblk(n, 256), extra);
     if (extra) MDRL_TRY(pme_add_energy(c, n));
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());
@@ -1311,7 +1331,8 @@ static mdrl_status enqueue_step(mdrl_ctx *c, bool extra) {
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[b], c->d_type[b], c->d_F64, c->d_F32, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    if (extra) launch_totals(c, force_slots(c, force_items(c->ncells)), nblk(n, 256), true);
+    const int slots = force_slots(c, force_items(c->ncells));
+    if (extra) launch_totals(c, TotUnits{slots}, slots, nblk(n, 256), true);
     if (extra) MDRL_TRY(pme_add_energy(c, n));
     if (extra) MDRL_TRY(bonded_add_energy(c, n));
     MDRL_CUDA(cudaGetLastError());

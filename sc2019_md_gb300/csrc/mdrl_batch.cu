@@ -99,9 +99,10 @@ __global__ void k_bkick_drift_bin(int n, float4 *__restrict__ pos, float4 *__res
  * half-shell [1] replicas. */
 struct ListSlots {
     int on;
-    ListBatch list[2];
-    const int *rep_pos;
-    int first[2], per_item[2];
+    const int2 *start;               /* first tiles by place */
+    const int *rep_place;            /* a replica's first place */
+    int place[3];                    /* list k: places [place[k], place[k + 1]) */
+    int first[2], fine[2];           /* its first slot; whether its items are fine ones */
 };
 
 /* Per-replica totals of the last force evaluation (its items, in item order) and, when vel is
@@ -122,29 +123,30 @@ __global__ void __launch_bounds__(128) k_rep_totals(const int *__restrict__ item
     __shared__ unsigned long long s_u[128][2];
     const int r = blockIdx.x, t = threadIdx.x;
     double a = 0, b = 0, c = 0, k = 0;
-    unsigned long long p = 0, q = 0;
+    unsigned long long p = 0, q2 = 0;
     for (int e = item_begin[r] + t; e < item_begin[r + 1]; e += 128) {
         const UnitOut u = uout[rep_items[e]];
         a += u.e_lj; b += u.e_coul; c += u.virial;
-        p += u.pairs; q += u.below;
+        p += u.pairs; q2 += u.below;
     }
     if (item_begin2)
         for (int e = G * item_begin2[r] + t; e < G * item_begin2[r + 1]; e += 128) {
             const UnitOut u = uout[slot0 + G * rep_items2[e / G] + e % G];
             a += u.e_lj; b += u.e_coul; c += u.virial;
-            p += u.pairs; q += u.below;
+            p += u.pairs; q2 += u.below;
         }
     if (ls.on && reps[r].path != kPathAllImages) {
-        const int k = reps[r].path == kPathHalfShell;
-        const ListBatch &l = ls.list[k];
-        const int at = ls.rep_pos[r], m = ls.per_item[k];
-        for (int cls = 0; cls < (k ? kClasses : 1); ++cls) {
-            const int *pre = cls == 2 ? l.pre1 : l.pre0;
-            const int base = ls.first[k] + m * (cls * l.total0);
-            for (int e = m * pre[at] + t; e < m * pre[at + 1]; e += 128) {
+        const int k = reps[r].path == kPathHalfShell, p0 = ls.rep_place[r];
+        const int2 lo = ls.start[ls.place[k]], hi = ls.start[ls.place[k + 1]];
+        const int2 at = ls.start[p0], to = ls.start[p0 + reps[r].g.nc[0] * reps[r].g.nc[1] * reps[r].g.nc[2]];
+        const int nt = hi.x - lo.x, runs = k == 0 ? 1 : (ls.fine[k] ? kFineRuns : kClasses);
+        for (int q = 0; q < runs; ++q) {
+            const bool last = k == 1 && !ls.fine[k] && q == 2;      /* class 2: tiles of the second kind */
+            const int base = ls.first[k] + q * nt - (last ? lo.y : lo.x);
+            for (int e = (last ? at.y : at.x) + t; e < (last ? to.y : to.x); e += 128) {
                 const UnitOut u = uout[base + e];
                 a += u.e_lj; b += u.e_coul; c += u.virial;
-                p += u.pairs; q += u.below;
+                p += u.pairs; q2 += u.below;
             }
         }
     }
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(128) k_rep_totals(const int *__restrict__ item
         }
     }
     s_d[t][0] = a; s_d[t][1] = b; s_d[t][2] = c; s_d[t][3] = k;
-    s_u[t][0] = p; s_u[t][1] = q;
+    s_u[t][0] = p; s_u[t][1] = q2;
     __syncthreads();
     for (int off = 64; off > 0; off >>= 1) {
         if (t < off) {
@@ -192,16 +194,14 @@ struct mdrl_batch {
     int n_hs = 0, n_cp = 0, n_ot = 0;
     BatchItem *d_items_hs = nullptr, *d_items_ot = nullptr;
     int *d_begin_hs = nullptr, *d_list_hs = nullptr, *d_begin_ot = nullptr, *d_list_ot = nullptr;
-    /* the list kernel's items (force evaluations): [0] the min-image replicas, [1] the half-shell ones,
-     * each by falling mean occupancy; rep_pos[r]: a replica's place in its list */
-    struct ListReps {
-        ListBatch dev{nullptr, nullptr, nullptr, 0, 0};
-        int *d_rep = nullptr, *d_pre0 = nullptr, *d_pre1 = nullptr;
-        int items = 0, tile_groups = 0;
-    } lists[2];
-    int *d_rep_pos = nullptr;
-    bool list_slots = false; /* the result slots are those of a list launch: */
-    int list_first[2] = {0, 0}, list_per_item[2] = {1, 1};   /* its first slots and slots per item */
+    /* the list kernel's tiles (force evaluations) are numbered by place: the cells of the min-image replicas
+     * (list 0), then those of the half-shell ones (list 1), each list's replicas by falling mean
+     * occupancy; rep_place[r]: a replica's first place */
+    int place[3] = {0, 0, 0};
+    long long list_upto[2] = {0, 0};    /* the most items of each list's launch */
+    bool list_fine[2] = {false, false};
+    int *d_cell_at = nullptr, *d_place_of = nullptr, *d_cell_groups = nullptr, *d_rep_of_cell = nullptr, *d_rep_place = nullptr;
+    bool list_slots = false; /* the result slots are those of a list launch */
     /* an evaluation's list launches run beside its all-image launch, on a stream of their own */
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -262,8 +262,8 @@ extern "C" mdrl_status mdrl_batch_destroy(mdrl_batch *b) {
     dfree(&b->d_reps); dfree(&b->d_items); dfree(&b->d_rep_of); dfree(&b->d_item_begin);
     dfree(&b->d_rep_items); dfree(&b->d_reptot);
     dfree(&b->d_items_hs); dfree(&b->d_items_ot); dfree(&b->d_begin_hs); dfree(&b->d_list_hs);
-    dfree(&b->d_begin_ot); dfree(&b->d_list_ot); dfree(&b->d_rep_pos);
-    for (auto &l : b->lists) { dfree(&l.d_rep); dfree(&l.d_pre0); dfree(&l.d_pre1); }
+    dfree(&b->d_begin_ot); dfree(&b->d_list_ot);
+    dfree(&b->d_cell_at); dfree(&b->d_place_of); dfree(&b->d_cell_groups); dfree(&b->d_rep_of_cell); dfree(&b->d_rep_place);
     if (b->c) mdrl_destroy(b->c);
     delete b;
     return MDRL_OK;
@@ -293,10 +293,8 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
         hrep[r].p_off = (int)ntot;
         hrep[r].cell_off = (int)ncells;
         ntot += reps[r].n;
-        const int ncr = hrep[r].g.nc[0] * hrep[r].g.nc[1] * hrep[r].g.nc[2], tg = tile_groups(ncr);
-        hrep[r].tile_groups = tg;
-        hrep[r].split0 = list_split(reps[r].n, ncr, tg & 0xff);
-        hrep[r].split1 = list_split(reps[r].n, ncr, tg >> 8);
+        const int ncr = hrep[r].g.nc[0] * hrep[r].g.nc[1] * hrep[r].g.nc[2];
+        hrep[r].tile_groups = tile_groups(ncr);
         ncells += ncr;
         if (ntot > (1LL << 28) || ncells > (1LL << 24)) {
             set_error("mdrl_batch_create: too many particles or cells in the batch");
@@ -381,7 +379,10 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     std::vector<int> begin_hs, list_hs, begin_ot, list_ot;
     rep_lists(items_hs, begin_hs, list_hs);
     rep_lists(items_ot, begin_ot, list_ot);
-    std::vector<int> lrep[2], lpre0[2], lpre1[2], rep_pos(nrep, 0);
+    std::vector<int> cell_at, place_of((size_t)ncells, -1), cell_groups((size_t)ncells, 0), rep_of_cell((size_t)ncells, 0),
+        rep_place(nrep, 0);
+    int list_groups[2] = {0, 0};
+    long long list_expected[2] = {0, 0}, list_most[2][2] = {{0, 0}, {0, 0}};    /* [list][fine] */
     {
         std::vector<int> by_load(nrep);
         std::iota(by_load.begin(), by_load.end(), 0);
@@ -390,25 +391,30 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
             return (long long)hrep[a].n * cells(b) > (long long)hrep[b].n * cells(a);
         });
         for (int k = 0; k < 2; ++k) {
-            long long t0 = 0, t1 = 0;
             int tg0 = 0, tg1 = 0;
             for (int r : by_load) {
                 if (hrep[r].path != (k ? kPathHalfShell : kPathMinImage)) continue;
-                rep_pos[r] = (int)lrep[k].size();
-                lrep[k].push_back(r); lpre0[k].push_back((int)t0); lpre1[k].push_back((int)t1);
-                t0 += (long long)cells(r) * hrep[r].split0;
-                t1 += (long long)cells(r) * hrep[r].split1;
-                tg0 = std::max(tg0, hrep[r].tile_groups & 0xff);
-                tg1 = std::max(tg1, hrep[r].tile_groups >> 8);
-                if (2 * t0 + t1 > 2147483647LL / kMaxItemGroups) {
+                const int ncr = cells(r), tg = hrep[r].tile_groups;
+                rep_place[r] = (int)cell_at.size();
+                for (int c = hrep[r].cell_off; c < hrep[r].cell_off + ncr; ++c) {
+                    place_of[c] = (int)cell_at.size();
+                    cell_groups[c] = tg;
+                    rep_of_cell[c] = r;
+                    cell_at.push_back(c);
+                }
+                tg0 = std::max(tg0, tg & 0xff);
+                tg1 = std::max(tg1, tg >> 8);
+                const long long tiles = tiles_max(hrep[r].n, ncr, tg & 0xff);
+                list_expected[k] += k ? items_expected(hrep[r].n, ncr, ncr) : tiles;
+                for (int fine = 0; fine < 2; ++fine) list_most[k][fine] += k ? items_max(hrep[r].n, ncr, fine) : tiles;
+                if (list_most[k][0] > 2147483647LL / kMaxItemGroups) {
                     delete bt;
                     set_error("mdrl_batch_create: work list too long");
                     return MDRL_ERR_RANGE;
                 }
             }
-            lpre0[k].push_back((int)t0); lpre1[k].push_back((int)t1);
-            bt->lists[k].items = (int)(k ? 2 * t0 + t1 : t0);
-            bt->lists[k].tile_groups = tg0 | (tg1 << 8);
+            bt->place[k + 1] = (int)cell_at.size();
+            list_groups[k] = tg0 | (tg1 << 8);
         }
     }
     /* the context carries the force field; its own box is the first replica's (never used) */
@@ -428,25 +434,26 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
         set_error(std::string("mdrl_batch_create: ") + cudaGetErrorString(se));
         return fail(MDRL_ERR_CUDA);
     }
-    if ((s = dalloc(&c->d_work, 2)) != MDRL_OK) return fail(s);
+    for (int k = 0; k < 2; ++k) {
+        bt->list_fine[k] = list_most[k][0] > 0 && fine_items(list_groups[k], list_expected[k], c->num_sms);
+        bt->list_upto[k] = list_most[k][bt->list_fine[k]];
+    }
+    if ((s = dalloc(&c->d_work, 4)) != MDRL_OK) return fail(s);
+    if ((s = dalloc(&c->d_tstart, cell_at.size() + 1)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_count, (size_t)bt->ncells)) != MDRL_OK) return fail(s);
     if ((s = dalloc(&c->d_start, (size_t)bt->ncells + 1)) != MDRL_OK) return fail(s);
-    /* result slots of any kernel and tile (fine items run below kFineItems per SM, kRuns slots each) */
-    const size_t list_slots = ((size_t)bt->lists[0].items + bt->lists[1].items) * kMaxItemGroups +
-                              (size_t)2 * kFineItems * c->num_sms * kRuns;
+    /* result slots of any kernel and tile */
+    const size_t list_slots = (size_t)(bt->list_upto[0] + bt->list_upto[1]);
     if ((s = dalloc(&c->d_unit, std::max((size_t)bt->nitems,
                                          (size_t)bt->n_ot + std::max(((size_t)bt->n_cp + bt->n_hs) * kMaxItemGroups,
                                                                      list_slots)))) != MDRL_OK)
         return fail(s);
-    for (int k = 0; k < 2; ++k) {
-        auto &l = bt->lists[k];
-        lrep[k].push_back(0);    /* never empty */
-        if ((s = dalloc(&l.d_rep, lrep[k].size())) != MDRL_OK) return fail(s);
-        if ((s = dalloc(&l.d_pre0, lpre0[k].size())) != MDRL_OK) return fail(s);
-        if ((s = dalloc(&l.d_pre1, lpre1[k].size())) != MDRL_OK) return fail(s);
-        l.dev = ListBatch{l.d_rep, l.d_pre0, l.d_pre1, (int)lrep[k].size() - 1, std::max(1, lpre0[k].back())};
-    }
-    if ((s = dalloc(&bt->d_rep_pos, (size_t)nrep)) != MDRL_OK) return fail(s);
+    cell_at.push_back(0);    /* never empty */
+    struct { int **dev; const std::vector<int> *host; } const per_cell[] = {
+        {&bt->d_cell_at, &cell_at}, {&bt->d_place_of, &place_of}, {&bt->d_cell_groups, &cell_groups},
+        {&bt->d_rep_of_cell, &rep_of_cell}, {&bt->d_rep_place, &rep_place}};
+    for (auto &v : per_cell)
+        if ((s = dalloc(v.dev, v.host->size())) != MDRL_OK) return fail(s);
     if ((s = ensure_capacity(c, bt->ntot)) != MDRL_OK) return fail(s);
     std::vector<int> rep_of(bt->ntot);
     for (int r = 0; r < nrep; ++r)
@@ -464,13 +471,8 @@ extern "C" mdrl_status mdrl_batch_create(const mdrl_params *p, int nrep, const m
     if ((s = dalloc(&bt->d_list_hs, std::max<size_t>(1, list_hs.size()))) != MDRL_OK) return fail(s);
     if ((s = dalloc(&bt->d_list_ot, std::max<size_t>(1, list_ot.size()))) != MDRL_OK) return fail(s);
     cudaError_t e = cudaMemcpy(bt->d_reps, bt->reps.data(), sizeof(BatchRep) * nrep, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(bt->d_rep_pos, rep_pos.data(), sizeof(int) * nrep, cudaMemcpyHostToDevice);
-    for (int k = 0; k < 2; ++k) {
-        auto &l = bt->lists[k];
-        if (e == cudaSuccess) e = cudaMemcpy(l.d_rep, lrep[k].data(), sizeof(int) * lrep[k].size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(l.d_pre0, lpre0[k].data(), sizeof(int) * lpre0[k].size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(l.d_pre1, lpre1[k].data(), sizeof(int) * lpre1[k].size(), cudaMemcpyHostToDevice);
-    }
+    for (auto &v : per_cell)
+        if (e == cudaSuccess) e = cudaMemcpy(*v.dev, v.host->data(), sizeof(int) * v.host->size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_items, bt->items.data(), sizeof(BatchItem) * bt->nitems, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_rep_of, rep_of.data(), sizeof(int) * bt->ntot, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(bt->d_item_begin, bt->item_begin.data(), sizeof(int) * (nrep + 1), cudaMemcpyHostToDevice);
@@ -542,55 +544,57 @@ static mdrl_status batch_launch_force(mdrl_batch *b, const float4 *pos, const in
     return MDRL_OK;
 }
 
-/* The list kernel's items of list k (0 min-image, 1 half-shell) and whether they are fine ones. */
-static int list_items(const mdrl_batch *b, int k, bool *fine) {
-    const int items = b->lists[k].items * (b->c->tile_asked ? b->c->tile.steps_per_piece : 1);
-    *fine = fine_items(b->lists[k].tile_groups, items, b->c->num_sms);
-    return *fine ? items * kRuns : items;
-}
-
-/* The list kernel over the min-image and the half-shell replicas on stream st; *slots: the result slots
- * so far. */
-static mdrl_status launch_lists(mdrl_batch *b, cudaStream_t st, const float4 *pos, const int *type, bool extra,
-                                int *slots) {
+/* The list kernel over the min-image and the half-shell replicas on stream st; their result slots follow
+ * the n_ot of the all-image launch. */
+static mdrl_status launch_lists(mdrl_batch *b, cudaStream_t st, const float4 *pos, const int *type, bool extra) {
     mdrl_ctx *c = b->c;
     const bool sep = c->p.arith == MDRL_ARITH_SEPARATE, coul = c->ke != 0.0f;
-    const int G = c->tile_asked ? c->tile.steps_per_piece : 1;
     const size_t smem = force_list_smem_bytes(c->p.ntypes, extra);
-    DevTotals *tot = extra ? nullptr : c->d_tot;
     for (int k = 0; k < 2; ++k) {
-        bool fine;
+        const bool fine = b->list_fine[k];
         int grid = 0;
-        const int items = list_items(b, k, &fine);
-        b->list_first[k] = *slots;
-        b->list_per_item[k] = G * (fine ? kRuns : 1);
-        if (items == 0) continue;
+        if (b->list_upto[k] == 0) continue;
         list_fn fn = k ? pick_force_list<kDiffShift, true>(eff_order(c), sep, extra, coul, fine)
                        : pick_force_list<kDiffWrap, true>(eff_order(c), sep, extra, coul, fine);
         MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
-        MDRL_TRY(list_grid(fn, smem, items, fine, c->num_sms, &grid));
+        MDRL_TRY(list_grid(fn, smem, b->list_upto[k], fine, c->num_sms, &grid));
+        ListTiles lt;
+        lt.first = c->d_tstart + b->place[k];
+        lt.last = c->d_tstart + b->place[k + 1];
+        lt.tile[0] = c->d_tile[0];
+        lt.tile[1] = c->d_tile[1];
+        lt.rep_of_cell = b->d_rep_of_cell;
         fn<<<grid, 32 * kWarpsPerCta, smem, st>>>(
             pos, type, c->d_start, c->g, table_dev(c), c->d_pcoef, c->p.ntypes, c->ke, b->ntot, c->d_F64, c->d_cnt,
-            c->d_unit + *slots, b->lists[k].dev, b->d_reps, G, c->d_err, 0, c->d_work + k, items, tot);
-        *slots += items;
+            c->d_unit + b->n_ot + (k ? b->list_upto[0] : 0), lt, b->d_reps, c->d_err, c->d_work + k, c->d_work + 2 + k,
+            extra ? nullptr : c->d_tot);
     }
     MDRL_CUDA(cudaGetLastError());
     return MDRL_OK;
 }
 
+/* Their result slots, and the most of them. */
+static TotUnits list_units(const mdrl_batch *b, long long *upto) {
+    TotUnits u{b->n_ot};
+    if (b->list_upto[0]) u.count = b->c->d_work + 2;
+    if (b->list_upto[1]) u.count2 = b->c->d_work + 3;
+    u.second = b->n_ot + (int)b->list_upto[0];
+    *upto = b->n_ot + b->list_upto[0] + b->list_upto[1];
+    return u;
+}
+
 /* A force evaluation's launches (list_eval): the all-image replicas in the CTA kernel and, beside it on
- * the side stream, the list kernel; *slots: their result slots, in that order.  The launches write
+ * the side stream, the list kernel.  The launches write
  * different replicas' particles and slots; the counts they share are atomic sums of integers.  The
  * all-image launch is a few long CTAs (15 replicas of 500 to 4,000 atoms: 309 us on a fraction of the
  * SMs, with the lists' 93 + 82 us after it); it is first in its stream, so its CTAs are placed before the
  * lists' persistent grids take the rest. */
-static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int *type, bool extra, int *slots) {
+static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int *type, bool extra) {
     mdrl_ctx *c = b->c;
     force_fn fo = pick_force_batch(eff_order(c), c->p.arith == MDRL_ARITH_SEPARATE, extra, false);
     MDRL_TRY(prepare_force_kernel(fo, c->p.device));
     MDRL_CUDA(cudaEventRecord(c->evf0, c->stream));
-    *slots = b->n_ot;
-    const bool both = b->n_ot && (b->lists[0].items || b->lists[1].items);
+    const bool both = b->n_ot && (b->list_upto[0] || b->list_upto[1]);
     if (both) MDRL_CUDA(cudaEventRecord(b->fork, c->stream));
     if (b->n_ot)
         fo<<<b->n_ot, kBatchFT, force_smem_bytes(c->p.ntypes, extra, kBatchFT / 32), c->stream>>>(
@@ -598,10 +602,10 @@ static mdrl_status batch_launch_list(mdrl_batch *b, const float4 *pos, const int
             c->d_cnt, c->d_unit, b->d_items_ot, b->d_reps, tile_word(kStepsPerPiece, 0), c->d_err, 0,
             extra ? nullptr : c->d_tot);
     if (!both) {
-        MDRL_TRY(launch_lists(b, c->stream, pos, type, extra, slots));
+        MDRL_TRY(launch_lists(b, c->stream, pos, type, extra));
     } else {
         MDRL_CUDA(cudaStreamWaitEvent(b->side, b->fork, 0));
-        const mdrl_status s = launch_lists(b, b->side, pos, type, extra, slots);
+        const mdrl_status s = launch_lists(b, b->side, pos, type, extra);
         cudaError_t e = cudaEventRecord(b->join, b->side);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, b->join, 0);
         if (e != cudaSuccess) cudaStreamSynchronize(b->side);    /* nothing of this call runs into the next */
@@ -622,10 +626,19 @@ static mdrl_status batch_bin_user(mdrl_batch *b, const float *q, const int *type
     MDRL_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
     k_bbin_user<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_ux, c->d_uy, c->d_uz, b->d_rep_of, b->d_reps,
                                                      c->d_cell_of, c->d_slot, c->d_count, c->d_err, c->d_key, hilbert ? 1 : 0);
+    Tiles tl;
+    if (hilbert) {
+        tl.start = c->d_tstart;
+        tl.tile[0] = c->d_tile[0];
+        tl.tile[1] = c->d_tile[1];
+        tl.pos = b->d_place_of;
+        tl.cell_groups = b->d_cell_groups;
+        k_tile_scan<<<1, 1024, 0, c->stream>>>(b->place[2], b->d_cell_at, c->d_count, tl);
+    }
     k_scan<<<1, 1024, 0, c->stream>>>(b->ncells, c->d_count, c->d_start, c->d_tot, c->d_work);
     k_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_cell_of, c->d_slot, c->d_start, c->d_tmp);
     k_cell_sort<<<b->ncells, 128, 0, c->stream>>>(c->d_start, c->d_tmp, c->d_sorted, c->d_key, c->d_sortkey,
-                                                   c->d_err);
+                                                   c->d_err, tl);
     k_gather_user<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_sorted, c->d_ux, c->d_uy, c->d_uz, q, type,
                                                        c->d_pos[buf], c->d_type[buf], c->d_id[buf], c->d_F64,
                                                        nullptr, c->d_cnt, c->p.ntypes, c->d_err);
@@ -682,12 +695,14 @@ extern "C" mdrl_status mdrl_batch_force_eval(mdrl_batch *b, const float *x, cons
     MDRL_CUDA(cudaMemsetAsync(c->d_tot, 0, sizeof(DevTotals), c->stream));
     MDRL_CUDA(cudaEventRecord(c->ev0, c->stream));
     const bool list = list_eval(c);
-    int slots = batch_slots(b);
+    TotUnits units{batch_slots(b)};
+    long long upto = units.n;
     MDRL_TRY(batch_bin_user(b, q ? c->d_uq : nullptr, type ? c->d_ut : nullptr, 0, list));
-    if (list) MDRL_TRY(batch_launch_list(b, c->d_pos[0], c->d_type[0], extra, &slots));
+    if (list) units = list_units(b, &upto);
+    if (list) MDRL_TRY(batch_launch_list(b, c->d_pos[0], c->d_type[0], extra));
     else MDRL_TRY(batch_launch_force(b, c->d_pos[0], c->d_type[0], extra, c->d_F64, extra ? nullptr : c->d_tot));
     b->list_slots = list;
-    if (extra) launch_totals(c, slots, 0, true);
+    if (extra) launch_totals(c, units, upto, 0, true);
     k_unsort<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_id[0], c->d_F64, nullptr, c->d_cnt, c->d_ox, c->d_oy,
                                                   c->d_oz, counts ? c->d_ocnt : nullptr);
     MDRL_CUDA(cudaGetLastError());
@@ -726,7 +741,7 @@ extern "C" mdrl_status mdrl_batch_set_state(mdrl_batch *b, const float *x, const
     b->list_slots = false;
     k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[0], c->d_type[0], c->d_F64, nullptr, c->d_mt, 0,
                                                 c->d_kepart);
-    launch_totals(c, batch_slots(b), nblk(n, 256), extra);
+    launch_totals(c, TotUnits{batch_slots(b)}, batch_slots(b), nblk(n, 256), extra);
     MDRL_CUDA(cudaGetLastError());
     MDRL_CUDA(cudaStreamSynchronize(c->stream));
     guard.done();
@@ -760,7 +775,7 @@ static mdrl_status batch_enqueue_step(mdrl_batch *b, bool extra) {
     if (vv || extra)
         k_kick<<<nblk(n, 256), 256, 0, c->stream>>>(n, c->d_vel[d], c->d_type[d], c->d_F64, nullptr, c->d_mt,
                                                     vv ? 1 : 0, extra ? c->d_kepart : nullptr);
-    if (extra) launch_totals(c, batch_slots(b), nblk(n, 256), true);
+    if (extra) launch_totals(c, TotUnits{batch_slots(b)}, batch_slots(b), nblk(n, 256), true);
     MDRL_CUDA(cudaGetLastError());
     return MDRL_OK;
 }
@@ -838,11 +853,12 @@ extern "C" mdrl_status mdrl_batch_replica_stats(mdrl_batch *b, mdrl_stats *out) 
     ListSlots ls{};
     if (list) {
         ls.on = 1;
-        ls.rep_pos = b->d_rep_pos;
+        ls.start = c->d_tstart;
+        ls.rep_place = b->d_rep_place;
+        for (int k = 0; k < 3; ++k) ls.place[k] = b->place[k];
         for (int k = 0; k < 2; ++k) {
-            ls.list[k] = b->lists[k].dev;
-            ls.first[k] = b->list_first[k];
-            ls.per_item[k] = b->list_per_item[k];
+            ls.first[k] = b->n_ot + (k ? (int)b->list_upto[0] : 0);
+            ls.fine[k] = b->list_fine[k];
         }
     }
     k_rep_totals<<<b->nrep, 128, 0, c->stream>>>(warp || list ? b->d_begin_ot : b->d_item_begin,

@@ -93,7 +93,8 @@ struct mdrl_ctx {
     int cur = 0;
     int *d_cell_of = nullptr, *d_slot = nullptr, *d_tmp = nullptr, *d_sorted = nullptr;
     int *d_count = nullptr, *d_start = nullptr;
-    int *d_work = nullptr;      /* the persistent force kernels' item counters [2] */
+    int *d_work = nullptr;      /* the persistent force kernels' item counters [2], then the list kernel's items [2] */
+    int2 *d_tstart = nullptr, *d_tile[2] = {nullptr, nullptr};   /* the list kernel's tiles (Tiles) */
     float *d_narrow = nullptr;  /* the narrow kernel's accumulators for crowded cells */
     bool narrow = false;        /* the state's steps take the narrow kernel (plan_narrow) */
     unsigned *d_key = nullptr;   /* in-cell sort key (Morton code inside the cell) */
@@ -152,9 +153,10 @@ mdrl_status prepare_force_kernel(force_fn fn, int device);
 /* Whether force evaluations run the list kernel, and its persistent grid: the CTAs that fit on the GPU
  * at once, or fewer when there are fewer items. */
 bool list_eval(const mdrl_ctx *c);
-/* The totals of the last force launch (nunits result slots, nke kinetic-energy partials) into d_tot. */
-void launch_totals(mdrl_ctx *c, int nunits, int nke, bool energy);
-mdrl_status list_grid(list_fn fn, size_t smem, int items, bool fine, int num_sms, int *grid);
+/* The totals of the last force launch (its result slots, at most `upto`; nke kinetic-energy partials) into
+ * d_tot. */
+void launch_totals(mdrl_ctx *c, const TotUnits &units, long long upto, int nke, bool energy);
+mdrl_status list_grid(list_fn fn, size_t smem, long long items, bool fine, int num_sms, int *grid);
 
 cudaStream_t pme_stream(const mdrl_ctx *c);    /* PME's own stream, or null without PME */
 

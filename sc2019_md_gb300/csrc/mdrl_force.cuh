@@ -246,7 +246,7 @@ struct BatchRep {
     int cell_off;    /* first global cell of the replica */
     int p_off, n;    /* its particles: [p_off, p_off + n) of the cell-sorted arrays */
     int path;        /* kPath* */
-    int tile_groups, split0, split1;   /* the list kernel's tiles and splits of a cell */
+    int tile_groups; /* the list kernel's (Tiles::groups) */
 };
 
 struct BatchItem {

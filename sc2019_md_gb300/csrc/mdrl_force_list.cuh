@@ -81,34 +81,25 @@ constexpr int kFineItems = 16;    /* per SM: below this many whole items a launc
 
 /* Whether a launch runs FINE items: the 4 warps of a CTA share each (one group of its tile each,
  * tiles of at most 4 groups), and an item is one run. */
-inline bool fine_items(int tg, int items, int num_sms) {
+inline bool fine_items(int tg, long long items, int num_sms) {
     return (tg & 0xff) <= kWarpsPerCta && (tg >> 8) <= kWarpsPerCta && items <= kFineItems * num_sms;
 }
 
-/* Splits of a home cell's tiles of tg groups (times the tile's steps_per_piece): about one tile
- * each, with 10 % to spare for fuller cells. */
-inline int list_split(long long n, int ncells, int tg) {
-    const double groups = 0.25 * (double)n / (ncells > 0 ? ncells : 1);
-    const int s = (int)(groups * 1.1 / tg) + 1;
-    return s < 1 ? 1 : (s > 64 ? 64 : s);
-}
-
-/* Result slots per home cell that any launch of a system can need. */
-inline int list_cell_slots(long long n, int ncells) {
-    const int tg = tile_groups(ncells), s0 = list_split(n, ncells, tg & 0xff), s1 = list_split(n, ncells, tg >> 8);
-    const bool may_fine = fine_items(tg, 0, 1);
-    return kMaxItemGroups * (may_fine ? kFineRuns * s0 : 2 * s0 + s1);
-}
-
-/* The cfg of a launch over `cells` home cells of one system of n particles and ncells cells, whether
- * its items are fine ones, and how many they are. */
-inline int list_cfg(long long n, int ncells, int cells, int G, int num_sms, bool *fine, int *items) {
+/* Items of a launch over `cells` of a system's ncells cells if its n particles fill them evenly, about one
+ * tile each with 10 % to spare: what the choice of FINE items goes by. */
+inline long long items_expected(long long n, int ncells, int cells) {
     const int tg = tile_groups(ncells);
-    const int s0 = std::min(255, list_split(n, ncells, tg & 0xff) * G), s1 = std::min(127, list_split(n, ncells, tg >> 8) * G);
-    *items = cells * (2 * s0 + s1);
-    *fine = fine_items(tg, *items, num_sms);
-    if (*fine) *items = cells * kFineRuns * s0;
-    return tg | (s0 << 16) | (s1 << 24);
+    const double groups = 1.1 * 0.25 * (double)n / (ncells > 0 ? ncells : 1);
+    return (long long)cells * (2 * ((int)(groups / (tg & 0xff)) + 1) + (int)(groups / (tg >> 8)) + 1);
+}
+
+/* The most tiles of tg groups that n particles in ncells cells can make, and the most items of a launch
+ * over them: its result slots. */
+inline long long tiles_max(long long n, int ncells, int tg) { return n / (4 * tg) + (n < ncells ? n : ncells); }
+inline long long items_max(long long n, int ncells, bool fine) {
+    const int tg = tile_groups(ncells);
+    const long long t0 = tiles_max(n, ncells, tg & 0xff);
+    return fine ? kFineRuns * t0 : 2 * t0 + tiles_max(n, ncells, tg >> 8);
 }
 
 /* Gathers of one table element per lane, issued only by the lanes whose candidate the filter accepted
@@ -179,7 +170,7 @@ struct ListSmem {
     unsigned char list[kListCap];        /* the current group's list: tile-list entries */
     /* the item's, tile's and column range's state: read back from here between the phases, so that
      * the pair loop has the registers */
-    int hs, ni, hz, cls, S, ti, ntile, i0, i1, ngr;
+    int hs, ni, hz, cls, i0, i1, ngr;
     int cbase[kMaxCols];                 /* first cell of each column */
     float sx, sy[kMaxCols];              /* the columns' x and y shifts */
     int range, jb, je, self, total, run, want;
@@ -200,19 +191,21 @@ inline size_t force_list_smem_bytes(int ntypes, bool extra) {
            kWarpsPerCta * (extra ? sizeof(ListSmem<true>) : sizeof(ListSmem<false>));
 }
 
-/* The replicas of a batch launch, by falling mean cell occupancy: replica rep[k]'s items of classes 0
- * and 1 are [pre0[k], pre0[k + 1]) of each class's total0, those of class 2 [pre1[k], pre1[k + 1]). */
-struct ListBatch {
-    const int *rep, *pre0, *pre1;
-    int nrep, total0;
+/* The tiles of a launch: of kind 0 tile[0][first->x .. last->x), of kind 1 tile[1][first->y .. last->y);
+ * groups per tile as Tiles::groups (a batch: its replicas').  Items, in launch order: the tiles of kind 0
+ * for class 0, for class 1, those of kind 1 for class 2; FINE (one kind) one per tile for every run of a
+ * class; MODE kDiffWrap one per tile. */
+struct ListTiles {
+    const int2 *first = nullptr, *last = nullptr;
+    const int2 *tile[2] = {nullptr, nullptr};
+    int groups = 0;
+    const int *rep_of_cell = nullptr;
 };
 
-/* The launch signature.  cfg: one system: tile groups (16 bits), splits of classes 0 and 1, splits of
- * class 2 (8 bits each); batch: the factor on each replica's splits.  cell0: first home cell (one
- * system).  work: the item counter, zero at launch. */
+/* The launch signature.  work: the item counter, zero at launch; nitems: receives the number of items. */
 typedef void (*list_fn)(const float4 *, const int *, const int *, Geom, TableDev, const float4 *, int, float, int,
-                        unsigned long long *, int *, UnitOut *, ListBatch, const BatchRep *, int, unsigned *, int,
-                        int *, int, DevTotals *);
+                        unsigned long long *, int *, UnitOut *, ListTiles, const BatchRep *, unsigned *, int *, int *,
+                        DevTotals *);
 
 /* Warp-wide minimum and maximum of floats. */
 __device__ __forceinline__ float warp_min(float v) {
@@ -282,17 +275,21 @@ __device__ __forceinline__ double hi_lo(const float (&v)[2]) {
     return isfinite(v[0]) ? (double)v[0] + v[1] : (double)v[0];
 }
 
-/* BATCH: the items are those of a batch's replicas (replica geometry, cell offset and splits from
- * reps); with MODE kDiffWrap they are (cell a, split) of replicas whose edges all exceed 2 rc: a's
- * particles against every later particle of the replica. */
+/* BATCH: the tiles are those of a batch's replicas (replica geometry, cell offset and tile groups from
+ * reps); with MODE kDiffWrap of replicas whose edges all exceed 2 rc: a tile's particles against every
+ * later particle of the replica. */
 template <int ORDER, bool SEP, bool EXTRA, int MODE, bool COUL, bool FINE, bool BATCH = false>
 __global__ void __launch_bounds__(32 * kWarpsPerCta, EXTRA ? 4 : kListCtas)
 k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, const int *__restrict__ cstart,
              Geom gparam, TableDev tab, const float4 *__restrict__ pcoef, int ntypes, float ke, int n,
              unsigned long long *__restrict__ F64, int *__restrict__ counts, UnitOut *__restrict__ uout,
-             ListBatch lb, const BatchRep *__restrict__ reps, int cfg, unsigned *__restrict__ err, int cell0,
-             int *__restrict__ work, int nitems, DevTotals *tot) {
+             ListTiles lt, const BatchRep *__restrict__ reps, unsigned *__restrict__ err, int *__restrict__ work,
+             int *__restrict__ nitems_out, DevTotals *tot) {
     constexpr bool kCellPair = BATCH && MODE == kDiffWrap;
+    const int2 tile0 = *lt.first, tile1 = *lt.last;
+    const int nt = tile1.x - tile0.x;
+    const int nitems = kCellPair ? nt : (FINE ? kFineRuns * nt : 2 * nt + (tile1.y - tile0.y));
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nitems_out = nitems;
     const int t2 = (ntypes * ntypes + 1) & ~1;
     extern __shared__ float4 wsm[];
     float2 *sCoefF = reinterpret_cast<float2 *>(wsm);           /* (A14, B8) [T^2] */
@@ -324,54 +321,36 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         }
         if (b >= nitems) break;
 
-        /* item -> home cell, class, split, run */
+        /* item -> class, run, home cell, tile */
         BatchRep rep;
         const Geom &g = BATCH ? rep.g : gparam;
-        int cend = 0, first_tile;
+        int cend = 0, tile, ntile;
         {
-            int h, cls = 0, sp, S, coff = 0, tgw, want = -1;    /* want: the one run of the item, -1: all */
+            int cls = 0, want = -1, coff = 0, tgw = lt.groups;      /* want: the one run of the item, -1: all */
+            int2 e;
+            if (kCellPair) {
+                e = lt.tile[0][tile0.x + b];
+                want = FINE ? 0 : -1;
+            } else if (FINE) {
+                const int q = b / nt;
+                cls = c_fine_class[q];
+                want = c_fine_run[q];
+                e = lt.tile[0][tile0.x + b - q * nt];
+            } else {
+                cls = b < nt ? 0 : (b < 2 * nt ? 1 : 2);
+                e = cls == 2 ? lt.tile[1][tile0.y + b - 2 * nt] : lt.tile[0][tile0.x + b - cls * nt];
+            }
             if (BATCH) {
-                const int q = FINE ? b / kRuns : b;
-                want = FINE ? b - q * kRuns : -1;
-                int u = q / cfg;
-                const int grp = q - u * cfg;
-                const int *pre = lb.pre0;
-                if (!kCellPair) {
-                    cls = min(u / lb.total0, 2);
-                    u -= cls * lb.total0;
-                    if (cls == 2) pre = lb.pre1;
-                }
-                int k0 = 0, k1 = lb.nrep - 1;        /* the last k with pre[k] <= u */
-                while (k0 < k1) {
-                    const int mid = (k0 + k1 + 1) >> 1;
-                    if (pre[mid] <= u) k0 = mid; else k1 = mid - 1;
-                }
-                rep = reps[lb.rep[k0]];
-                u -= pre[k0];
+                rep = reps[lt.rep_of_cell[e.x]];
                 coff = rep.cell_off;
                 cend = coff + g.nc[0] * g.nc[1] * g.nc[2];
                 tgw = rep.tile_groups;
-                const int split = cls == 2 ? rep.split1 : rep.split0;
-                h = u / split;
-                S = split * cfg;
-                sp = (u - h * split) * cfg + grp;
-            } else {
-                tgw = cfg & 0xffff;
-                const int S0 = (cfg >> 16) & 0xff, S1 = (cfg >> 24) & 0xff;
-                const int nh = nitems / (FINE ? kFineRuns * S0 : 2 * S0 + S1);
-                const int q = b / (nh * S0);
-                cls = FINE ? c_fine_class[q] : min(q, 2);
-                want = FINE ? c_fine_run[q] : -1;
-                S = cls == 2 ? S1 : S0;
-                const int rem = b - (FINE ? q : cls) * nh * S0;
-                h = rem / S;
-                sp = rem - h * S;
-                h += cell0;
             }
-            const int tg = cls == 2 ? tgw >> 8 : tgw & 0xff;
-            const int hs = cstart[coff + h], ni = cstart[coff + h + 1] - hs;
+            const int h = e.x - coff;
+            tile = e.y;
+            const int hs = cstart[e.x], ni = cstart[e.x + 1] - hs;
             /* the column: cells (cx, cy, hz - 1 .. hz + 1), or the home cell and the one above */
-            bool skip = ni > kMaxCellOcc;
+            bool skip = false;
             if (!kCellPair) {
                 const int nyz = g.nc[1] * g.nc[2];
                 const int hx = h / nyz, hy = (h / g.nc[2]) % g.nc[1], hz = h % g.nc[2];
@@ -393,11 +372,10 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                 }
                 s.hz = hz;
             }
-            s.hs = hs; s.ni = ni; s.cls = cls; s.S = S;
+            s.hs = hs; s.ni = ni; s.cls = cls;
             if (FINE) s.want = want;
-            /* the cell's tiles follow from its occupancy alone; the split takes every S-th */
-            s.ntile = skip ? 0 : (((ni + 3) >> 2) + tg - 1) / tg;
-            first_tile = sp;
+            /* the cell's tiles follow from its occupancy alone */
+            ntile = skip ? 0 : cell_tiles(ni, cls == 2 ? tgw >> 8 : tgw & 0xff);
         }
         __syncwarp();
 
@@ -405,14 +383,14 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         if (EXTRA && lane < kTileGroups)
             for (int d = 0; d < 3; ++d) s.eg[lane][d][0] = s.eg[lane][d][1] = 0.0f;
 
-        for (int ti = first_tile; ti < s.ntile; ti = s.ti + s.S) {
+        if (ntile) {
             {
-                const int ng = (s.ni + 3) >> 2, ga = ng * ti / s.ntile, gb = ng * (ti + 1) / s.ntile;
+                const int ng = (s.ni + 3) >> 2, ga = ng * tile / ntile, gb = ng * (tile + 1) / ntile;
                 const int i0 = s.hs + 4 * ga, i1 = min(s.hs + s.ni, s.hs + 4 * gb);
                 s.it[lane] = i0 + lane < i1 ? __ldg(ptype + i0 + lane) * ntypes : 0;
                 if (EXTRA) s.ci[lane] = 0;
                 __syncwarp();
-                s.ti = ti; s.i0 = i0; s.i1 = i1; s.ngr = gb - ga;
+                s.i0 = i0; s.i1 = i1; s.ngr = gb - ga;
                 s.range = 0; s.jb = 0; s.je = 0; s.run = -1; s.csy = s.csz = 3.0e38f;
                 __syncwarp();
             }

@@ -354,16 +354,66 @@ static __global__ void k_bin_user(int n, const float *__restrict__ x, const floa
     slot[i] = cell_slot(count, c);
 }
 
-/* Exclusive scan of the cell counts (one CTA), plus the largest occupancy; zeroes the totals' counts and
+/* The list kernel's tiles: a cell's groups of 4 particles are cut into tiles of at most `groups` groups,
+ * the low byte of it for the column classes 0 and 1, the next for class 2.  The scan of the counts numbers
+ * them, start[p] the first tiles of cell p (x, y: the two kinds), and the in-cell sort writes tile[kind][k] =
+ * (cell, tile of the cell).  So a launch has one item per tile that there is, however unevenly the cells
+ * are filled.  Batches: pos[c] the place of cell c in the order of the scan (-1: none), groups by cell. */
+struct Tiles {
+    int groups = 0;
+    int2 *start = nullptr;       /* null: no tiles wanted */
+    int2 *tile[2] = {nullptr, nullptr};
+    const int *pos = nullptr, *cell_groups = nullptr;
+};
+
+/* Tiles of 4 or 8 groups of a cell of m particles (none above the occupancy limit: what touches the cell
+ * is skipped). */
+__host__ __device__ constexpr int cell_tiles(int m, int groups) {
+    return m > kMaxCellOcc ? 0 : (groups == 8 ? (m + 31) >> 5 : (m + 15) >> 4);
+}
+__device__ __forceinline__ unsigned long long cell_tiles2(int m, int groups) {
+    return ((unsigned long long)cell_tiles(m, groups >> 8) << 32) | (unsigned)cell_tiles(m, groups & 0xff);
+}
+__device__ __forceinline__ int2 tiles_of(unsigned long long v) { return make_int2((int)(unsigned)v, (int)(v >> 32)); }
+
+/* The sum of `own` over the threads before this one plus carry; carry grows by the CTA's sum (1,024
+ * threads, one barrier: s_sum is another one at the next call). */
+template <class T>
+__device__ __forceinline__ T block_scan(T own, T &carry, T (&s_sum)[32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T sum = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+    }
+    if (lane == 31) s_sum[warp] = sum;
+    __syncthreads();
+    T ws = s_sum[lane];                  /* every warp scans the warp sums for itself */
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T v = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += v;
+    }
+    const T before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
+    const T first = carry + (warp ? before : T(0)) + sum - own;
+    carry += __shfl_sync(0xffffffffu, ws, 31);
+    return first;
+}
+
+/* Exclusive scan of the cell counts (one CTA), plus the largest occupancy, and of the tiles if wanted; zeroes the totals' counts and
  * the force launches' item counters work[0..1] on the way (a memset less per launch), and with clear the
  * counts it has read, for the next step's binning.  Latency-bound: 4 counts per
  * thread and pass in one 16-byte load, warp scans by shuffles, one barrier per pass of 4,096 cells.
  * (A strided run of cells per thread and a 20-barrier scan: 486 cells 3.8 us, 10,648 cells 9.9 us, 28k
  * cells 53 us; now 2.2, 3.3 and 6.) */
 static __global__ void __launch_bounds__(1024) k_scan(int ncells, int *__restrict__ count, int *__restrict__ start,
-                                               DevTotals *tot, int *work = nullptr, bool clear = false) {
+                                               DevTotals *tot, int *work = nullptr, bool clear = false,
+                                               Tiles tl = Tiles()) {
     __shared__ int s_sum[2][32], s_max[32];
+    __shared__ unsigned long long s_tiles[2][32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    unsigned long long tcarry = 0ull;
     if (work && t < 2) work[t] = 0;
     if (t == 0) tot->pairs = tot->below = 0ull;
     int carry = 0, mx = 0, pass = 0;
@@ -382,24 +432,21 @@ static __global__ void __launch_bounds__(1024) k_scan(int ncells, int *__restric
                 for (int u = k; u < ncells; ++u) count[u] = 0;
         }
         mx = max(mx, max(max(c.x, c.y), max(c.z, c.w)));
-        const int own = c.x + c.y + c.z + c.w;
-        int sum = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, sum, o);
-            if (lane >= o) sum += v;
+        const int first = block_scan(c.x + c.y + c.z + c.w, carry, s_sum[pass]);
+        if (tl.start) {
+            const unsigned long long t0 = cell_tiles2(c.x, tl.groups), t1 = t0 + cell_tiles2(c.y, tl.groups),
+                                     t2 = t1 + cell_tiles2(c.z, tl.groups), t3 = t2 + cell_tiles2(c.w, tl.groups);
+            const unsigned long long f = block_scan(t3, tcarry, s_tiles[pass]);
+            const int2 a = tiles_of(f), b = tiles_of(f + t0), d = tiles_of(f + t1), e = tiles_of(f + t2);
+            if (k + 3 < ncells) {
+                *reinterpret_cast<int4 *>(tl.start + k) = make_int4(a.x, a.y, b.x, b.y);
+                *reinterpret_cast<int4 *>(tl.start + k + 2) = make_int4(d.x, d.y, e.x, e.y);
+            } else {
+                if (k < ncells) tl.start[k] = a;
+                if (k + 1 < ncells) tl.start[k + 1] = b;
+                if (k + 2 < ncells) tl.start[k + 2] = d;
+            }
         }
-        if (lane == 31) s_sum[pass][warp] = sum;
-        __syncthreads();
-        int ws = s_sum[pass][lane];          /* every warp scans the warp sums for itself */
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, ws, o);
-            if (lane >= o) ws += v;
-        }
-        const int before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
-        const int first = carry + (warp ? before : 0) + sum - own;
-        carry += __shfl_sync(0xffffffffu, ws, 31);
         const int4 r = make_int4(first, first + c.x, first + c.x + c.y, first + c.x + c.y + c.z);
         if (k + 3 < ncells) *reinterpret_cast<int4 *>(start + k) = r;
         else {
@@ -413,8 +460,35 @@ static __global__ void __launch_bounds__(1024) k_scan(int ncells, int *__restric
     __syncthreads();
     if (warp == 0) {
         mx = __reduce_max_sync(0xffffffffu, s_max[lane]);
-        if (lane == 0) { start[ncells] = carry; tot->max_occ = mx; }
+        if (lane == 0) {
+            start[ncells] = carry;
+            tot->max_occ = mx;
+            if (tl.start) tl.start[ncells] = tiles_of(tcarry);
+        }
     }
+}
+
+/* The tiles of a batch's cells in another order than the storage's: place p holds cell cell_at[p]. */
+static __global__ void __launch_bounds__(1024) k_tile_scan(int nplaces, const int *__restrict__ cell_at,
+                                                    const int *__restrict__ count, Tiles tl) {
+    __shared__ unsigned long long s_tiles[2][32];
+    unsigned long long carry = 0ull;
+    int pass = 0;
+    for (int base = 0; base < nplaces; base += 4096, pass ^= 1) {
+        const int p = base + 4 * threadIdx.x;
+        unsigned long long t[4], sum = 0ull;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int c = p + u < nplaces ? cell_at[p + u] : -1;
+            t[u] = sum;
+            if (c >= 0) sum += cell_tiles2(count[c], tl.cell_groups[c]);
+        }
+        const unsigned long long f = block_scan(sum, carry, s_tiles[pass]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (p + u < nplaces) tl.start[p + u] = tiles_of(f + t[u]);
+    }
+    if (threadIdx.x == 0) tl.start[nplaces] = tiles_of(carry);
 }
 
 static __global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__restrict__ slot,
@@ -424,7 +498,7 @@ static __global__ void k_scatter(int n, const int *__restrict__ cell_of, const i
     tmp[start[cell_of[i]] + slot[i]] = i;
 }
 
-/* Order each cell's particles: by index (the reference's in-cell order, input order), or, when
+/* Also writes the cells' tiles (tl).  Order each cell's particles: by index (the reference's in-cell order, input order), or, when
  * key is given, by (key, index).  The rank of an element is the number of smaller ones (the
  * (key, index) pairs are distinct).  scratch[n] (64-bit) holds the sorted chunks of cells above
  * kSortSmall. */
@@ -433,11 +507,18 @@ static __global__ void __launch_bounds__(128) k_cell_sort(const int *__restrict_
                                                           int *__restrict__ sorted,
                                                           const unsigned *__restrict__ key,
                                                           unsigned long long *__restrict__ scratch,
-                                                          unsigned *__restrict__ err) {
+                                                          unsigned *__restrict__ err, Tiles tl = Tiles()) {
     __shared__ __align__(16) unsigned long long s_k[kSortSmall];
     const int c = blockIdx.x;
     const int s = start[c], m = start[c + 1] - s;
     if (m == 0) return;
+    const int place = !tl.start ? -1 : (tl.pos ? tl.pos[c] : c);
+    if (place >= 0) {
+        const int g = tl.cell_groups ? tl.cell_groups[c] : tl.groups;
+        const int2 at = tl.start[place];
+        for (int t = threadIdx.x; t < cell_tiles(m, g & 0xff); t += blockDim.x) tl.tile[0][at.x + t] = make_int2(c, t);
+        for (int t = threadIdx.x; t < cell_tiles(m, g >> 8); t += blockDim.x) tl.tile[1][at.y + t] = make_int2(c, t);
+    }
     if (m > kMaxCellOcc) {
         if (threadIdx.x == 0) atomicOr(err, kErrCellOverflow);
         for (int e = threadIdx.x; e < m; e += blockDim.x) sorted[s + e] = tmp[s + e];
@@ -543,6 +624,13 @@ struct TotScratch {
     TotPart part[kTotBlocks];
     unsigned done;                   /* CTAs finished; 0 between launches */
 };
+/* The result slots of a force launch: n; or of an evaluation by lists n, then count[0] more and, from slot
+ * `second` on, count2[0] (null: none), numbers that the launches have left on the device. */
+struct TotUnits {
+    int n;
+    const int *count = nullptr, *count2 = nullptr;
+    int second = 0;
+};
 inline int tot_blocks(int nunits, int nke) {
     const int b = ((nunits > nke ? nunits : nke) + 4 * kTotThreads - 1) / (4 * kTotThreads);
     return b < 1 ? 1 : (b > kTotBlocks ? kTotBlocks : b);
@@ -564,9 +652,11 @@ __device__ __forceinline__ void tot_tree(TotPart *s, int n, bool fp) {
     }
 }
 
-static __global__ void __launch_bounds__(kTotThreads) k_totals(int nunits, const UnitOut *__restrict__ uout,
+static __global__ void __launch_bounds__(kTotThreads) k_totals(TotUnits units, const UnitOut *__restrict__ uout,
                                                                int nke, const double *__restrict__ kepart,
                                                                DevTotals *tot, int with_energy, TotScratch *scr) {
+    const int upto = units.n + (units.count ? units.count[0] : 0);      /* slots [0, upto), then those from second */
+    const int nunits = upto + (units.count2 ? units.count2[0] : 0), skip = units.second - upto;
     __shared__ TotPart s[kTotThreads];
     __shared__ unsigned s_last;
     const int t = threadIdx.x, stride = gridDim.x * kTotThreads;
@@ -574,10 +664,11 @@ static __global__ void __launch_bounds__(kTotThreads) k_totals(int nunits, const
     TotPart a{};
 #pragma unroll 4
     for (int u = blockIdx.x * kTotThreads + t; u < nunits; u += stride) {
-        a.u[0] += uout[u].pairs;
+        const UnitOut &o = uout[u < upto ? u : u + skip];
+        a.u[0] += o.pairs;
         if (with_energy) {
-            a.e[0] += uout[u].e_lj; a.e[1] += uout[u].e_coul; a.e[2] += uout[u].virial;
-            a.u[1] += uout[u].below;
+            a.e[0] += o.e_lj; a.e[1] += o.e_coul; a.e[2] += o.virial;
+            a.u[1] += o.below;
         }
     }
 #pragma unroll 4
@@ -744,13 +835,14 @@ struct SmallShared {
     unsigned short cell[kSmallN];            /* the cell of each entry */
     unsigned short at[kSmallN];              /* cell-order position by index */
     int warp_sum[kSmallThreads / 32], warp_max[kSmallThreads / 32];
+    unsigned long long warp_tiles[kSmallThreads / 32];
 };
 
 /* Cell-order position of each of the thread's particles (index threadIdx.x + p * kSmallThreads, cell[p],
- * key[p]); fills start[] and tot->max_occ. */
+ * key[p]); fills start[], tot->max_occ and, if wanted, the tiles. */
 __device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, const int (&cell)[kSmallPer],
                                            const unsigned (&key)[kSmallPer], int (&at)[kSmallPer],
-                                           int *__restrict__ start, DevTotals *tot) {
+                                           int *__restrict__ start, DevTotals *tot, const Tiles &tl) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int k = t; k < ncells; k += kSmallThreads) s.count[k] = 0;
     __syncthreads();
@@ -788,6 +880,22 @@ __device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, co
     for (int k = 0; k < 4; ++k) {
         if (4 * t + k < ncells) { s.count[4 * t + k] = first; start[4 * t + k] = first; }
         first += c[k];
+    }
+    if (tl.start) {
+        unsigned long long own_t = 0ull, carry = 0ull;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) own_t += cell_tiles2(c[k], tl.groups);
+        unsigned long long f = block_scan(own_t, carry, s.warp_tiles);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (4 * t + k >= ncells) continue;
+            const int2 to = tiles_of(f);
+            tl.start[4 * t + k] = to;
+            for (int u = 0; u < cell_tiles(c[k], tl.groups & 0xff); ++u) tl.tile[0][to.x + u] = make_int2(4 * t + k, u);
+            for (int u = 0; u < cell_tiles(c[k], tl.groups >> 8); ++u) tl.tile[1][to.y + u] = make_int2(4 * t + k, u);
+            f += cell_tiles2(c[k], tl.groups);
+        }
+        if (t == 0) tl.start[ncells] = tiles_of(carry);
     }
     mx = __reduce_max_sync(0xffffffffu, s.warp_max[lane]);
     if (t == 0) { start[ncells] = n; tot->max_occ = mx; tot->pairs = tot->below = 0ull; }
@@ -837,7 +945,7 @@ k_small_user(int n, const float *__restrict__ x, const float *__restrict__ y, co
              const float *__restrict__ q, const int *__restrict__ type, Geom g, int ncells, int hilbert,
              float4 *__restrict__ pos, int *__restrict__ ptype, int *__restrict__ pid, int *__restrict__ inv,
              unsigned long long *__restrict__ F64, float *__restrict__ F32, int *__restrict__ counts, int ntypes,
-             int *__restrict__ start, DevTotals *tot, int *__restrict__ work, unsigned *__restrict__ err) {
+             int *__restrict__ start, DevTotals *tot, int *__restrict__ work, unsigned *__restrict__ err, Tiles tl) {
     extern __shared__ float4 small_sm[];
     SmallShared &s = *reinterpret_cast<SmallShared *>(small_sm);
     __shared__ unsigned s_err;
@@ -863,7 +971,7 @@ k_small_user(int n, const float *__restrict__ x, const float *__restrict__ y, co
         cell[k] = cell_of_pos(g, p[k].x, p[k].y, p[k].z);
         key[k] = hilbert ? cell_hilbert(g, p[k].x, p[k].y, p[k].z, cell[k]) : cell_morton(g, p[k].x, p[k].y, p[k].z, cell[k]);
     }
-    small_sort(s, n, ncells, cell, key, at, start, tot);
+    small_sort(s, n, ncells, cell, key, at, start, tot, tl);
 #pragma unroll
     for (int k = 0; k < kSmallPer; ++k) {
         const int i = threadIdx.x + k * kSmallThreads;
@@ -910,7 +1018,7 @@ k_small_state(int n, const float4 *__restrict__ pos0, const float4 *__restrict__
         key[q] = cell_morton(g, p[q].x, p[q].y, p[q].z, cell[q]);
         clear_force(n, k, F64, F32, counts);     /* the thread's own entries, read above */
     }
-    small_sort(s, n, ncells, cell, key, at, start, tot);
+    small_sort(s, n, ncells, cell, key, at, start, tot, Tiles());
 #pragma unroll
     for (int q = 0; q < kSmallPer; ++q) {
         if ((int)threadIdx.x + q * kSmallThreads >= n) continue;

@@ -54,10 +54,14 @@ namespace {
 
 constexpr size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
+constexpr int kStaticTiles = kStaticMaxN / 16 + kStaticMaxCells;   /* the list kernel's, of one kind */
+/* its items: 3 per tile, or 10 in launches of few (items_expected is above 0.2 n) */
+static_assert(3 * kStaticTiles <= kHalfShellCells * kStaticMaxCells, "result slots");
+
 /* Byte offsets of the sub-buffers inside the array. */
 struct Layout {
     size_t err, tot, count, start, unit, cell_of, slot, tmp, sorted, key, sortkey, pos, type, id, F64, tabf,
-        tabe, wa, wb, wc, pcoef, work, end;
+        tabe, wa, wb, wc, pcoef, work, tstart, tile, end;
 };
 
 constexpr Layout make_layout() {
@@ -84,7 +88,9 @@ constexpr Layout make_layout() {
     l.wb = o;      o = align256(o + sizeof(float4) * kStaticMaxTable);
     l.wc = o;      o = align256(o + sizeof(float2) * kStaticMaxTable);
     l.pcoef = o;   o = align256(o + sizeof(float4) * MDRL_MAX_TYPES * MDRL_MAX_TYPES);
-    l.work = o;    o = align256(o + 2 * sizeof(int));
+    l.work = o;    o = align256(o + 4 * sizeof(int));
+    l.tstart = o;  o = align256(o + sizeof(int2) * (kStaticMaxCells + 1));
+    l.tile = o;    o = align256(o + 2 * sizeof(int2) * kStaticTiles);
     l.end = o;
     return l;
 }
@@ -326,18 +332,25 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
     const int blk = 256, grid = (n + blk - 1) / blk;
     if (n > 0) k_bin_user<<<grid, blk, 0, st>>>(n, x, y, z, g, d_cell_of, d_slot, d_count, d_err, d_key, nullptr,
                                              nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 1);
-    k_scan<<<1, 1024, 0, st>>>(nc, d_count, d_start, d_tot, (int *)(b + kLayout.work));
+    int *d_work = (int *)(b + kLayout.work);
+    int2 *d_tile = (int2 *)(b + kLayout.tile);
+    Tiles tl;
+    tl.groups = tile_groups(nc);
+    tl.start = (int2 *)(b + kLayout.tstart);
+    tl.tile[0] = d_tile;
+    tl.tile[1] = d_tile + kStaticTiles;
+    k_scan<<<1, 1024, 0, st>>>(nc, d_count, d_start, d_tot, d_work, false, tl);
     if (n > 0) {
         k_scatter<<<grid, blk, 0, st>>>(n, d_cell_of, d_slot, d_start, d_tmp);
-        k_cell_sort<<<nc, 128, 0, st>>>(d_start, d_tmp, d_sorted, d_key, d_sortkey, d_err);
+        k_cell_sort<<<nc, 128, 0, st>>>(d_start, d_tmp, d_sorted, d_key, d_sortkey, d_err, tl);
         k_gather_user<<<grid, blk, 0, st>>>(n, d_sorted, x, y, z, q, type, d_pos, d_type, d_id, d_F64, nullptr,
                                             nullptr, p->ntypes, d_err);
     }
     const int ord = p->eval == MDRL_EVAL_DIRECT ? 0 : order;
-    int sms = 0, items = 0, ctas = 0;
-    bool fine;
+    int sms = 0;
     ST_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int cfg = list_cfg(n, nc, nc, 1, sms, &fine, &items);
+    const bool fine = fine_items(tl.groups, items_expected(n, nc, nc), sms);
+    const long long items = items_max(n, nc, fine);
     if (items > kHalfShellCells * kStaticMaxCells) return fail(MDRL_ERR_RANGE, "too many work items for the static scratch");
     const bool sep = p->arith == MDRL_ARITH_SEPARATE, coul = p->coulomb_k != 0.0;
     list_fn fn = (p->flags & MDRL_FLAG_EXACT_DIFF) ? pick_force_list<kDiffExact, false>(ord, false, false, coul, fine)
@@ -347,10 +360,16 @@ extern "C" mdrl_status mdrl_force_eval_static(const mdrl_params *p, int n, const
                                  (int)force_smem_bytes(MDRL_MAX_TYPES, true, 8)));
     int per_sm = 0;
     ST_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, 32 * kWarpsPerCta, smem));
-    ctas = std::min(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta, std::max(1, per_sm) * std::max(1, sms));
-    fn<<<ctas, 32 * kWarpsPerCta, smem, st>>>(d_pos, d_type, d_start, g, tab, d_pcoef, p->ntypes, (float)p->coulomb_k, n,
-                                              d_F64, nullptr, d_unit, ListBatch{}, nullptr, cfg, d_err, 0,
-                                              (int *)(b + kLayout.work), items, d_tot);
+    const int ctas = (int)std::min<long long>(fine ? items : (items + kWarpsPerCta - 1) / kWarpsPerCta,
+                                              std::max(1, per_sm) * std::max(1, sms));
+    ListTiles lt;
+    lt.first = tl.start;
+    lt.last = tl.start + nc;
+    lt.tile[0] = tl.tile[0];
+    lt.tile[1] = tl.tile[1];
+    lt.groups = tl.groups;
+    fn<<<std::max(1, ctas), 32 * kWarpsPerCta, smem, st>>>(d_pos, d_type, d_start, g, tab, d_pcoef, p->ntypes, (float)p->coulomb_k, n,
+                                              d_F64, nullptr, d_unit, lt, nullptr, d_err, d_work, d_work + 2, d_tot);
     if (n > 0)
         k_unsort<<<grid, blk, 0, st>>>(n, d_id, d_F64, nullptr, nullptr, fx, fy, fz, nullptr);
     ST_CUDA(cudaGetLastError());
