@@ -182,7 +182,7 @@ struct ListSmem {
     unsigned pairs, below;               /* sums of a warp that shares its items */
     int ci[EXTRA ? 32 : 1];              /* partner counts (energy launches) */
     int cj[EXTRA ? kListCap : 1];
-    float eg[EXTRA ? kTileGroups : 1][3][2];   /* the item's energies and virial by group, as hi + lo */
+    double e[EXTRA ? 3 : 1];             /* energies and virial of a warp that shares its items */
 };
 
 inline size_t force_list_smem_bytes(int ntypes, bool extra) {
@@ -249,31 +249,8 @@ __device__ __forceinline__ void reduce_scatter12(float (&v)[12], int lane) {
     v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-/* Sums of a, b and c over the 32 lanes as hi (returned) + lo, of a in lanes 0-7, of b in 8-15, of c in
- * 16-23: every addition's rounding error goes to lo, so the sum is one to ~2^-46 of its largest term (an
- * FP64 shuffle tree without FP64, which this part runs at 1/64 of its FP32 rate; evaluation of 31,007 atoms with energies 304 -> 310 us). */
-__device__ __forceinline__ float warp_sums(float a, float b, float c, int lane, float &lo) {
-    const bool b16 = lane & 16, b8 = lane & 8;
-    float e0, e1, e;
-    /* lanes 0-15 keep a and b, lanes 16-31 c (and nothing) */
-    const float r0 = __shfl_xor_sync(0xffffffffu, b16 ? a : c, 16), r1 = __shfl_xor_sync(0xffffffffu, b16 ? b : 0.0f, 16);
-    const float s0 = two_sum(b16 ? c : a, r0, e0), s1 = two_sum(b16 ? 0.0f : b, r1, e1);
-    const float h = __shfl_xor_sync(0xffffffffu, b8 ? s0 : s1, 8), l = __shfl_xor_sync(0xffffffffu, b8 ? e0 : e1, 8);
-    float hi = two_sum(b8 ? s1 : s0, h, e);
-    lo = (b8 ? e1 : e0) + l + e;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-        const float h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-        hi = two_sum(hi, h2, e);
-        lo += l2 + e;
-    }
-    return hi;
-}
-
 /* hi + lo in FP64; an infinite or NaN hi by itself, whose lo is NaN. */
-__device__ __forceinline__ double hi_lo(const float (&v)[2]) {
-    return isfinite(v[0]) ? (double)v[0] + v[1] : (double)v[0];
-}
+__device__ __forceinline__ double hi_lo(float hi, float lo) { return isfinite(hi) ? (double)hi + lo : (double)hi; }
 
 /* BATCH: the tiles are those of a batch's replicas (replica geometry, cell offset and tile groups from
  * reps); with MODE kDiffWrap of replicas whose edges all exceed 2 rc: a tile's particles against every
@@ -380,8 +357,10 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         __syncwarp();
 
         unsigned acc_pairs = 0, acc_below = 0;
-        if (EXTRA && lane < kTileGroups)
-            for (int d = 0; d < 3; ++d) s.eg[lane][d][0] = s.eg[lane][d][1] = 0.0f;
+        /* energies and virial of the lane over the item: a visit's FP32 sums are added up with their rounding
+         * errors beside them (2^-46 of the largest; FP64 runs at 1/64 of the FP32 rate), so that the totals do
+         * not depend on how visits are shared among warps and items */
+        float ehi[3] = {0.0f, 0.0f, 0.0f}, elo[3] = {0.0f, 0.0f, 0.0f};
 
         if (ntile) {
             {
@@ -660,15 +639,10 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                                 const int c = __reduce_add_sync(0xffffffffu, ci[k]);
                                 if (lane == 0) s.ci[4 * gi + k] += c;
                             }
-                            /* to the group's sums: lanes 0, 8, 16 hold the three as hi + lo */
-                            float lo;
-                            const float hi = warp_sums(acc_elj, acc_ec, acc_vir, lane, lo);
-                            if ((lane & 7) == 0 && lane < 24) {
-                                float (&sum)[2] = s.eg[gi][lane >> 3];
-                                float e;
-                                sum[0] = two_sum(sum[0], hi, e);
-                                sum[1] += e + lo;
-                            }
+                            float e;
+                            ehi[0] = two_sum(ehi[0], acc_elj, e); elo[0] += e;
+                            if (COUL) { ehi[1] = two_sum(ehi[1], acc_ec, e); elo[1] += e; }
+                            ehi[2] = two_sum(ehi[2], acc_vir, e); elo[2] += e;
                         }
                         __syncwarp();   /* the next group's lanes hold other entries of the list */
                     }
@@ -706,23 +680,25 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         unsigned c1 = __reduce_add_sync(0xffffffffu, acc_pairs);
         unsigned c2 = EXTRA ? __reduce_add_sync(0xffffffffu, acc_below) : 0u;
         double e1 = 0.0, e2 = 0.0, e3 = 0.0;
+        if (EXTRA) {
+            e1 = hi_lo(ehi[0], elo[0]); e2 = COUL ? hi_lo(ehi[1], elo[1]) : 0.0; e3 = hi_lo(ehi[2], elo[2]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                e1 += __shfl_xor_sync(0xffffffffu, e1, o);
+                if (COUL) e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+                e3 += __shfl_xor_sync(0xffffffffu, e3, o);
+            }
+        }
         if (FINE) {
-            if (lane == 0) { s.pairs = c1; s.below = c2; }
+            if (lane == 0) {
+                s.pairs = c1; s.below = c2;
+                if (EXTRA) { s.e[0] = e1; s.e[1] = e2; s.e[2] = e3; }
+            }
             __syncthreads();
             if (warp != 0) continue;
-            c1 = c2 = 0;
-            for (int w = 0; w < kWarpsPerCta; ++w) { c1 += all[w].pairs; c2 += all[w].below; }
-        }
-        if (EXTRA) {
-            if (lane < (FINE ? kWarpsPerCta : kTileGroups)) {
-                const float (*eg)[2] = FINE ? all[lane].eg[lane] : s.eg[lane];
-                e1 = hi_lo(eg[0]); e2 = hi_lo(eg[1]); e3 = hi_lo(eg[2]);
-            }
-#pragma unroll
-            for (int o = kTileGroups / 2; o > 0; o >>= 1) {
-                e1 += __shfl_xor_sync(0xffffffffu, e1, o);
-                e2 += __shfl_xor_sync(0xffffffffu, e2, o);
-                e3 += __shfl_xor_sync(0xffffffffu, e3, o);
+            for (int w = 1; w < kWarpsPerCta; ++w) {
+                c1 += all[w].pairs; c2 += all[w].below;
+                if (EXTRA) { e1 += all[w].e[0]; e2 += all[w].e[1]; e3 += all[w].e[2]; }
             }
         }
         if (lane == 0) {
