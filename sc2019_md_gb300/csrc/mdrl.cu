@@ -522,7 +522,7 @@ mdrl_status mdrl::prepare_force_kernel(force_fn fn, int device) {
     const std::pair<const void *, int> key((const void *)fn, device);
     if (!done.count(key)) {
         MDRL_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)force_smem_bytes(MDRL_MAX_TYPES, true, 8)));
+                                       (int)std::max(force_smem_bytes(MDRL_MAX_TYPES, true, 8), sizeof(SmallShared))));
         done.insert(key);
     }
     return MDRL_OK;
@@ -695,9 +695,10 @@ static mdrl_status bin_user(mdrl_ctx *c, int n, const float *x, const float *y, 
         tl.tile[1] = c->d_tile[1];
     }
     if (spatial && small_system(c, n)) {
-        MDRL_TRY(prepare_force_kernel((force_fn)k_small_user, c->p.device));
-        k_small_user<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
-            n, x, y, z, q, type, c->g, c->ncells, hilbert ? 1 : 0, c->d_pos[buf], c->d_type[buf], c->d_id[buf],
+        auto fn = hilbert ? k_small_user<true> : k_small_user<false>;
+        MDRL_TRY(prepare_force_kernel((force_fn)fn, c->p.device));
+        fn<<<1, kSmallThreads, sizeof(SmallShared), c->stream>>>(
+            n, x, y, z, q, type, c->g, c->ncells, c->d_pos[buf], c->d_type[buf], c->d_id[buf],
             inv ? c->d_inv : nullptr, c->d_F64, c->d_F32, c->d_cnt, c->p.ntypes, c->d_start, c->d_tot, c->d_work,
             c->d_err, tl);
         MDRL_CUDA(cudaGetLastError());

@@ -179,6 +179,8 @@ struct ListSmem {
     float js[3];                         /* exact rule: taken off the j coordinates */
     float sd[3];                         /* kDiffShift: added to every difference */
     int next;                            /* the CTA's item when its warps share items */
+    int2 tile0;                          /* the launch's first tiles, tiles of kind 0 and items */
+    int nt, nitems;
     unsigned pairs, below;               /* sums of a warp that shares its items */
     int ci[EXTRA ? 32 : 1];              /* partner counts (energy launches) */
     int cj[EXTRA ? kListCap : 1];
@@ -264,9 +266,6 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
              int *__restrict__ nitems_out, DevTotals *tot) {
     constexpr bool kCellPair = BATCH && MODE == kDiffWrap;
     const int2 tile0 = *lt.first, tile1 = *lt.last;
-    const int nt = tile1.x - tile0.x;
-    const int nitems = kCellPair ? nt : (FINE ? kFineRuns * nt : 2 * nt + (tile1.y - tile0.y));
-    if (blockIdx.x == 0 && threadIdx.x == 0) *nitems_out = nitems;
     const int t2 = (ntypes * ntypes + 1) & ~1;
     extern __shared__ float4 wsm[];
     float2 *sCoefF = reinterpret_cast<float2 *>(wsm);           /* (A14, B8) [T^2] */
@@ -281,23 +280,34 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
     }
     __syncthreads();
 
+    {
+        const int nt = tile1.x - tile0.x;
+        const int nitems = kCellPair ? nt : (FINE ? kFineRuns * nt : 2 * nt + (tile1.y - tile0.y));
+        if (blockIdx.x == 0 && threadIdx.x == 0) *nitems_out = nitems;
+        s.tile0 = tile0;
+        s.nt = nt;
+        s.nitems = nitems;
+        __syncwarp();
+    }
+
     const float far = 1.0e18f;
     const unsigned below = (1u << lane) - 1u;
 
     unsigned long long pairs_sum = 0;    /* lane 0: the warp's items' */
-    for (;;) {
+    /* the items of this warp (FINE: CTA): its own number first, then the next from the counter */
+    const int workers = FINE ? gridDim.x : kWarpsPerCta * gridDim.x;
+    auto next = [&]() {
         int b = 0;
         if (FINE) {
             __syncthreads();
-            if (threadIdx.x == 0) all[0].next = atomicAdd(work, 1);
+            if (threadIdx.x == 0) all[0].next = workers + atomicAdd(work, 1);
             __syncthreads();
-            b = all[0].next;
-        } else {
-            if (lane == 0) b = atomicAdd(work, 1);
-            b = __shfl_sync(0xffffffffu, b, 0);
+            return all[0].next;
         }
-        if (b >= nitems) break;
-
+        if (lane == 0) b = workers + atomicAdd(work, 1);
+        return __shfl_sync(0xffffffffu, b, 0);
+    };
+    for (int b = FINE ? blockIdx.x : kWarpsPerCta * blockIdx.x + warp; b < s.nitems; b = next()) {
         /* item -> class, run, home cell, tile */
         BatchRep rep;
         const Geom &g = BATCH ? rep.g : gparam;
@@ -305,6 +315,8 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
         {
             int cls = 0, want = -1, coff = 0, tgw = lt.groups;      /* want: the one run of the item, -1: all */
             int2 e;
+            const int2 tile0 = s.tile0;
+            const int nt = s.nt;
             if (kCellPair) {
                 e = lt.tile[0][tile0.x + b];
                 want = FINE ? 0 : -1;

@@ -834,15 +834,17 @@ struct SmallShared {
     unsigned long long key[kSmallN];         /* (key, index), cell by cell */
     unsigned short cell[kSmallN];            /* the cell of each entry */
     unsigned short at[kSmallN];              /* cell-order position by index */
-    int warp_sum[kSmallThreads / 32], warp_max[kSmallThreads / 32];
-    unsigned long long warp_tiles[kSmallThreads / 32];
+    int warp_max[kSmallThreads / 32];
+    union { int i[kSmallThreads / 32]; unsigned long long u[kSmallThreads / 32]; } warp_sum;
+    unsigned tile_start[kSmallCells];        /* first tiles of the two kinds, 16 bits each */
 };
 
 /* Cell-order position of each of the thread's particles (index threadIdx.x + p * kSmallThreads, cell[p],
  * key[p]); fills start[], tot->max_occ and, if wanted, the tiles. */
+template <bool TILES>
 __device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, const int (&cell)[kSmallPer],
                                            const unsigned (&key)[kSmallPer], int (&at)[kSmallPer],
-                                           int *__restrict__ start, DevTotals *tot, const Tiles &tl) {
+                                           int *__restrict__ start, DevTotals *tot, const Tiles &tl = Tiles()) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int k = t; k < ncells; k += kSmallThreads) s.count[k] = 0;
     __syncthreads();
@@ -851,51 +853,43 @@ __device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, co
     for (int p = 0; p < kSmallPer; ++p)
         if (t + p * kSmallThreads < n) slot[p] = atomicAdd(&s.count[cell[p]], 1);
     __syncthreads();
-    /* exclusive scan, 4 cells per thread */
-    int c[4], own = 0, mx = 0;
+    /* exclusive scan, 4 cells per thread; with tiles, of counts and both kinds of tiles together (at most
+     * 4,096 + 256 each, 20 bits) */
+    int c[4], mx = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         c[k] = 4 * t + k < ncells ? s.count[4 * t + k] : 0;
-        own += c[k];
         mx = max(mx, c[k]);
     }
-    int sum = own;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, sum, o);
-        if (lane >= o) sum += v;
-    }
     mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane == 31) { s.warp_sum[warp] = sum; s.warp_max[warp] = mx; }
-    __syncthreads();
-    int ws = s.warp_sum[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, ws, o);
-        if (lane >= o) ws += v;
-    }
-    const int before = __shfl_sync(0xffffffffu, ws, max(warp - 1, 0));
-    int first = (warp ? before : 0) + sum - own;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (4 * t + k < ncells) { s.count[4 * t + k] = first; start[4 * t + k] = first; }
-        first += c[k];
-    }
-    if (tl.start) {
-        unsigned long long own_t = 0ull, carry = 0ull;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) own_t += cell_tiles2(c[k], tl.groups);
-        unsigned long long f = block_scan(own_t, carry, s.warp_tiles);
+    if (lane == 0) s.warp_max[warp] = mx;
+    if (TILES) {
+        unsigned long long v[4], own = 0ull, carry = 0ull;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (4 * t + k >= ncells) continue;
-            const int2 to = tiles_of(f);
-            tl.start[4 * t + k] = to;
-            for (int u = 0; u < cell_tiles(c[k], tl.groups & 0xff); ++u) tl.tile[0][to.x + u] = make_int2(4 * t + k, u);
-            for (int u = 0; u < cell_tiles(c[k], tl.groups >> 8); ++u) tl.tile[1][to.y + u] = make_int2(4 * t + k, u);
-            f += cell_tiles2(c[k], tl.groups);
+            v[k] = (unsigned)c[k] | ((unsigned long long)cell_tiles(c[k], tl.groups & 0xff) << 20) |
+                   ((unsigned long long)cell_tiles(c[k], tl.groups >> 8) << 40);
+            own += v[k];
         }
-        if (t == 0) tl.start[ncells] = tiles_of(carry);
+        unsigned long long f = block_scan(own, carry, s.warp_sum.u);
+#pragma unroll
+        for (int k = 0; k < 4; ++k, f += v[k - 1]) {
+            if (4 * t + k >= ncells) continue;
+            const int first = (int)(f & 0xfffffu);
+            const int2 to = make_int2((int)(f >> 20) & 0xfffff, (int)(f >> 40));
+            s.count[4 * t + k] = first;
+            start[4 * t + k] = first;
+            s.tile_start[4 * t + k] = (unsigned)to.x | ((unsigned)to.y << 16);
+            tl.start[4 * t + k] = to;
+        }
+        if (t == 0) tl.start[ncells] = make_int2((int)(carry >> 20) & 0xfffff, (int)(carry >> 40));
+    } else {
+        int carry = 0, first = block_scan(c[0] + c[1] + c[2] + c[3], carry, s.warp_sum.i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (4 * t + k < ncells) { s.count[4 * t + k] = first; start[4 * t + k] = first; }
+            first += c[k];
+        }
     }
     mx = __reduce_max_sync(0xffffffffu, s.warp_max[lane]);
     if (t == 0) { start[ncells] = n; tot->max_occ = mx; tot->pairs = tot->below = 0ull; }
@@ -918,6 +912,11 @@ __device__ __forceinline__ void small_sort(SmallShared &s, int n, int ncells, co
         if (e >= n) continue;
         const unsigned long long me = s.key[e];
         const int cl = s.cell[e], a = s.count[cl], b = cl + 1 < ncells ? s.count[cl + 1] : n;
+        if (TILES) {      /* entry u of a cell writes tile u (a tile has at least one particle) */
+            const unsigned to = s.tile_start[cl];
+            if (e - a < cell_tiles(b - a, tl.groups & 0xff)) tl.tile[0][(to & 0xffffu) + e - a] = make_int2(cl, e - a);
+            if (e - a < cell_tiles(b - a, tl.groups >> 8)) tl.tile[1][(to >> 16) + e - a] = make_int2(cl, e - a);
+        }
         int rank = 0;
 #pragma unroll 4
         for (int q = a; q < b; ++q) rank += s.key[q] < me;
@@ -939,10 +938,12 @@ __device__ __forceinline__ void clear_force(int n, int k, unsigned long long *F6
 }
 
 /* User-order inputs (device memory, or host memory the device reads) into cell order: k_bin_user, k_scan,
- * k_scatter, k_cell_sort and k_gather_user in one.  Also clears the error word and the item counters. */
+ * k_scatter, k_cell_sort and k_gather_user in one, in the list kernel's order and with its tiles or in the
+ * other kernels' order.  Also clears the error word and the item counters. */
+template <bool LIST>
 static __global__ void __launch_bounds__(kSmallThreads)
 k_small_user(int n, const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-             const float *__restrict__ q, const int *__restrict__ type, Geom g, int ncells, int hilbert,
+             const float *__restrict__ q, const int *__restrict__ type, Geom g, int ncells,
              float4 *__restrict__ pos, int *__restrict__ ptype, int *__restrict__ pid, int *__restrict__ inv,
              unsigned long long *__restrict__ F64, float *__restrict__ F32, int *__restrict__ counts, int ntypes,
              int *__restrict__ start, DevTotals *tot, int *__restrict__ work, unsigned *__restrict__ err, Tiles tl) {
@@ -969,9 +970,9 @@ k_small_user(int n, const float *__restrict__ x, const float *__restrict__ y, co
         if (!in_box(g, p[k].x, p[k].y, p[k].z)) atomicOr(&s_err, kErrPosition);
         if (ty[k] < 0 || ty[k] >= ntypes) { atomicOr(&s_err, kErrType); ty[k] = 0; }
         cell[k] = cell_of_pos(g, p[k].x, p[k].y, p[k].z);
-        key[k] = hilbert ? cell_hilbert(g, p[k].x, p[k].y, p[k].z, cell[k]) : cell_morton(g, p[k].x, p[k].y, p[k].z, cell[k]);
+        key[k] = LIST ? cell_hilbert(g, p[k].x, p[k].y, p[k].z, cell[k]) : cell_morton(g, p[k].x, p[k].y, p[k].z, cell[k]);
     }
-    small_sort(s, n, ncells, cell, key, at, start, tot, tl);
+    small_sort<LIST>(s, n, ncells, cell, key, at, start, tot, tl);
 #pragma unroll
     for (int k = 0; k < kSmallPer; ++k) {
         const int i = threadIdx.x + k * kSmallThreads;
@@ -1018,7 +1019,7 @@ k_small_state(int n, const float4 *__restrict__ pos0, const float4 *__restrict__
         key[q] = cell_morton(g, p[q].x, p[q].y, p[q].z, cell[q]);
         clear_force(n, k, F64, F32, counts);     /* the thread's own entries, read above */
     }
-    small_sort(s, n, ncells, cell, key, at, start, tot, Tiles());
+    small_sort<false>(s, n, ncells, cell, key, at, start, tot);
 #pragma unroll
     for (int q = 0; q < kSmallPer; ++q) {
         if ((int)threadIdx.x + q * kSmallThreads >= n) continue;
