@@ -170,7 +170,7 @@ struct ListSmem {
     unsigned char list[kListCap];        /* the current group's list: tile-list entries */
     /* the item's, tile's and column range's state: read back from here between the phases, so that
      * the pair loop has the registers */
-    int hs, ni, hz, cls, i0, i1, ngr;
+    int hs, ni, hx, hy, hz, cls, i0, i1, ngr;
     int cbase[kMaxCols];                 /* first cell of each column */
     float sx, sy[kMaxCols];              /* the columns' x and y shifts */
     int range, jb, je, self, total, run, want;
@@ -179,8 +179,6 @@ struct ListSmem {
     float js[3];                         /* exact rule: taken off the j coordinates */
     float sd[3];                         /* kDiffShift: added to every difference */
     int next;                            /* the CTA's item when its warps share items */
-    int2 tile0;                          /* the launch's first tiles, tiles of kind 0 and items */
-    int nt, nitems;
     unsigned pairs, below;               /* sums of a warp that shares its items */
     int ci[EXTRA ? 32 : 1];              /* partner counts (energy launches) */
     int cj[EXTRA ? kListCap : 1];
@@ -208,6 +206,44 @@ struct ListTiles {
 typedef void (*list_fn)(const float4 *, const int *, const int *, Geom, TableDev, const float4 *, int, float, int,
                         unsigned long long *, int *, UnitOut *, ListTiles, const BatchRep *, unsigned *, int *, int *,
                         DevTotals *);
+
+/* Cells along an axis that can hold a partner of a particle of cell 0, on either side: 1 as the cells are
+ * at least rc wide, 2 where one that is barely so could lose a pair to rounding. */
+__device__ __forceinline__ int axis_reach(const Geom &g, int d) { return g.edge[d] * g.edge[d] > 1.00001f * g.rc2 ? 1 : 2; }
+
+/* The cells that the particles of cell (hx, hy, hz) of a replica with minimum images pair with, among the
+ * later ones of its storage order: range r of ranges(), cells [z0, z1] of column (cx, cy); false:
+ * none.  Two ranges per column of the window around the home cell, the second one for what lies across
+ * the z face; the home column starts at the home cell. */
+struct WrapWindow {
+    int rx, ry, rz, nx, ny;              /* reach; columns of the window along x and y */
+    __device__ __forceinline__ WrapWindow(const Geom &g) {
+        rx = axis_reach(g, 0); ry = axis_reach(g, 1); rz = axis_reach(g, 2);
+        nx = min(g.nc[0], 2 * rx + 1);
+        ny = min(g.nc[1], 2 * ry + 1);
+    }
+    __device__ __forceinline__ int ranges() const { return 2 * nx * ny; }
+    __device__ __forceinline__ bool range(const Geom &g, int hx, int hy, int hz, int r, int &col, int &z0, int &z1) const {
+        const int k = r >> 1, ix = k / ny, iy = k - ix * ny;
+        int cx = ix, cy = iy;
+        if (nx < g.nc[0]) { cx = hx - rx + ix; cx += cx < 0 ? g.nc[0] : (cx >= g.nc[0] ? -g.nc[0] : 0); }
+        if (ny < g.nc[1]) { cy = hy - ry + iy; cy += cy < 0 ? g.nc[1] : (cy >= g.nc[1] ? -g.nc[1] : 0); }
+        const int home = hx * g.nc[1] + hy, nz = g.nc[2];
+        col = cx * g.nc[1] + cy;
+        if (col < home) return false;
+        const int lo = hz - rz, hi = hz + rz;
+        const bool whole = nz <= 2 * rz + 1;
+        if (!(r & 1)) {
+            z0 = col == home ? hz : (whole ? 0 : max(lo, 0));
+            z1 = whole ? nz - 1 : min(hi, nz - 1);
+            return true;
+        }
+        if (whole) return false;
+        if (lo < 0) { z0 = nz + lo; z1 = nz - 1; return true; }       /* later than the home cell in any column */
+        z0 = 0; z1 = hi - nz;
+        return hi >= nz && col != home;
+    }
+};
 
 /* Warp-wide minimum and maximum of floats. */
 __device__ __forceinline__ float warp_min(float v) {
@@ -255,8 +291,8 @@ __device__ __forceinline__ void reduce_scatter12(float (&v)[12], int lane) {
 __device__ __forceinline__ double hi_lo(float hi, float lo) { return isfinite(hi) ? (double)hi + lo : (double)hi; }
 
 /* BATCH: the tiles are those of a batch's replicas (replica geometry, cell offset and tile groups from
- * reps); with MODE kDiffWrap of replicas whose edges all exceed 2 rc: a tile's particles against every
- * later particle of the replica. */
+ * reps); with MODE kDiffWrap of replicas whose edges all exceed 2 rc: a tile's particles against the later
+ * ones of the cells within reach (WrapWindow). */
 template <int ORDER, bool SEP, bool EXTRA, int MODE, bool COUL, bool FINE, bool BATCH = false>
 __global__ void __launch_bounds__(32 * kWarpsPerCta, EXTRA ? 4 : kListCtas)
 k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, const int *__restrict__ cstart,
@@ -280,43 +316,35 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
     }
     __syncthreads();
 
-    {
-        const int nt = tile1.x - tile0.x;
-        const int nitems = kCellPair ? nt : (FINE ? kFineRuns * nt : 2 * nt + (tile1.y - tile0.y));
-        if (blockIdx.x == 0 && threadIdx.x == 0) *nitems_out = nitems;
-        s.tile0 = tile0;
-        s.nt = nt;
-        s.nitems = nitems;
-        __syncwarp();
-    }
+    const int nt = tile1.x - tile0.x;
+    const int nitems = kCellPair ? nt : (FINE ? kFineRuns * nt : 2 * nt + (tile1.y - tile0.y));
+    if (blockIdx.x == 0 && threadIdx.x == 0) *nitems_out = nitems;
 
     const float far = 1.0e18f;
     const unsigned below = (1u << lane) - 1u;
 
     unsigned long long pairs_sum = 0;    /* lane 0: the warp's items' */
-    /* the items of this warp (FINE: CTA): its own number first, then the next from the counter */
-    const int workers = FINE ? gridDim.x : kWarpsPerCta * gridDim.x;
+    /* the next item of this warp; FINE: of this CTA, whose first one is that of its own number (the launch is
+     * short: the counter's latency would show) */
     auto next = [&]() {
         int b = 0;
         if (FINE) {
             __syncthreads();
-            if (threadIdx.x == 0) all[0].next = workers + atomicAdd(work, 1);
+            if (threadIdx.x == 0) all[0].next = gridDim.x + atomicAdd(work, 1);
             __syncthreads();
             return all[0].next;
         }
-        if (lane == 0) b = workers + atomicAdd(work, 1);
+        if (lane == 0) b = atomicAdd(work, 1);
         return __shfl_sync(0xffffffffu, b, 0);
     };
-    for (int b = FINE ? blockIdx.x : kWarpsPerCta * blockIdx.x + warp; b < s.nitems; b = next()) {
+    for (int b = FINE ? blockIdx.x : next(); b < nitems; b = next()) {
         /* item -> class, run, home cell, tile */
         BatchRep rep;
         const Geom &g = BATCH ? rep.g : gparam;
-        int cend = 0, tile, ntile;
+        int coff = 0, tile, ntile;
         {
-            int cls = 0, want = -1, coff = 0, tgw = lt.groups;      /* want: the one run of the item, -1: all */
+            int cls = 0, want = -1, tgw = lt.groups;      /* want: the one run of the item, -1: all */
             int2 e;
-            const int2 tile0 = s.tile0;
-            const int nt = s.nt;
             if (kCellPair) {
                 e = lt.tile[0][tile0.x + b];
                 want = FINE ? 0 : -1;
@@ -332,7 +360,6 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
             if (BATCH) {
                 rep = reps[lt.rep_of_cell[e.x]];
                 coff = rep.cell_off;
-                cend = coff + g.nc[0] * g.nc[1] * g.nc[2];
                 tgw = rep.tile_groups;
             }
             const int h = e.x - coff;
@@ -340,9 +367,12 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
             const int hs = cstart[e.x], ni = cstart[e.x + 1] - hs;
             /* the column: cells (cx, cy, hz - 1 .. hz + 1), or the home cell and the one above */
             bool skip = false;
-            if (!kCellPair) {
-                const int nyz = g.nc[1] * g.nc[2];
-                const int hx = h / nyz, hy = (h / g.nc[2]) % g.nc[1], hz = h % g.nc[2];
+            const int nyz = g.nc[1] * g.nc[2];
+            const int hx = h / nyz, hy = (h / g.nc[2]) % g.nc[1], hz = h % g.nc[2];
+            if (kCellPair) {
+                s.hx = hx;
+                s.hy = hy;
+            } else {
                 int cx = hx + (cls == 1 ? 1 : 0);
                 s.sx = cx >= g.nc[0] ? -g.L[0] : 0.0f;
                 cx = cx >= g.nc[0] ? cx - g.nc[0] : cx;
@@ -359,8 +389,8 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                         skip = skip || cstart[cbase + cz + 1] - cstart[cbase + cz] > kMaxCellOcc;
                     }
                 }
-                s.hz = hz;
             }
+            s.hz = hz;
             s.hs = hs; s.ni = ni; s.cls = cls;
             if (FINE) s.want = want;
             /* the cell's tiles follow from its occupancy alone */
@@ -398,13 +428,25 @@ k_force_list(const float4 *__restrict__ pos, const int *__restrict__ ptype, cons
                         if (jb >= je) {
                             /* the next range: the columns' unwrapped cells, then their cells across a z
                              * face */
-                            const int range = s.range, ncol = kCellPair ? 1 : c_class_cols[s.cls];
-                            if (range == (kCellPair ? 1 : 2 * ncol)) break;
+                            const int range = s.range, ncol = c_class_cols[s.cls];
                             float sy = 0.0f, sz = 0.0f;
                             int lo, hi;
                             bool own = s.cls == 0;
                             if (kCellPair) {
-                                lo = s.hs; hi = cstart[cend]; own = true;
+                                const WrapWindow win(g);
+                                if (range == win.ranges()) break;
+                                int col, z0, z1;
+                                lo = hi = 0;
+                                own = true;
+                                if (win.range(g, s.hx, s.hy, s.hz, range, col, z0, z1)) {
+                                    const int c0 = coff + col * g.nc[2];
+                                    lo = cstart[c0 + z0];
+                                    hi = cstart[c0 + z1 + 1];
+                                    for (int z = z0; z <= z1; ++z)     /* an overflowing cell: bounded time */
+                                        if (cstart[c0 + z + 1] - cstart[c0 + z] > kMaxCellOcc) hi = lo;
+                                }
+                            } else if (range == 2 * ncol) {
+                                break;
                             } else if (range < ncol) {
                                 const int z0 = s.cls ? max(s.hz - 1, 0) : s.hz, z1 = min(s.hz + 1, g.nc[2] - 1);
                                 lo = cstart[s.cbase[range] + z0]; hi = cstart[s.cbase[range] + z1 + 1];
