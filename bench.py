@@ -176,10 +176,20 @@ def measured_peaks() -> dict:
     return {}
 
 
+def force_kernel_signature(tile, order: int, exact: bool, batch: bool) -> str:
+    """The instantiation that a step's (half-shell) force launch runs, as a profiler prints it: order,
+    separate arithmetic, energies, accumulation, difference rule, then k_force_warp: Coulomb, batch;
+    k_force: batch, warps, pruning.  The workloads are charged."""
+    head = f"{order},0,0,0,{3 if exact else 1}"
+    if tile[0] == 1:
+        return f"k_force_warp<{head},1,{int(batch)}>"
+    return f"k_force<{head},{int(batch)},{tile[0]},{tile[2]}>"
+
+
 def ncu_capture(workload: str, tile, order: int, bins: int, exact: bool, min_log2: int) -> dict:
     """The committed ncu figures for this kernel configuration, or a record saying none matches.
-    Each capture names the tile, tables and datapath it was taken with; figures of another
-    configuration are not reported for this one."""
+    Each capture names the tile, tables and datapath it was taken with and the kernel it measured;
+    figures of another configuration, or of a kernel that a launch no longer runs, are not reported."""
     want = {"workload": workload, "tile": list(tile), "order": order, "bins": bins, "exact": bool(exact),
             "table_min_log2": min_log2}
     try:
@@ -187,7 +197,8 @@ def ncu_capture(workload: str, tile, order: int, bins: int, exact: bool, min_log
     except (OSError, json.JSONDecodeError):
         caps = []
     for c in caps:
-        if all(c.get(k) == v for k, v in want.items()):
+        if (all(c.get(k) == v for k, v in want.items()) and
+                c.get("kernel", "").split(" (")[0] == force_kernel_signature(tile, order, exact, workload.startswith("batch"))):
             return {"matched": True, "source": f"profiles/{CAPTURES.name}", **c}
     near = [c for c in caps if c.get("workload") == workload]
     return {"matched": False, "source": f"profiles/{CAPTURES.name}", "wanted": want,
