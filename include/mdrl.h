@@ -133,8 +133,8 @@ typedef struct mdrl_ctx mdrl_ctx;
  * Default {4, 6, 0}; mdrl_autotune picks among both kinds.
  * Force evaluations (mdrl_force_eval*, mdrl_batch_force_eval; MDRL_ACC_FIXED64) run a third kernel,
  * over particle lists, until a CTA tile is asked for by mdrl_set_tile / mdrl_batch_set_tile (the
- * tuner's choice is for dynamics, and ends an earlier call's); under {1, groups, 1} groups splits its items,
- * without effect on the result. */
+ * tuner's choice is for dynamics, and ends an earlier call's); also under {1, groups, 1}, whose groups do
+ * not concern it. */
 typedef struct {
     int warps_per_cta;
     int steps_per_piece;

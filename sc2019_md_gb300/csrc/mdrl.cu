@@ -492,11 +492,11 @@ force_fn pick_force_batch(int order, bool sep, bool extra, bool prune) {
 }  // namespace mdrl
 
 /* Force evaluations take the list kernel unless a caller asked for a CTA tile (the tuner times dynamics'
- * kernels, so its choice says nothing here): it is the faster one at
- * every size measured (92k system, order 1: 250 us against 577 us for the default CTA tile and 374 us
- * for {1, 1, 1}; 1M system, order 2: 1.71 ms against 4.06 and 2.61; 1,728 atoms: within 2 us of the
- * CTA kernel's 18 us).  Dynamics keeps the kernels of its tile: its FP32 partial sums, and so every
- * bit of a trajectory, stay those of runs made before. */
+ * kernels, so its choice says nothing here): it is the faster one at every size measured (92k system,
+ * order 1: 260 us against 577 us for the default CTA tile and 374 us for {1, 1, 1}; 1M system, order 2:
+ * 1.74 ms against 4.06 and 2.61; 1,728 atoms: 20 us, within 2 of the CTA kernel).  Dynamics keeps the
+ * kernels of its tile: its FP32 partial sums, and so every bit of a trajectory, stay those of runs made
+ * before. */
 bool mdrl::list_eval(const mdrl_ctx *c) {
     return c->p.accum == MDRL_ACC_FIXED64 && (!c->tile_asked || c->tile.warps_per_cta == 1);
 }

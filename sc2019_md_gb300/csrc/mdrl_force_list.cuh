@@ -2,14 +2,17 @@
  * mdrl_force_list.cuh — the half-shell pair-force kernel of force evaluations, over particle lists
  * (sm_103a).
  *
- * Work item = (home cell, column class, split).  The 14 half-shell cells of a home cell
+ * Work item = (tile of a home cell, column class).  The 14 half-shell cells of a home cell
  * (SC/Particle_Pair_Gen_HalfShell.v:14-24) are 5 columns of cells along z -- (0,0): the home cell and
  * the one above; (0,1), (1,-1), (1,0), (1,1): three cells each -- and cells that follow one another in
  * z follow one another in the cell-sorted arrays, so a column is one contiguous range of particles
  * plus, at the z faces of the box, one wrapped cell.  Classes: (0,0); (1,0) with its two diagonal
  * neighbours; (0,1).  The home cell's particles are cut into groups of 4 (consecutive on the in-cell
- * Hilbert curve, so compact in space) and these into even tiles of at most 8 groups; split s of S
- * takes tiles s, s + S, ...  Per tile one warp
+ * Hilbert curve, so compact in space) and these into even tiles of at most 4 or 8 groups, which the binning
+ * numbers and writes down (Tiles in mdrl_kernels.cuh): a launch has as many items as there are tiles,
+ * however unevenly the cells are filled.  (Items by the mean occupancy: a droplet of 13,000 atoms in a
+ * 200 A box 1,250 us, 60,000 in 300 A 19.95 ms; now 207 us and 0.95 ms, evenly filled systems alike.)
+ * Per item one warp
  *   1. lists the class's particles that lie within rc of the tile's bounding box (one lane per
  *      particle, ballot + popc compaction);
  *   2. marks, per listed particle, the groups whose bounding box it is within rc of: 2 in 3 of the
@@ -28,7 +31,7 @@
  * mdrl_force_warp.cuh (tests/test_cull_bound.py) with one particle for the second box.  So the accepted
  * pairs are those of the plain traversal, bit for bit.  Deterministic: every FP32 partial sum is of one
  * tile and one list, whose order follows from the particles of its cells alone, and the int64
- * global sums are exact; so the result does not depend on scheduling, on S, or on what else a launch
+ * global sums are exact; so the result does not depend on scheduling or on what else a launch
  * holds (other replicas, other slabs), nor on whether the items are fine (below).
  *
  * The grid is persistent: as many CTAs as fit, 4 independent warps each, which share the type-pair
@@ -36,10 +39,11 @@
  * last.  A launch with few items runs fine ones: an item is one run, and the 4 warps of a CTA share it,
  * one group each.
  *
- * What bounds it (92k system, order 2, exact rule: 276 us, 362 us for the kernel it replaces; 1M system
- * 1.71 ms, 2.61; order 1 92k 250 us): the L1 data pipe, 79 % busy, most of it on the table gathers.
- * Timed without parts: no table 210 us (at 299), no c2 gather of r^-3 274, no j accumulation 278, no
- * i reduction 284, no atomics 290, lists alone 77.  The gathers of one table element are therefore
+ * What bounds it (92k system, order 2, exact rule: 283 us, 362 us for the kernel it replaces; 1M system
+ * 1.74 ms, 2.61; order 1 92k 260 us): the L1 data pipe, 73 % busy at 92k and 82 % at 1M
+ * (profiles/evaluation_and_dynamics_kernels.md), most of it on the table gathers.  An earlier build timed
+ * without parts: no table 210 us (at 299), no c2 gather of r^-3 274, no j accumulation 278, no i
+ * reduction 284, no atomics 290, lists alone 77.  The gathers of one table element are therefore
  * kept in arrays of their own: 16-byte elements at a 32-byte stride use half the banks (299 -> 276 us
  * with the 13-shuffle reduction and the prefetch of the next block's positions).  20 warps per SM at 96
  * registers: 16 at 128 are 2-5 % slower.  What a phase does not need is kept in shared memory, or the
