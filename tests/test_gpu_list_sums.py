@@ -114,3 +114,20 @@ def test_infinite_energies_stay_infinite():
     assert st["e_lj"] == np.inf and np.isfinite(st["virial"])
     st = _planted([1, 2], [[24.5, 18.0, 18.0], [26.0, 17.0, 18.0]], 1, (-3.0e38, 1.0), (1.0, 1.0))
     assert st["e_lj"] == -np.inf and np.isfinite(st["virial"])
+
+
+@pytest.mark.parametrize("each,ok", [(1.0e11, True), (4.0e11, False)])
+def test_sums_beyond_the_fixed_point_range_are_reported(each, ok):
+    """Two forces that the accumulators hold and whose sum (8e11 kcal/mol/A) they do not, in one list."""
+    pos = np.array([[24.0, 18.0, 18.0], [26.0, 19.0, 18.0], [26.0, 17.0, 18.0]], np.float32)
+    coef = np.zeros((3, 3, 4))
+    coef[0, 1, 0] = coef[1, 0, 0] = each / 2.0 * 5.0 ** 7
+    with m.Context(_params()) as ctx:
+        ctx.set_pair_coefficients(coef)
+        call = lambda: ctx.force(*(np.ascontiguousarray(pos[:, k]) for k in range(3)), type=np.array([0, 1, 1], np.int32))  # noqa: E731
+        if ok:
+            assert abs(call()[0][0, 0] + 2 * each) < 1e-2 * each
+        else:
+            with pytest.raises(m.MdrlError) as e:
+                call()
+            assert e.value.status == 3
