@@ -41,7 +41,7 @@
  *
  * What bounds it (92k system, order 2, exact rule: 283 us, 362 us for the kernel it replaces; 1M system
  * 1.74 ms, 2.61; order 1 92k 260 us): the L1 data pipe, 73 % busy at 92k and 82 % at 1M
- * (profiles/evaluation_and_dynamics_kernels.md), most of it on the table gathers.  An earlier build timed
+ * under the profiler, most of it on the table gathers.  An earlier build timed
  * without parts: no table 210 us (at 299), no c2 gather of r^-3 274, no j accumulation 278, no i
  * reduction 284, no atomics 290, lists alone 77.  The gathers of one table element are therefore
  * kept in arrays of their own: 16-byte elements at a 32-byte stride use half the banks (299 -> 276 us
